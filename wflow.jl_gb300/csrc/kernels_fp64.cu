@@ -23,9 +23,15 @@
 #include "wf_ff.cuh"
 #include "wf_walker.cuh"
 
+using wfm::div_;
+using wfm::div_by_;
+using wfm::gt0_;
+using wfm::gt_;
 using wfm::jclamp;
 using wfm::jmax;
 using wfm::jmin;
+using wfm::le0_;
+using wfm::lt_;
 
 namespace {
 
@@ -37,29 +43,33 @@ constexpr double PERCENT = 1e-2;                                  // units.jl PE
 constexpr double NANV = __builtin_nan("");
 
 // ------------------------------------------------------------------ process functions ----
+// Divisors that a cell divides by several times (the step, the porosity, a layer's saturated
+// depth) come with their reciprocal (rdt, r...): such a quotient costs 3 FP64 instructions
+// (wf_math.cuh div_by_), and each FP64 instruction of a warp 64 cycles.
 
 // vegetation/rainfall_interception.jl:9-70
 __device__ void interception_gash(double cmax, double e_r, double gap, double P, double max_evap, double dt,
-                                  double& tf, double& ic, double& sf) {
-    if (cmax > 0.0) {
+                                  double rdt, double& tf, double& ic, double& sf) {
+    if (gt0_(cmax)) {
         double fs, fi, psat;
-        if (gap < 1.0 / 1.1) {
+        if (lt_(gap, 1.0 / 1.1)) {
             fs = 0.1 * gap;
             fi = 1.0 - 1.1 * gap;
-            psat = e_r > fi ? 0.0 : -cmax / (e_r * dt) * wfm::log(1.0 - e_r / fi);
+            psat = gt_(e_r, fi) ? 0.0 : div_(-cmax, e_r * dt) * wfm::log(1.0 - div_(e_r, fi));
         } else {
             fs = 1.0 - gap;
             fi = 0.0;
             psat = 0.0;
         }
-        if (P > psat) {
-            ic = (fi * psat - cmax / dt) + e_r * (P - psat) + cmax / dt;
+        if (gt_(P, psat)) {
+            const double cmax_dt = div_by_(cmax, dt, rdt);
+            ic = (fi * psat - cmax_dt) + e_r * (P - psat) + cmax_dt;
         } else {
             ic = fi * P;
         }
         sf = fs * P;
         tf = P - ic - sf;
-        if (ic > max_evap) {
+        if (gt_(ic, max_evap)) {
             const double drain = ic - max_evap;
             ic = max_evap;
             tf += drain;
@@ -73,9 +83,9 @@ __device__ void interception_gash(double cmax, double e_r, double gap, double P,
 
 // vegetation/rainfall_interception.jl:78-130
 __device__ void interception_modrut(double P, double pet, double& cs, double gap, double cmax, double dt,
-                                    double& tf, double& ce, double& sf) {
+                                    double rdt, double& tf, double& ce, double& sf) {
     double fs, pc;
-    if (gap < 1.0 / 1.1) {
+    if (lt_(gap, 1.0 / 1.1)) {
         fs = 0.1 * gap;
         pc = (1.0 - gap - fs) * P;
     } else {
@@ -84,54 +94,65 @@ __device__ void interception_modrut(double P, double pet, double& cs, double gap
     }
     sf = fs * P;
     tf = gap * P;
-    if (cs > cmax) {
+    if (gt_(cs, cmax)) {
         const double d = cs - cmax;
         cs = cmax;
-        tf += d / dt;
+        tf += div_by_(d, dt, rdt);
     }
     cs += pc * dt;
-    const double max_evap = cs / dt;
-    if (pet > max_evap) {
+    const double max_evap = div_by_(cs, dt, rdt);
+    if (gt_(pet, max_evap)) {
         ce = max_evap;
         cs = 0.0;
     } else {
         ce = pet;
         cs -= ce * dt;
     }
-    if (cs > cmax) {
+    if (gt_(cs, cmax)) {
         const double d = cs - cmax;
         cs = cmax;
-        tf += d / dt;
+        tf += div_by_(d, dt, rdt);
     }
 }
 
 // utils.jl:27-30
 __device__ __forceinline__ double scurve(double x, double a, double b, double c) {
-    return 1.0 / (b + wfm::exp(-c * (x - a)));
+    return div_(1.0, b + wfm::exp(-c * (x - a)));
 }
 
 // utils.jl:1070-1076 with Wflow's pow
-__device__ __forceinline__ double bounded_power(double base, double p) { return base > 1.0 ? 1.0 : wfm::pow(base, p); }
+__device__ __forceinline__ double bounded_power(double base, double p) { return gt_(base, 1.0) ? 1.0 : wfm::pow(base, p); }
 
-// soil/soil_process.jl:51-92
-__device__ void unsatzone_flow_layer(double usd, double kv_z, double l_sat, double c, double dt, double& usd_out,
-                                     double& flow) {
-    if (usd <= 0.0) {
+// soil/soil_process.jl:51-92. The iteration is the longest serial chain of the column (a daily step
+// takes hundreds): its quotients by l_sat and dt use the reciprocals, and `st < usd / dt` is decided
+// from st dt, which the update needs anyway, unless the two are within 16 ulps. 55 FP64
+// instructions per iteration (119 with plain divisions, comparisons and the generic exp and log).
+__device__ void unsatzone_flow_layer(double usd, double kv_z, double l_sat, double c, double dt, double rdt,
+                                     double& usd_out, double& flow) {
+    if (le0_(usd)) {
         usd_out = 0.0;
         flow = 0.0;
         return;
     }
+    const double r_sat = div_(1.0, l_sat);
     const double st_sat = jmax(0.0, usd - l_sat);
-    double st = kv_z * bounded_power(usd / l_sat, c);
-    double sum_ast = jmin(st, st_sat / dt);
+    double st = kv_z * bounded_power(div_by_(usd, l_sat, r_sat), c);
+    double sum_ast = jmin(st, div_by_(st_sat, dt, rdt));
     usd -= sum_ast * dt;
     const double remainder = jmin((st - sum_ast) * dt, usd);
     const long its = (long)wfm::cld(remainder, 2e-4);
+    const double kv_it = its > 0 ? div_(kv_z, (double)its) : 0.0;
     for (long i = 0; i < its; ++i) {
-        st = (kv_z / (double)its) * bounded_power(usd / l_sat, c);
-        const double st_max = usd / dt;
-        if (st < st_max) {
-            usd -= st * dt;
+        st = kv_it * bounded_power(div_by_(usd, l_sat, r_sat), c);
+        const double taken = st * dt;
+        bool below = gt0_(taken) && gt0_(usd) && wfm::to_bits(taken) + 16 < wfm::to_bits(usd);
+        double st_max = 0.0;
+        if (!below) {
+            st_max = div_by_(usd, dt, rdt);
+            below = lt_(st, st_max);
+        }
+        if (below) {
+            usd -= taken;
             sum_ast += st;
         } else {
             usd = 0.0;
@@ -145,28 +166,43 @@ __device__ void unsatzone_flow_layer(double usd, double kv_z, double l_sat, doub
 
 // soil/soil_process.jl:113-130
 __device__ __forceinline__ double head_brooks_corey(double vwc, double ts, double tr, double c, double psi) {
-    const double lam = 2.0 / (c - 3.0);
-    return lam > 0.0 ? psi / wfm::pow(vwc / (ts - tr), 1.0 / lam) : psi;
+    const double lam = div_(2.0, c - 3.0);
+    return gt0_(lam) ? div_(psi, wfm::pow(div_(vwc, ts - tr), div_(1.0, lam))) : psi;
 }
 
 // soil/soil_process.jl:166-176
 __device__ __forceinline__ double feddes_h3(double h3h, double h3l, double tpot) {
-    const double td = tpot / MM_PER_DAY;
-    if (td <= 1.0) return h3l;
-    if (td < 5.0) return h3l + (h3h - h3l) * (td - 1.0) / (5.0 - 1.0);
+    const double td = div_by_(tpot, MM_PER_DAY, 1.0 / MM_PER_DAY);
+    if (wfm::le_(td, 1.0)) return h3l;
+    if (lt_(td, 5.0)) return h3l + (h3h - h3l) * (td - 1.0) / (5.0 - 1.0);
     return h3h;
 }
 
 // soil/soil_process.jl:183-200
 __device__ __forceinline__ double rwu_feddes(double h, double h1, double h2, double h3, double h4, double a1) {
-    if (h < h4) return 0.0;
-    if (h < h3) return (h - h4) / (h3 - h4);
-    if (a1 == 0.0) {
-        if (h < h2) return 1.0;
-        if (h < h1) return (h1 - h) / (h1 - h2);
+    if (lt_(h, h4)) return 0.0;
+    if (lt_(h, h3)) return div_(h - h4, h3 - h4);
+    if (wfm::is_zero_(a1)) {
+        if (lt_(h, h2)) return 1.0;
+        if (lt_(h, h1)) return div_(h1 - h, h1 - h2);
         return 0.0;
     }
     return 1.0;
+}
+
+// rwu_feddes of a layer's Brooks-Corey head. The reduction is 0 below h4 and, for a1 != 0, 1 from h3
+// up: an FP32 head (within 1e-5) decides those cases when it is more than 0.1 % away from both
+// heads, and only the heads between them pay the power and three divisions (80 FP64 instructions).
+__device__ __forceinline__ double rwu_layer(double vwc, double ts, double tr, double c, double psi, double h1, double h2,
+                                            double h3, double h4, double a1) {
+    const float x = wfm::f32_of(vwc) / (wfm::f32_of(ts) - wfm::f32_of(tr));
+    const float p32 = wfm::f32_of(psi), c32 = wfm::f32_of(c), lo = wfm::f32_of(h4), hi = wfm::f32_of(h3);
+    if (c32 > 3.01f && c32 < 60.0f && p32 < 0.0f && lo < hi && hi < 0.0f && x > 1e-6f && x < 1e6f) {
+        const float head = p32 * exp2f(-0.5f * (c32 - 3.0f) * log2f(x));
+        if (head > hi * 0.999f && !wfm::is_zero_(a1)) return 1.0;
+        if (head < lo * 1.001f) return 0.0;
+    }
+    return rwu_feddes(head_brooks_corey(vwc, ts, tr, c, psi), h1, h2, h3, h4, a1);
 }
 
 __device__ __forceinline__ double lb_drainable(double ts, double tfc) { return jmax(ts - tfc, 0.02); }
@@ -234,11 +270,12 @@ struct Column {
 #pragma unroll
         for (int k = 0; k < MAXN; ++k) {
             if (k >= N) break;
-            double t = act[k] * NANV;
-            if (ref > cum[k + 1]) {
+            double t = NANV;
+            if (gt_(ref, cum[k + 1])) {
                 t = act[k];
-            } else if (ref - cum[k] > 0.0) {
-                t = ref - cum[k];
+            } else {
+                const double above = ref - cum[k];
+                if (gt0_(above)) t = above;
             }
             thick[k] = t;
             if (wfm::isnan_(t)) nu -= 1;
@@ -247,7 +284,7 @@ struct Column {
     // utils.jl:727-761 (n is 1-based)
     __device__ __forceinline__ double kv_at(const double* kvf, double z, int n) const {
         double zz = z;
-        if (profile == WF_KV_EXPONENTIAL_CONSTANT && !(z < zexp)) zz = zexp;
+        if (profile == WF_KV_EXPONENTIAL_CONSTANT && !lt_(z, zexp)) zz = zexp;
         return kvf[n - 1] * kv0 * wfm::exp(-f * zz);
     }
     // soil.jl:1213-1259
@@ -258,14 +295,14 @@ struct Column {
         for (int k = 0; k < MAXN; ++k) tprev[k] = thick[k];
         set_thickness(zi);
         const int n_new = nu;
-        if (zi < zi_prev) {
+        if (lt_(zi, zi_prev)) {
 #pragma unroll
             for (int k = 1; k <= MAXN; ++k) {
                 if (k < n_new || k > n_prev) continue;
                 if (wfm::isnan_(thick[k - 1])) {
                     usld[k - 1] = 0.0;
                 } else {
-                    const double sc = thick[k - 1] / tprev[k - 1];
+                    const double sc = div_(thick[k - 1], tprev[k - 1]);
                     usld[k - 1] = sc * usld[k - 1];
                 }
             }
@@ -282,23 +319,23 @@ struct Column {
     // utils.jl:1090-1131
     __device__ void water_table_change(double net_flux, double sy, double dt, double& dh, double& exfilt) const {
         const double te = ts - tr;
-        if (net_flux <= 0.0) {
-            dh = net_flux * dt / sy;
+        if (le0_(net_flux)) {
+            dh = div_(net_flux * dt, sy);
         } else {
             dh = 0.0;
 #pragma unroll
             for (int k = MAXN; k >= 1; --k) {
                 if (k > nu) continue;
-                const double cap = jmax(thick[k - 1] * te - usld[k - 1], 0.0) / dt;
+                const double cap = div_(jmax(thick[k - 1] * te - usld[k - 1], 0.0), dt);
                 const double fl = jmin(net_flux, cap);
-                if (cap <= net_flux) {
+                if (wfm::le_(cap, net_flux)) {
                     dh += thick[k - 1];
                 } else {
-                    const double syk = te - (usld[k - 1] / thick[k - 1]);
-                    dh += fl * dt / syk;
+                    const double syk = te - div_(usld[k - 1], thick[k - 1]);
+                    dh += div_(fl * dt, syk);
                 }
                 net_flux -= fl;
-                if (net_flux == 0.0) break;
+                if (wfm::is_zero_(net_flux)) break;
             }
         }
         exfilt = jmax(net_flux, 0.0);
@@ -426,7 +463,7 @@ template <int MAXN, int PHASE>
 __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
     const int M = F.M;
     const int64_t E = F.land_slots * M;
-    const double dt = F.dt;
+    const double dt = F.dt, rdt = div_(1.0, F.dt);
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t slot = e / M;
         if (F.land_node_of_slot[slot] < 0) continue;
@@ -445,26 +482,26 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
             Mf[BL_PREV][e] = Mf[TSWS][e] + canopy + (snow + snow_water) + glacier_storage(F, e, slot) + 0.0;
         // ---- interception (canopy.jl:213-226 Gash, :259-271 Rutter)
         if (F.gash) {
-            interception_gash(cmax, L[E_R][slot], gap, Pr, potevap, dt, tf, ic, sf);
+            interception_gash(cmax, L[E_R][slot], gap, Pr, potevap, dt, rdt, tf, ic, sf);
         } else {
-            interception_modrut(Pr, potevap, canopy, gap, cmax, dt, tf, ic, sf);
+            interception_modrut(Pr, potevap, canopy, gap, cmax, dt, rdt, tf, ic, sf);
         }
         // ---- snow (snow.jl:238-293, snow_process.jl:26-116)
         if (F.snow) {
             const double eff = tf + sf;
             const double tti = L[TTI][slot], tt = L[TT][slot];
             double rainfrac;
-            if (tti == 0.0) {
-                rainfrac = T > tt ? 1.0 : 0.0;
+            if (wfm::is_zero_(tti)) {
+                rainfrac = gt_(T, tt) ? 1.0 : 0.0;
             } else {
-                rainfrac = jclamp((T - (tt - tti / 2.0)) / tti, 0.0, 1.0);
+                rainfrac = jclamp(div_(T - (tt - tti * 0.5), tti), 0.0, 1.0);
             }
             const double snowfrac = 1.0 - rainfrac;
             const double sp = snowfrac * 1.0 * eff, lp = rainfrac * 1.0 * eff;
             const double ttm = L[TTM][slot], ddf = L[DDF][slot], whc = L[WHC][slot];
             double melt;
-            if (T > ttm) {
-                melt = jmin(ddf * (T - ttm), snow / dt);
+            if (gt_(T, ttm)) {
+                melt = jmin(ddf * (T - ttm), div_by_(snow, dt, rdt));
                 snow -= melt * dt;
                 snow_water += melt * dt;
             } else {
@@ -478,8 +515,8 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
             snow += sp * dt;
             snow_water += lp * dt;
             const double maxsw = snow * whc;
-            if (snow_water > maxsw) {
-                srunoff = (snow_water - maxsw) / dt;
+            if (gt_(snow_water, maxsw)) {
+                srunoff = div_by_(snow_water - maxsw, dt, rdt);
                 snow_water = maxsw;
             } else {
                 srunoff = 0.0;
@@ -493,9 +530,9 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
             Mf[SNOW_WATER][e] = snow_water;
             F.GM[GM_SRUNOFF][e] = srunoff;
             F.GM[GM_IC][e] = ic;
-            const double frac = jmin(0.5, L[SLOPE][slot] / 5.67) * jmin(1.0, snow / 10.0);
-            F.GM[GM_CAP][e] = frac * snow / dt;
-            F.GM[GM_CAPW][e] = snow_water * frac / dt;
+            const double frac = jmin(0.5, div_(L[SLOPE][slot], 5.67)) * jmin(1.0, div_(snow, 10.0));
+            F.GM[GM_CAP][e] = div_by_(frac * snow, dt, rdt);
+            F.GM[GM_CAPW][e] = div_by_(snow_water * frac, dt, rdt);
             continue;
         }
         } else {
@@ -524,8 +561,8 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
         const double wd_river = rs >= 0 ? F.RM[RV_H][rs * M + m] : 0.0;
         const double runoff_river = jmin(1.0, rfrac) * wfs;
         const double runoff_land = jmin(1.0, wfrac) * wfs;
-        const double ae_river = rfrac * jmin(wd_river / dt, PET);
-        const double ae_land = wfrac * jmin(wd_land / dt, PET);
+        const double ae_river = rfrac * jmin(div_by_(wd_river, dt, rdt), PET);
+        const double ae_land = wfrac * jmin(div_by_(wd_land, dt, rdt), PET);
         // ---- soil (soil.jl:643-682, 1150-1211)
         const double soil_fraction = jmax(gap - wfrac - rfrac - gfrac, 0.0);
         const double pot_trans = jmax(0.0, potevap - ic);
@@ -554,7 +591,8 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
 #pragma unroll
         for (int k = 0; k < MAXN; ++k)
             if (k < col.nl) usd += col.usld[k];
-        double zi = jmax(0.0, col.d - sat / (ts - tr));
+        const double te = ts - tr, rte = div_(1.0, te);
+        double zi = jmax(0.0, col.d - div_by_(sat, te, rte));
         double drain = (col.d - zi) * lb_drainable(ts, col.tfc);
         double ucap = swc - sat - usd;
         col.set_thickness(zi);
@@ -574,7 +612,7 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
         const double pathinf = wfs_soil * cfrac;
         const double mis = jmin(cap_soil * fred, soilinf);
         const double mip = jmin(cap_comp * fred, pathinf);
-        const double infiltration = jmin(mip + mis, jmax(0.0, ucap / dt));
+        const double infiltration = jmin(mip + mis, jmax(0.0, div_by_(ucap, dt, rdt)));
         const double infex = (soilinf - mis) + (pathinf - mip);
         // unsaturated_zone_flow! (soil.jl:764-804)
         double transfer = 0.0;
@@ -588,7 +626,7 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
                 const double kv_z = col.kv_at(kvf, z, k + 1);
                 const double u = k == 0 ? col.usld[k] + infiltration * dt : col.usld[k] + flow * dt;
                 double uo;
-                unsatzone_flow_layer(u, kv_z, l_sat, cexp[k], dt, uo, flow);
+                unsatzone_flow_layer(u, kv_z, l_sat, cexp[k], dt, rdt, uo, flow);
                 col.usld[k] = uo;
             }
             transfer = flow;
@@ -601,17 +639,17 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
             if (col.nu == 0) {
                 se = 0.0;
             } else if (col.nu == 1) {
-                se = pot * jmin(1.0, col.usld[0] / (zi * (ts - tr)));
+                se = pot * jmin(1.0, div_(col.usld[0], zi * (ts - tr)));
             } else {
-                se = pot * jmin(1.0, col.usld[0] / (col.thick[0] * (ts - tr)));
+                se = pot * jmin(1.0, div_(col.usld[0], col.thick[0] * (ts - tr)));
             }
-            se = jmin(se, col.usld[0] / dt);
+            se = jmin(se, div_by_(col.usld[0], dt, rdt));
             pot -= se;
             col.usld[0] = col.usld[0] - se * dt;
             const double thd = lb_drainable(ts, col.tfc);
             if (col.nu == 0 || col.nu == 1) {
-                esat = pot * jmin(1.0, (col.act[0] - zi) / col.act[0]);
-                esat = jmin(esat, (col.act[0] - zi) * thd / dt);
+                esat = pot * jmin(1.0, div_(col.act[0] - zi, col.act[0]));
+                esat = jmin(esat, div_by_((col.act[0] - zi) * thd, dt, rdt));
             } else {
                 esat = 0.0;
             }
@@ -630,25 +668,27 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
             for (int k = 1; k <= MAXN; ++k) {
                 if (k > col.nu) break;
                 double r;
-                if (k == col.nu && zi < rd) {
+                if (k == col.nu && lt_(zi, rd)) {
                     const double rl = jmin(col.act[k - 1], rd - col.cum[k - 1]);
-                    r = rfr[k - 1] * (col.thick[k - 1] / rl);
+                    r = rfr[k - 1] * div_(col.thick[k - 1], rl);
                 } else {
                     r = rfr[k - 1];
                 }
                 sum_rf += r;
                 rf_low = r;
             }
+            const double root_scale = jmax(div_(1.0, sum_rf), 1.0);
 #pragma unroll
             for (int k = 1; k <= MAXN; ++k) {
                 if (k > col.nu) break;
                 const double r = k < col.nu ? rfr[k - 1] : rf_low;
-                const double rs_ = rd > 0.0 ? jmax(1.0 / sum_rf, 1.0) * r : 0.0;
-                const double vwc = jmax(col.usld[k - 1] / col.thick[k - 1], 1e-7);
-                const double head = head_brooks_corey(vwc, ts, tr, cexp[k - 1], psi);
-                const double alpha = rwu_feddes(head, h1, h2, h3, h4, a1);
-                const double availcap = jmin(1.0, jmax(0.0, (rd - col.cum[k - 1]) / col.thick[k - 1]));
-                const double maxextr = col.usld[k - 1] * availcap / dt;
+                const double rs_ = gt0_(rd) ? root_scale * r : 0.0;
+                const double r_thick = div_(1.0, col.thick[k - 1]);
+                const double vwc = jmax(div_by_(col.usld[k - 1], col.thick[k - 1], r_thick), 1e-7);
+                const double alpha = rwu_layer(vwc, ts, tr, cexp[k - 1], psi, h1, h2, h3, h4, a1);
+                const double availcap =
+                    jmin(1.0, jmax(0.0, div_by_(rd - col.cum[k - 1], col.thick[k - 1], r_thick)));
+                const double maxextr = div_by_(col.usld[k - 1] * availcap, dt, rdt);
                 const double a = jmin(alpha * rs_ * pot_trans, maxextr);
                 col.usld[k - 1] = col.usld[k - 1] - a * dt;
                 actevapustore += a;
@@ -656,7 +696,7 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
             const double wetroots = scurve(zi, rd, 1.0, L[ROOTDISTPAR][slot]);
             const double alpha0 = rwu_feddes(0.0, h1, h2, h3, h4, a1);
             const double rest = pot_trans - actevapustore;
-            act_sat = jmin(rest * wetroots * alpha0, drain / dt);
+            act_sat = jmin(rest * wetroots * alpha0, div_by_(drain, dt, rdt));
             drain -= act_sat * dt;
             transpiration = actevapustore + act_sat;
         }
@@ -669,7 +709,7 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
             col.usld[k - 1] = col.usld[k - 1] - excess;
             if (k > 1) col.usld[k - 2] = col.usld[k - 2] + excess;
         }
-        const double act_infilt = infiltration - excess / dt;
+        const double act_infilt = infiltration - div_by_(excess, dt, rdt);
         const double satex = (wfs_soil - act_infilt) - infex;
         // unsaturated store and capacity for the capillary flux (soil.jl:1193-1196)
         usd = 0.0;
@@ -681,15 +721,15 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
         double capflux_act = 0.0;
         if (col.nu > 0) {
             const double ksat = col.kv_at(kvf, zi, col.nu);
-            const double maxcap = jmax(0.0, jmin(jmin(jmin(ksat, actevapustore), ucap / dt), drain / dt));
+            const double maxcap = jmax(0.0, jmin(jmin(jmin(ksat, actevapustore), div_by_(ucap, dt, rdt)), div_by_(drain, dt, rdt)));
             const double rd = L[ROOTING_DEPTH][slot];
             const double chmax = L[CAP_HMAX][slot];
-            double capflux = zi > rd ? maxcap * wfm::pow(1.0 - jmin(zi, chmax) / chmax, L[CAP_N][slot]) : 0.0;
+            double capflux = gt_(zi, rd) ? maxcap * wfm::pow(1.0 - div_(jmin(zi, chmax), chmax), L[CAP_N][slot]) : 0.0;
 #pragma unroll
             for (int k = MAXN; k >= 1; --k) {
                 if (k > col.nu) continue;
                 const double toadd =
-                    jmin(capflux, jmax((col.thick[k - 1] * (ts - tr) - col.usld[k - 1]) / dt, 0.0));
+                    jmin(capflux, jmax(div_by_(col.thick[k - 1] * (ts - tr) - col.usld[k - 1], dt, rdt), 0.0));
                 col.usld[k - 1] = col.usld[k - 1] + toadd * dt;
                 capflux -= toadd;
                 capflux_act += toadd;
@@ -697,7 +737,7 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
         }
         // leakage! (soil.jl:1118-1136)
         const double deepksat = col.kv_at(kvf, col.d, col.nl);
-        const double leak = jmax(0.0, jmin(L[MAX_LEAKAGE][slot], jmin(drain / dt, deepksat)));
+        const double leak = jmax(0.0, jmin(L[MAX_LEAKAGE][slot], jmin(div_by_(drain, dt, rdt), deepksat)));
         const double recharge = (transfer - capflux_act - leak - act_sat - esat);
         double aet = soilevap + transpiration + ae_river + ae_land + 0.0;
         aet += ic;  // sbm.jl:130

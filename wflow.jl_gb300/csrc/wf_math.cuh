@@ -16,6 +16,15 @@
 //   * cbrt: split off the exponent in thirds, Newton iterations on y^3 = m.
 // Polynomials use explicit fma(); the translation units that include this header for the
 // FP64 form are compiled with --fmad=false so nothing else is contracted.
+//
+// Device paths. On a GB300 every FP64-pipe instruction of a warp (DADD, DMUL, DFMA, compares,
+// rint, conversions) holds its scheduler for 64 cycles, whatever the number of active lanes and
+// however independent the instructions are, while an integer instruction takes about 4 (measured
+// with chains of one instruction kind: 63.6 cycles per DFMA with 1 or 32 lanes and 1 or 4
+// independent chains; a division 563, a square root 597, rcp.approx.ftz.f64 19). So the device
+// paths below take comparisons, classifications and scalings by powers of two to the integer
+// pipe, fuse a multiply and an add where the product is exact, and divide in 6 FP64 instructions.
+// The results are the host paths' bit for bit.
 #pragma once
 
 #include <cstdint>
@@ -49,7 +58,75 @@ WF_HD uint64_t to_bits(double d) {
     return b;
 #endif
 }
-WF_HD bool isnan_(double x) { return x != x; }
+// FP64 comparisons on the integer pipe. order_key maps the values to integers of the same order
+// (-0.0 just below +0.0), for everything but NaN.
+WF_HD long long order_key(double x) {
+    const long long b = (long long)to_bits(x);
+    return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
+}
+#ifdef __CUDACC__
+// exponent field all ones: infinity or NaN
+__device__ __forceinline__ bool special_(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+#endif
+WF_HD bool isnan_(double x) {
+#ifdef __CUDA_ARCH__
+    return (to_bits(x) & 0x7fffffffffffffffULL) > 0x7ff0000000000000ULL;
+#else
+    return x != x;
+#endif
+}
+#ifdef __CUDACC__
+// x in FP32, rounded towards zero, on the integer pipe (the conversion instruction is an FP64 one):
+// exponent rebias and the leading 24 bits. Below 2^-126 it gives 0, from 2^128 on infinity (NaN
+// too): for estimates only.
+__device__ __forceinline__ float f32_of(double x) {
+    const uint64_t b = to_bits(x) & 0x7fffffffffffffffULL;
+    const uint32_t s = (uint32_t)__double2hiint(x) & 0x80000000u;
+    uint32_t f = (uint32_t)((b - 0x3800000000000000ULL) >> 29);
+    if (b < 0x3810000000000000ULL) f = 0u;
+    if (b >= 0x47f0000000000000ULL) f = 0x7f800000u;
+    return __uint_as_float(f | s);
+}
+#endif
+// x < y and x == 0 as IEEE comparisons
+WF_HD bool lt_(double x, double y) {
+#ifdef __CUDA_ARCH__
+    if (special_(x) || special_(y)) return x < y;
+    return order_key(x) < order_key(y) && ((to_bits(x) | to_bits(y)) << 1) != 0;
+#else
+    return x < y;
+#endif
+}
+WF_HD bool gt_(double x, double y) { return lt_(y, x); }
+WF_HD bool le_(double x, double y) {  // x <= y
+#ifdef __CUDA_ARCH__
+    if (special_(x) || special_(y)) return x <= y;
+    return order_key(x) <= order_key(y) || ((to_bits(x) | to_bits(y)) << 1) == 0;
+#else
+    return x <= y;
+#endif
+}
+WF_HD bool is_zero_(double x) {
+#ifdef __CUDA_ARCH__
+    return (to_bits(x) << 1) == 0;
+#else
+    return x == 0.0;
+#endif
+}
+WF_HD bool gt0_(double x) {  // x > 0
+#ifdef __CUDA_ARCH__
+    return (long long)to_bits(x) > 0 && to_bits(x) <= 0x7ff0000000000000ULL;
+#else
+    return x > 0.0;
+#endif
+}
+WF_HD bool le0_(double x) {  // x <= 0
+#ifdef __CUDA_ARCH__
+    return ((long long)to_bits(x) <= 0 && to_bits(x) <= 0xfff0000000000000ULL);
+#else
+    return x <= 0.0;
+#endif
+}
 WF_HD bool signbit_(double x) { return (to_bits(x) >> 63) != 0; }
 WF_HD double fabs_(double x) { return from_bits(to_bits(x) & 0x7fffffffffffffffULL); }
 WF_HD double rint_(double x) {
@@ -100,29 +177,99 @@ WF_HD double copysign_(double x, double s) {
 
 // Julia Base.min / Base.max / clamp for Float64
 WF_HD double jmin(double x, double y) {
+#ifdef __CUDA_ARCH__
+    if (!special_(x) && !special_(y)) return order_key(x) < order_key(y) ? x : y;
+#endif
     if (isnan_(x) || isnan_(y)) return x + y;
     if (x < y) return x;
     if (y < x) return y;
     return signbit_(x) ? x : y;
 }
 WF_HD double jmax(double x, double y) {
+#ifdef __CUDA_ARCH__
+    if (!special_(x) && !special_(y)) return order_key(x) > order_key(y) ? x : y;
+#endif
     if (isnan_(x) || isnan_(y)) return x + y;
     if (x > y) return x;
     if (y > x) return y;
     return signbit_(x) ? y : x;
 }
-WF_HD double jclamp(double x, double lo, double hi) { return x > hi ? hi : (x < lo ? lo : x); }
+WF_HD double jclamp(double x, double lo, double hi) { return gt_(x, hi) ? hi : (lt_(x, lo) ? lo : x); }
+
+// ---- division
+//
+// A quotient q = a r from a reciprocal r of b, corrected once by its exact remainder, is the
+// correctly rounded a / b (Markstein, IBM J. Res. Dev. 34 (1990); Cornea, Harrison & Tang,
+// Scientific Computing on Itanium-based Systems (2002), ch. 8) as long as nothing over- or
+// underflows on the way, which quot_in_range checks on the exponents; the other cases take the
+// compiler's division. That holds with the correctly rounded r; rcp_raw's is only within an ulp of it,
+// which decides wrongly where a / b lies within 2^-105 of a rounding boundary: a and b a few ulps
+// below powers of two (1 / (1 - 2^-53), root fractions summing to just below 1), so such divisors
+// (below_power) take the compiler's division as well. With the reciprocal of a divisor that is used several times (a step size, a
+// cell length) at hand the quotient costs 3 FP64 instructions, else 6 (563 cycles -> 192 / 403).
+#ifdef __CUDACC__
+__device__ __forceinline__ bool quot_in_range(double a, double b) {
+    const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+    return ((unsigned)(ea - 160) <= 1700u || to_bits(a) == 0) && (unsigned)(eb - 160) <= 1700u &&
+           ((unsigned)(ea - eb + 800) <= 1600u || to_bits(a) == 0);
+}
+__device__ __forceinline__ double rcp_seed(double b) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    return r;
+}
+// 1 / b to within an ulp, b in range: the seed's relative error e is taken to e^3
+__device__ __forceinline__ double rcp_raw(double b) {
+    const double r = rcp_seed(b);
+    const double e = __fma_rn(-b, r, 1.0);
+    return __fma_rn(__fma_rn(e, e, e), r, r);
+}
+__device__ __forceinline__ double quot_raw(double a, double b, double rb) {
+    const double q = a * rb;
+    return __fma_rn(__fma_rn(-b, q, a), rb, q);
+}
+// mantissa within 16 ulps of all ones
+__device__ __forceinline__ bool below_power(double b) { return (to_bits(b) & 0x000fffffffffffffULL) >= 0x000ffffffffffff0ULL; }
+#endif
+// a / b, correctly rounded
+WF_HD double div_(double a, double b) {
+#ifdef __CUDA_ARCH__
+    if (quot_in_range(a, b) && !below_power(b)) return quot_raw(a, b, rcp_raw(b));
+#endif
+    return a / b;
+}
+// a / b, correctly rounded, with rb = 1 / b (correctly rounded or within an ulp)
+WF_HD double div_by_(double a, double b, double rb) {
+#ifdef __CUDA_ARCH__
+    if (quot_in_range(a, b)) return quot_raw(a, b, rb);
+#endif
+    (void)rb;
+    return a / b;
+}
 
 constexpr double LN2_HI = 0x1.62e42fee00000p-1;
 constexpr double LN2_LO = 0x1.a39ef35793c76p-33;
 constexpr double INV_LN2 = 0x1.71547652b82fep+0;
 
 WF_HD double exp(double x) {
+#ifdef __CUDA_ARCH__
+    // |x| < 700: no special case, a normal result, the scaling by 2^k an exponent addition; k has 11
+    // bits and LN2_HI 33, so their product is exact and the fused subtraction rounds like the
+    // separate one. 19 FP64 instructions.
+    const bool plain = (__double2hiint(x) & 0x7fffffff) < 0x4085e000;
+    if (!plain) {
+#endif
     if (isnan_(x)) return x;
     if (x > 709.782712893384) return from_bits(0x7ff0000000000000ULL);
     if (x < -745.1332191019412) return 0.0;
+#ifdef __CUDA_ARCH__
+    }
+    const double k = rint(x * INV_LN2);
+    const double r = __fma_rn(-k, LN2_HI, x) - k * LN2_LO;
+#else
     const double k = rint_(x * INV_LN2);
     const double r = (x - k * LN2_HI) - k * LN2_LO;
+#endif
     double p = 0x1.6124613a86d09p-33;            // 1/13!
     p = fma_(p, r, 0x1.1eed8eff8d898p-29);       // 1/12!
     p = fma_(p, r, 0x1.ae64567f544e4p-26);       // 1/11!
@@ -138,12 +285,46 @@ WF_HD double exp(double x) {
     p = fma_(p, r, 1.0);
     p = fma_(p, r, 1.0);
     const int ki = (int)k;
+#ifdef __CUDA_ARCH__
+    if (plain) return from_bits(to_bits(p) + ((uint64_t)(int64_t)ki << 52));
+#endif
     if (ki > 1023) return p * 0x1p1023 * from_bits((uint64_t)ki << 52);
     if (ki < -1022) return (p * from_bits((uint64_t)(ki + 1022 + 1023) << 52)) * 0x1p-1022;
     return p * from_bits((uint64_t)(ki + 1023) << 52);
 }
 
 WF_HD double log(double x) {
+#ifdef __CUDA_ARCH__
+    // A positive normal x: classification, scaling by powers of two and the choice of m on the
+    // integer pipe, s by the 6-instruction division (f = 0 for x a power of two: s = 0), the exact
+    // product e LN2_HI fused into the last addition. 28 FP64 instructions.
+    const unsigned hx = (unsigned)__double2hiint(x);
+    if (hx - 0x00100000u < 0x7fe00000u) {
+        const bool up = (to_bits(x) & 0x000fffffffffffffULL) > 0x6a09e667f3bcdULL;
+        const int ex = (int)(hx >> 20) - 1023 + (up ? 1 : 0);
+        const double mx = from_bits((to_bits(x) & 0x000fffffffffffffULL) | (up ? 0x3fe0000000000000ULL : 0x3ff0000000000000ULL));
+        const double f = mx - 1.0;
+        const double b = 2.0 + f;
+        const double s = below_power(b) ? f / b : quot_raw(f, b, rcp_raw(b));
+        const double s2 = s * s;
+        double R = 0x1.8618618618618p-4;
+        R = __fma_rn(R, s2, 0x1.af286bca1af28p-4);
+        R = __fma_rn(R, s2, 0x1.e1e1e1e1e1e1ep-4);
+        R = __fma_rn(R, s2, 0x1.1111111111111p-3);
+        R = __fma_rn(R, s2, 0x1.3b13b13b13b14p-3);
+        R = __fma_rn(R, s2, 0x1.745d1745d1746p-3);
+        R = __fma_rn(R, s2, 0x1.c71c71c71c71cp-3);
+        R = __fma_rn(R, s2, 0x1.2492492492492p-2);
+        R = __fma_rn(R, s2, 0x1.999999999999ap-2);
+        R = __fma_rn(R, s2, 0x1.5555555555555p-1);
+        R = R * s2;
+        const uint64_t ff = to_bits(f * f);  // (f f) / 2 = (f / 2) f: |f| is 0 or at least 2^-53
+        const double hfsq = from_bits(ff != 0 ? ff - 0x0010000000000000ULL : 0);
+        const double lm = f - (hfsq - s * (hfsq + R));
+        const double de = (double)ex;
+        return __fma_rn(de, LN2_HI, lm + de * LN2_LO);
+    }
+#endif
     if (isnan_(x) || x < 0.0) return from_bits(0x7ff8000000000000ULL);
     if (x == 0.0) return -from_bits(0x7ff0000000000000ULL);
     if (x == from_bits(0x7ff0000000000000ULL)) return x;
@@ -197,7 +378,7 @@ WF_HD double cbrt(double x) {
     if (r == 1) m *= 2.0;
     if (r == 2) m *= 4.0;
     double y = 0.6 + 0.2 * m;
-    for (int i = 0; i < 6; ++i) y = y - (y * y * y - m) / (3.0 * y * y);
+    for (int i = 0; i < 6; ++i) y = y - div_(y * y * y - m, 3.0 * y * y);
     y = y * from_bits((uint64_t)(q + 1023) << 52);
     return x < 0.0 ? -y : y;
 }
@@ -207,6 +388,19 @@ WF_HD double pow(double x, double y) { return exp(y * log(x)); }
 
 // Base.div(x, y, RoundUp) (cld) for y > 0
 WF_HD double cld(double x, double y) {
+#ifdef __CUDA_ARCH__
+    // The smallest integer n with n y >= x: the rounded quotient's ceiling, moved by the sign of the
+    // remainders, which a fused multiply-add gives exactly.
+    if (gt0_(x) && quot_in_range(x, y)) {
+        const double q = quot_raw(x, y, rcp_raw(y));
+        if ((__double2hiint(q) & 0x7fffffff) < 0x41300000) {  // q < 2^20
+            const double n = ::ceil(q);
+            if (gt0_(__fma_rn(-n, y, x))) return n + 1.0;
+            if (le0_(__fma_rn(-(n - 1.0), y, x))) return n - 1.0;
+            return n;
+        }
+    }
+#endif
     const double r = fmod_(x, -y);
     double m;
     if (r == 0.0) {
