@@ -158,7 +158,8 @@ __device__ bool li_grid_sync(LiLoop* s) {
             atomicAdd(&s->gen, 1u);
         } else {
             const uint64_t t0 = li_now_ns();
-            while (*gen == g) {
+            for (int spin = 0; *gen == g; ++spin) {
+                if (spin < 64) continue;  // a phase lasts a few microseconds: poll without sleeping first
                 __nanosleep(32);
                 if (*(volatile int*)&s->status) {
                     ok = 0;
@@ -178,24 +179,41 @@ __device__ bool li_grid_sync(LiLoop* s) {
     return ok_s != 0;
 }
 
-// Block minimum of the non-NaN candidates into minbits[p][w] (the bit patterns of non-negative
-// doubles order as the values), and the NaN flag.
-__device__ void li_reduce_min(LiLoop* s, int p, int w, double m, bool nan) {
-    __shared__ double red[32];
-    __shared__ int nan_s;
-    if (threadIdx.x == 0) nan_s = 0;
-    __syncthreads();
+// Block maximum of an FP32 rank (every thread gets it).
+__device__ float li_block_max(float v) {
+    __shared__ float red[32];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, off));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    if (nan) nan_s = 1;
+    for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double b = red[0];
-        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) b = fmin(b, red[k]);
-        atomicMin(&s->minbits[p][w], (unsigned long long)__double_as_longlong(b));
-        if (nan_s) atomicOr(&s->nanflag[p][w], 1);
-    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) v = fmaxf(v, red[k]);
+    return v;
+}
+
+// A candidate of the grid's minimum stable sub-step into minbits[p][w] (the bit patterns of
+// non-negative doubles order as the values), a NaN into the flag.
+__device__ __forceinline__ void li_offer_min(LiLoop* s, int p, int w, double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    if (wfm::isnan_(v)) atomicOr(&s->nanflag[p][w], 1);
+    else if (b < *(volatile unsigned long long*)&s->minbits[p][w]) atomicMin(&s->minbits[p][w], b);
+}
+
+// The stable sub-steps of the cells tid, tid + nt, ... into minbits[p][w]. A square root and a
+// division per cell are 20 FP64 instructions, as much as the depth update itself, and only the
+// smallest is needed: the cells are ranked in FP32 first (`rank`, by the caller, in its update
+// loop: the thread's largest), and only those within 1e-5 of the block's largest rank, usually one,
+// are computed. Every cell of the block that could hold its minimum is among them. Below 1e-30 (a
+// domain all but dry) the ranks lose their precision and every cell is computed.
+template <class Rank, class Step>
+__device__ __forceinline__ void li_min_timestep(LiLoop* s, int p, int w, float rank, int64_t tid, int64_t nt, int64_t n,
+                                                Rank rank_of, Step step_of) {
+    const float top = li_block_max(rank);
+    const float least = top > 1e-30f ? top * 0.99999f : 0.0f;
+    if (!(rank >= least)) return;
+    for (int64_t i = tid; i < n; i += nt)
+        if (rank_of(i) >= least) li_offer_min(s, p, w, step_of(i));
 }
 
 __device__ __forceinline__ double li_read_min(LiLoop* s, int p, int w) {
@@ -216,27 +234,36 @@ __global__ void li_loop_init_kernel(LiLoop* s) {
     s->t = 0.0;
 }
 
+// The loops below end a sub-step with the cells' update and the minimum of the next sub-step's
+// stable sub-steps in one phase (two grid barriers per sub-step: edges | cells and minimum).
+constexpr float LI_NO_RANK = -1.0f;  // below every rank
+
 // the river alone (wf_li_river_step)
 __global__ void __launch_bounds__(256) li_river_loop_kernel(LiDev d, LiLoop* s, double dt) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    auto minimum = [&](int p) {
+        if (d.manning) {  // Manning: the edges' sub-steps
+            unsigned long long m = INF_BITS;
+            for (int64_t i = tid; i < d.n_edges; i += nt) {
+                const double v = wfli::edge_timestep_manning(d, i);
+                if (wfm::isnan_(v)) atomicOr(&s->nanflag[p][0], 1);
+                else m = min(m, (unsigned long long)__double_as_longlong(v));
+            }
+            for (int off = 16; off > 0; off >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, off));
+            if ((threadIdx.x & 31) == 0 && m < INF_BITS) atomicMin(&s->minbits[p][0], m);
+            return;
+        }
+        auto rank_of = [&](int64_t i) { return wfli::timestep_rank(d.h[i], d.flow_length[i]); };
+        float rank = LI_NO_RANK;
+        for (int64_t i = tid; i < d.n_dt; i += nt) rank = fmaxf(rank, rank_of(i));
+        li_min_timestep(s, p, 0, rank, tid, nt, d.n_dt, rank_of, [&](int64_t i) { return wfli::cell_timestep(d, i); });
+    };
+    minimum(0);
+    if (!li_grid_sync(s)) return;
     double t = 0.0;
     long long k = 0;
     while (t < dt) {
         const int p = (int)(k & 1);
-        double m = wfm::from_bits(INF_BITS);
-        bool nan = false;
-        const int64_t nv = d.manning ? d.n_edges : d.n_dt;  // Manning: the edges' sub-steps
-        for (int64_t i = tid; i < nv; i += nt) {
-            const double v = d.manning ? wfli::edge_timestep_manning(d, i) : wfli::cell_timestep(d, i);
-            if (v != v) nan = true;
-            else m = fmin(m, v);
-        }
-        li_reduce_min(s, p, 0, m, nan);
-        if (!li_grid_sync(s)) return;
-        if (tid == 0) {  // the other parity's slot serves the next sub-step
-            s->minbits[p ^ 1][0] = INF_BITS;
-            s->nanflag[p ^ 1][0] = 0;
-        }
         double dt_s = wfli::finish_timestep(li_read_min(s, p, 0));
         if (t + dt_s > dt) dt_s = dt - t;
         for (int64_t e = tid; e < d.n_edges; e += nt) {
@@ -244,7 +271,12 @@ __global__ void __launch_bounds__(256) li_river_loop_kernel(LiDev d, LiLoop* s, 
             else wfli::update_edge(d, e, dt_s);
         }
         if (!li_grid_sync(s)) return;
+        if (tid == 0) {  // every thread has read this parity's minimum: free it for the sub-step after next
+            s->minbits[p][0] = INF_BITS;
+            s->nanflag[p][0] = 0;
+        }
         for (int64_t i = tid; i < d.n_active; i += nt) wfli::update_cell(d, i, dt_s);
+        minimum(p ^ 1);
         t += dt_s;
         ++k;
         if (!li_grid_sync(s)) return;
@@ -265,29 +297,37 @@ __global__ void __launch_bounds__(256) li_domain_loop_kernel(wfli::LiLand L, LiD
                                                              double dt, double* qx0b, double* qx1b, double* qy0b,
                                                              double* qy1b, int cur0) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    auto land_rank = [&](int64_t i) {
+        return L.river[i] < 0 ? wfli::timestep_rank(L.h[i], wfm::jmin(L.xl[i], L.yl[i])) : LI_NO_RANK;
+    };
+    auto river_rank = [&](int64_t r) { return wfli::timestep_rank(R.h[r], R.flow_length[r]); };
+    auto minima = [&](int p, float rank_land) {
+        li_min_timestep(s, p, 1, rank_land, tid, nt, L.n, land_rank,
+                        [&](int64_t i) { return wfli::land_timestep(L, i); });
+    };
+    // the river minimum over the river cells of this thread's land cells, which it has just updated
+    auto river_minima = [&](int p, float rank_river) {
+        auto rank_of = [&](int64_t i) {
+            const int64_t r = L.river[i];
+            return r >= 0 && r < R.n_dt ? river_rank(r) : LI_NO_RANK;
+        };
+        li_min_timestep(s, p, 0, rank_river, tid, nt, L.n, rank_of,
+                        [&](int64_t i) { return wfli::cell_timestep(R, L.river[i]); });
+    };
+    auto ranks = [&](int64_t i, float& land, float& river) {
+        const int64_t r = L.river[i];
+        if (r < 0) land = fmaxf(land, wfli::timestep_rank(L.h[i], wfm::jmin(L.xl[i], L.yl[i])));
+        else if (r < R.n_dt) river = fmaxf(river, river_rank(r));
+    };
+    float rank_land = LI_NO_RANK, rank_river = LI_NO_RANK;
+    for (int64_t i = tid; i < L.n; i += nt) ranks(i, rank_land, rank_river);
+    minima(0, rank_land);
+    river_minima(0, rank_river);
+    if (!li_grid_sync(s)) return;
     double t = 0.0;
     long long k = 0;
     while (t < dt) {
         const int p = (int)(k & 1);
-        double mr = wfm::from_bits(INF_BITS), ml = wfm::from_bits(INF_BITS);
-        bool nr = false, nl = false;
-        for (int64_t i = tid; i < R.n_dt; i += nt) {
-            const double v = wfli::cell_timestep(R, i);
-            if (v != v) nr = true;
-            else mr = fmin(mr, v);
-        }
-        for (int64_t i = tid; i < L.n; i += nt) {
-            const double v = wfli::land_timestep(L, i);
-            if (v != v) nl = true;
-            else ml = fmin(ml, v);
-        }
-        li_reduce_min(s, p, 0, mr, nr);
-        li_reduce_min(s, p, 1, ml, nl);
-        if (!li_grid_sync(s)) return;
-        if (tid == 0) {
-            s->minbits[p ^ 1][0] = s->minbits[p ^ 1][1] = INF_BITS;
-            s->nanflag[p ^ 1][0] = s->nanflag[p ^ 1][1] = 0;
-        }
         const double dt_river = wfli::finish_timestep(li_read_min(s, p, 0));
         const double dt_land = wfli::finish_timestep(li_read_min(s, p, 1));
         double dt_s = wfm::jmin(dt_river, dt_land);
@@ -301,9 +341,20 @@ __global__ void __launch_bounds__(256) li_domain_loop_kernel(wfli::LiLand L, LiD
             wfli::land_direction(L, i, dt_s, true);
             wfli::land_direction(L, i, dt_s, false);
         }
-        for (int64_t e = tid; e < R.n_edges; e += nt) wfli::update_edge(R, e, dt_s);
+        // the river edges from the last thread down: those have fewer land cells when the last round is ragged
+        for (int64_t e = nt - 1 - tid; e < R.n_edges; e += nt) wfli::update_edge(R, e, dt_s);
         if (!li_grid_sync(s)) return;
-        for (int64_t i = tid; i < L.n; i += nt) wfli::land_depth(L, R, B, i, dt_s);
+        if (tid == 0) {  // every thread has read this parity's minima
+            s->minbits[p][0] = s->minbits[p][1] = INF_BITS;
+            s->nanflag[p][0] = s->nanflag[p][1] = 0;
+        }
+        rank_land = rank_river = LI_NO_RANK;
+        for (int64_t i = tid; i < L.n; i += nt) {
+            wfli::land_depth(L, R, B, i, dt_s);
+            ranks(i, rank_land, rank_river);
+        }
+        minima(p ^ 1, rank_land);
+        river_minima(p ^ 1, rank_river);
         t += dt_s;
         ++k;
         if (!li_grid_sync(s)) return;
@@ -318,15 +369,19 @@ __global__ void __launch_bounds__(256) li_domain_loop_kernel(wfli::LiLand L, LiD
     }
 }
 
-// Blocks of a cooperative loop launch: every block resident (occupancy x SMs), no more than the
-// work needs.
+// Launch shape of a cooperative loop: every block resident (occupancy x SMs), no more than the work
+// needs. Work that leaves SMs idle with blocks of 256 threads takes smaller blocks: each scheduler
+// issues an FP64 instruction per 64 cycles, so 6000 edges in 24 blocks wait for 2 warps per
+// scheduler while 128 SMs idle, in 94 blocks of 64 for one.
 template <class Kernel>
-int li_loop_blocks(Kernel kernel, int device, int64_t work) {
+int li_loop_blocks(Kernel kernel, int device, int64_t work, int& threads) {
     int per_sm = 0, sms = 0, coop = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return 0;
-    const int64_t need = (work + 255) / 256;
+    threads = 256;
+    while (threads > 32 && (work + threads - 1) / threads < sms) threads >>= 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess) return 0;
+    const int64_t need = (work + threads - 1) / threads;
     int64_t b = (int64_t)per_sm * sms;
     if (b > need) b = need;
     return (int)(b < 1 ? 1 : b);
@@ -470,6 +525,15 @@ int li_upload_river(LiOwner* o, LiDev& d, int64_t n, int64_t n_active, int64_t n
         (rc = li_upload<double>(o, &d.dt_min, nullptr, 1)) || (rc = li_upload<double>(o, &d.error, nullptr, n)) ||
         (rc = li_upload<double>(o, &d.abstraction_cum, nullptr, n)))
         return rc;
+    std::vector<double> rlen(n_edges), rplan(n, 0.0);
+    for (int64_t k = 0; k < n_edges; ++k) rlen[k] = 1.0 / length_edge[k];
+    for (int64_t i = 0; i < n_active; ++i) rplan[i] = 1.0 / (flow_length[i] * flow_width[i]);
+    double *p_rlen, *p_rplan;
+    if ((rc = li_upload(o, &p_rlen, (const double*)rlen.data(), n_edges)) ||
+        (rc = li_upload(o, &p_rplan, (const double*)rplan.data(), n)))
+        return rc;
+    d.rlen_e = p_rlen;
+    d.rplan = p_rplan;
     double *p_abs, *p_ext;
     if ((rc = li_upload<double>(o, &p_abs, nullptr, n)) || (rc = li_upload<double>(o, &p_ext, nullptr, n))) return rc;
     d.abstraction = p_abs;
@@ -630,15 +694,16 @@ int32_t wf_li_river_step(WfLiRiver* r, double dt, int64_t* substeps) {
          cudaMemsetAsync(r->d.q_cum, 0, r->d.n_edges * sizeof(double), r->stream) != cudaSuccess) ||
         cudaMemsetAsync(r->d.abstraction_cum, 0, r->d.n * sizeof(double), r->stream) != cudaSuccess)
         return li_fail(r, WF_ERR_CUDA, "reset of the cumulative discharge failed");
+    int threads = 0;
     const int blocks = r->host_loop ? 0 : li_loop_blocks(li_river_loop_kernel, r->device,
-                                                          std::max(r->d.n, r->d.n_edges));
+                                                          std::max(r->d.n, r->d.n_edges), threads);
     if (blocks > 0) {  // the sub-step loop on the device, one launch
         li_loop_init_kernel<<<1, 1, 0, r->stream>>>(r->loop);
         LiDev dd = r->d;
         LiLoop* lp = r->loop;
         double dtv = dt;
         void* args[] = {&dd, &lp, &dtv};
-        if (cudaLaunchCooperativeKernel((const void*)li_river_loop_kernel, blocks, 256, args, 0, r->stream) !=
+        if (cudaLaunchCooperativeKernel((const void*)li_river_loop_kernel, blocks, threads, args, 0, r->stream) !=
             cudaSuccess)
             return li_fail(r, WF_ERR_CUDA, "cooperative launch of the sub-step loop failed");
         if (r->d.n_edges > 0)
@@ -735,6 +800,13 @@ int32_t wf_li_domain_create(const WfLiLandGrid* land, const WfLiRiverNetwork* ri
     wfli::land_edge_parameters(n, ld.ind_x_up, ld.ind_y_up, ld.elevation, zx_max, zy_max);
     wfli::bankfull_storage(rv.n, rv.bankfull_depth, rv.flow_width, rv.flow_length, bankfull);
 
+    std::vector<double> rlx(n, 0.0), rly(n, 0.0), rarea(n);
+    for (int64_t i = 0; i < n; ++i) {
+        if (ld.ind_x_up[i] < n) rlx[i] = 1.0 / (0.5 * (ld.x_length[i] + ld.x_length[ld.ind_x_up[i]]));
+        if (ld.ind_y_up[i] < n) rly[i] = 1.0 / (0.5 * (ld.y_length[i] + ld.y_length[ld.ind_y_up[i]]));
+        rarea[i] = 1.0 / (ld.x_length[i] * ld.y_length[i]);
+    }
+
     WfLiDomain* d = new WfLiDomain();
     wfli::LiLand& L = d->L;
     L.n = n;
@@ -743,7 +815,8 @@ int32_t wf_li_domain_create(const WfLiLandGrid* land, const WfLiRiverNetwork* ri
     L.alpha = ld.alpha;
     L.froude = ld.froude_limit;
     int64_t *p_ixu, *p_ixd, *p_iyu, *p_iyd, *p_riv;
-    double *p_xl, *p_yl, *p_z, *p_nsq, *p_xw, *p_yw, *p_zx, *p_zy, *p_bd, *p_bs;
+    double *p_xl, *p_yl, *p_z, *p_nsq, *p_xw, *p_yw, *p_zx, *p_zy, *p_bd, *p_bs, *p_rlx, *p_rly, *p_ra;
+    const double *c_rlx = rlx.data(), *c_rly = rly.data(), *c_ra = rarea.data();
     const double *c_zx = zx_max.data(), *c_zy = zy_max.data(), *c_bs = bankfull.data();
     if ((rc = li_open(d, device)) ||
         (rc = li_upload_river(d, d->R, rv.n, rv.n_active, rv.n_edges, rv.src, rv.dst, rv.zb, rv.flow_length,
@@ -756,7 +829,9 @@ int32_t wf_li_domain_create(const WfLiLandGrid* land, const WfLiRiverNetwork* ri
         (rc = li_upload(d, &p_nsq, ld.mannings_n_sq, n)) || (rc = li_upload(d, &p_xw, ld.xwidth_at_edge, n)) ||
         (rc = li_upload(d, &p_yw, ld.ywidth_at_edge, n)) || (rc = li_upload(d, &p_zx, c_zx, n)) ||
         (rc = li_upload(d, &p_zy, c_zy, n)) || (rc = li_upload(d, &p_bd, rv.bankfull_depth, rv.n)) ||
-        (rc = li_upload(d, &p_bs, c_bs, rv.n)) || (rc = li_upload<double>(d, &d->runoff, nullptr, n)) ||
+        (rc = li_upload(d, &p_bs, c_bs, rv.n)) ||
+        (rc = li_upload(d, &p_rlx, c_rlx, n)) || (rc = li_upload(d, &p_rly, c_rly, n)) ||
+        (rc = li_upload(d, &p_ra, c_ra, n)) || (rc = li_upload<double>(d, &d->runoff, nullptr, n)) ||
         (rc = li_upload<double>(d, &d->ext, nullptr, rv.n)) ||
         (rc = li_upload<double>(d, &d->abstraction, nullptr, rv.n)) ||
         (rc = li_upload<double>(d, &d->B.abstraction_cum, nullptr, rv.n)) ||
@@ -790,6 +865,9 @@ int32_t wf_li_domain_create(const WfLiLandGrid* land, const WfLiRiverNetwork* ri
     L.yw = p_yw;
     L.zx_max = p_zx;
     L.zy_max = p_zy;
+    L.rlx = p_rlx;
+    L.rly = p_rly;
+    L.rarea = p_ra;
     L.runoff = d->runoff;
     d->B.bankfull_depth = p_bd;
     d->B.bankfull_storage = p_bs;
@@ -875,7 +953,7 @@ int32_t wf_li_domain_substep(WfLiDomain* d, double dt_s) {
 namespace {
 // set_flow_vars! of the river and the land (:1165-1166), the device sub-step loop (one
 // cooperative launch) and the averages, on stream st; 0 blocks when the device cannot run it.
-int li_domain_launch(WfLiDomain* d, double dt, cudaStream_t st, int blocks) {
+int li_domain_launch(WfLiDomain* d, double dt, cudaStream_t st, int blocks, int threads) {
     const int64_t n = d->L.n, ne = d->R.n_edges;
     if ((ne > 0 && cudaMemsetAsync(d->R.q_cum, 0, ne * sizeof(double), st) != cudaSuccess) ||
         cudaMemsetAsync(d->B.abstraction_cum, 0, d->R.n * sizeof(double), st) != cudaSuccess ||
@@ -891,7 +969,7 @@ int li_domain_launch(WfLiDomain* d, double dt, cudaStream_t st, int blocks) {
     double *qx0b = d->qx_buf[0], *qx1b = d->qx_buf[1], *qy0b = d->qy_buf[0], *qy1b = d->qy_buf[1];
     int cur0 = d->cur;
     void* args[] = {&LL, &RR, &BB, &lp, &dtv, &qx0b, &qx1b, &qy0b, &qy1b, &cur0};
-    if (cudaLaunchCooperativeKernel((const void*)li_domain_loop_kernel, blocks, 256, args, 0, st) != cudaSuccess)
+    if (cudaLaunchCooperativeKernel((const void*)li_domain_loop_kernel, blocks, threads, args, 0, st) != cudaSuccess)
         return li_fail(d, WF_ERR_CUDA, "cooperative launch of the sub-step loop failed");
     if (ne > 0) li_average_kernel<<<grid_of(ne), 256, 0, st>>>(d->R.q_cum, d->q_avg, ne, dt);
     li_average_kernel<<<grid_of(n + 1), 256, 0, st>>>(d->L.qx_cum, d->qx_avg, n + 1, dt);
@@ -899,18 +977,19 @@ int li_domain_launch(WfLiDomain* d, double dt, cudaStream_t st, int blocks) {
     return li_check(d, "sub-step loop");
 }
 
-int li_domain_blocks(WfLiDomain* d) {
+int li_domain_blocks(WfLiDomain* d, int& threads) {
     const int64_t n = d->L.n, ne = d->R.n_edges;
-    return li_loop_blocks(li_domain_loop_kernel, d->device, std::max(std::max(n + 1, d->R.n), ne));
+    return li_loop_blocks(li_domain_loop_kernel, d->device, std::max(std::max(n + 1, d->R.n), ne), threads);
 }
 }  // namespace
 
 int32_t wf_li_domain_step(WfLiDomain* d, double dt, int64_t* substeps) {
     if (!d || !(dt > 0.0)) return li_fail(d, WF_ERR_INVALID, "step must be positive");
     const int64_t n = d->L.n, ne = d->R.n_edges;
-    const int blocks = d->host_loop ? 0 : li_domain_blocks(d);
+    int threads = 0;
+    const int blocks = d->host_loop ? 0 : li_domain_blocks(d, threads);
     if (blocks > 0) {  // the sub-step loop on the device, one launch
-        int rc = li_domain_launch(d, dt, d->stream, blocks);
+        int rc = li_domain_launch(d, dt, d->stream, blocks, threads);
         if (rc) return rc;
         int64_t k = 0;
         rc = li_finish_loop(d, &k);
@@ -1006,9 +1085,10 @@ int wf_li_domain_couple_view(WfLiDomain* d, WfLiCoupleView* v, const int64_t** r
 
 int wf_li_domain_enqueue_step(WfLiDomain* d, double dt, cudaStream_t stream) {
     if (!d || !(dt > 0.0)) return WF_ERR_INVALID;
-    const int blocks = li_domain_blocks(d);
+    int threads = 0;
+    const int blocks = li_domain_blocks(d, threads);
     if (blocks <= 0) return li_fail(d, WF_ERR_UNSUPPORTED, "the device cannot run the cooperative sub-step loop");
-    return li_domain_launch(d, dt, stream, blocks);
+    return li_domain_launch(d, dt, stream, blocks, threads);
 }
 
 int wf_li_domain_complete_step(WfLiDomain* d, int64_t* substeps, const char** err) {

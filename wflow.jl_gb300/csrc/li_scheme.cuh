@@ -14,6 +14,12 @@
 
 #include "wf_math.cuh"
 
+// On the device the loops are bound by the FP64 pipe (64 cycles per warp and instruction, see
+// wf_math.cuh), not by memory. The results stay the host's bit for bit, with fewer FP64 instructions:
+// divisions by lengths and areas through reciprocals laid down at create, the other divisions in 6
+// instructions, comparisons on the integer pipe, and the Froude number, which only decides whether
+// the flow is limited, in FP32 unless it is within 0.01 % of 1 (three divisions, a square root).
+
 namespace wfli {
 
 constexpr double GRAVITY = 9.80665;  // Wflow.GRAVITATIONAL_ACCELERATION (Wflow.jl:77)
@@ -37,19 +43,38 @@ struct LiNet {
     int32_t manning;
     const double *slope_e, *n_e;
     double* hf_e;
+    const double *rlen_e, *rplan;  // device: 1 / length_e per edge, 1 / (length width) per cell
 };
 
 constexpr double BETA_KINWAVE = 0.6;  // Wflow.BETA_KINWAVE (routing/surface/surface_kinwave.jl:2)
 
-// local_inertial_flow for a general cross-section of area A and hydraulic radius R
-WF_HD double flow(double q0, double zs0, double zs1, double hf, double A, double R, double length, double nsq,
-                  bool froude, double dt) {
-    const double slope = (zs1 - zs0) / length;
+// Whether the Froude number |q| / (A sqrt(g hf)) of a discharge is above 1, as far as FP32 can tell
+// (relative error 3e-7): 1 yes, 0 no, -1 too close to say. -1 on the host.
+WF_HD int supercritical(double q, double A, double hf) {
+#ifdef __CUDA_ARCH__
+    const float a = fabsf(wfm::f32_of(q)), c = sqrtf((float)GRAVITY * wfm::f32_of(hf)) * wfm::f32_of(A);
+    if (a > c * 1.0001f) return 1;
+    if (a < c * 0.9999f) return 0;
+#endif
+    return -1;
+}
+
+// local_inertial_flow for a general cross-section of area A and hydraulic radius R; rlen = 1 / length
+// (device)
+WF_HD double flow(double q0, double zs0, double zs1, double hf, double A, double R, double length, double rlen,
+                  double nsq, bool froude, double dt) {
+    const double slope = wfm::div_by_(zs1 - zs0, length, rlen);
     const double pow_R = wfm::cbrt(R * R * R * R);
-    double q = (q0 - GRAVITY * A * dt * slope) / (1.0 + GRAVITY * dt * nsq * wfm::fabs_(q0) / (pow_R * A));
-    const double fr = ((q / A) / wfm::sqrt_(GRAVITY * hf)) * (froude ? 1.0 : 0.0);
-    if (wfm::fabs_(fr) > 1.0 && q > 0.0) q = wfm::sqrt_(GRAVITY * hf) * A;
-    if (wfm::fabs_(fr) > 1.0 && q < 0.0) q = -wfm::sqrt_(GRAVITY * hf) * A;
+    double q = wfm::div_(q0 - GRAVITY * A * dt * slope,
+                         1.0 + wfm::div_(GRAVITY * dt * nsq * wfm::fabs_(q0), pow_R * A));
+    if (!froude) return q;
+    const int above = supercritical(q, A, hf);
+    if (above == 0) return q;
+    const double c = wfm::sqrt_(GRAVITY * hf);
+    if (above > 0 || wfm::gt_(wfm::fabs_(wfm::div_(wfm::div_(q, A), c)), 1.0)) {
+        if (wfm::gt0_(q)) q = c * A;
+        else if (wfm::lt_(q, 0.0)) q = -c * A;
+    }
     return q;
 }
 
@@ -64,12 +89,18 @@ WF_HD void update_edge(const LiNet& d, int64_t k, double dt) {
     const double zs_e = wfm::jmax(zs_src, zs_dst);
     const double hf = zs_e - d.zb_e[k];
     const double A = d.width_e[k] * hf;
-    const double R = A / (2.0 * hf + d.width_e[k]);
-    double q = hf > d.h_thresh
-                   ? flow(q_prev, zs_src, zs_dst, hf, A, R, d.length_e[k], d.nsq_e[k], d.froude != 0, dt)
-                   : 0.0;
-    if (d.h[a] <= 0.0) q = wfm::jmin(q, 0.0);
-    if (d.h[b] <= 0.0) q = wfm::jmax(q, 0.0);
+    double q = 0.0;
+    if (wfm::gt_(hf, d.h_thresh)) {
+        const double R = wfm::div_(A, 2.0 * hf + d.width_e[k]);
+#ifdef __CUDA_ARCH__
+        const double rlen = d.rlen_e[k];
+#else
+        const double rlen = 0.0;
+#endif
+        q = flow(q_prev, zs_src, zs_dst, hf, A, R, d.length_e[k], rlen, d.nsq_e[k], d.froude != 0, dt);
+    }
+    if (wfm::le0_(d.h[a])) q = wfm::jmin(q, 0.0);
+    if (wfm::le0_(d.h[b])) q = wfm::jmax(q, 0.0);
     d.q[k] = q;
     d.q_cum[k] += q * dt;
 }
@@ -107,25 +138,29 @@ WF_HD void update_cell(const LiNet& d, int64_t i, double dt) {
     for (int64_t o = d.in_ptr[i]; o < d.in_ptr[i + 1]; ++o) qin = qin + d.q[d.in_edge[o]];
     for (int64_t o = d.out_ptr[i]; o < d.out_ptr[i + 1]; ++o) qout = qout + d.q[d.out_edge[o]];
     double s = d.storage[i] + (qin - qout + d.inwater[i] - d.abstraction[i]) * dt;
-    if (s < 0.0) {
+    if (wfm::lt_(s, 0.0)) {
         d.error[i] = d.error[i] + wfm::fabs_(s);
         s = 0.0;
     }
     const double ext = d.external_inflow[i];
     double inflow = ext;
-    if (ext < 0.0) {
-        const double taken = wfm::jmin(-ext, s / dt * 0.80);
+    if (wfm::lt_(ext, 0.0)) {
+        const double taken = wfm::jmin(-ext, wfm::div_(s, dt) * 0.80);
         d.abstraction_cum[i] += taken * dt;
         inflow = -taken;
     }
-    s += inflow * dt;
+    if (!wfm::is_zero_(inflow)) s += inflow * dt;
     d.storage[i] = s;
+#ifdef __CUDA_ARCH__
+    d.h[i] = wfm::div_by_(s, d.flow_length[i] * d.flow_width[i], d.rplan[i]);
+#else
     d.h[i] = s / (d.flow_length[i] * d.flow_width[i]);
+#endif
 }
 
 // the stable sub-step of cell i (inf for a dry cell)
 WF_HD double cell_timestep(const LiNet& d, int64_t i) {
-    return d.alpha * d.flow_length[i] / wfm::sqrt_(GRAVITY * d.h[i]);
+    return wfm::div_(d.alpha * d.flow_length[i], wfm::sqrt_(GRAVITY * d.h[i]));
 }
 
 // min over cells of the stable sub-step, 60 s when it is infinite (every cell dry)
@@ -149,6 +184,8 @@ struct LiLand {
     double *qx, *qy, *qx_cum, *qy_cum, *dt_min;
     double theta, h_thresh, alpha;
     int32_t froude;
+    // device: 1 / the edge lengths in x and y (0 without an upstream cell), 1 / the cell's area
+    const double *rlx, *rly, *rarea;
 };
 
 // Per river cell boundary data of the coupled scheme.
@@ -158,19 +195,20 @@ struct LiRiverBC {
 };
 
 // local_inertial_flow, rectangular cross-section with the theta weighting
-// (surface_process.jl:124-163)
+// (surface_process.jl:124-163); rlen = 1 / length (device)
 WF_HD double flow_rect(double theta, double q0, double qd, double qu, double zs0, double zs1, double hf, double width,
-                       double length, double nsq, bool froude, double dt) {
-    const double slope = (zs1 - zs0) / length;
+                       double length, double rlen, double nsq, bool froude, double dt) {
+    const double slope = wfm::div_by_(zs1 - zs0, length, rlen);
     const double pow_hf = wfm::cbrt(hf * hf * hf * hf * hf * hf * hf);
-    double q = ((theta * q0 + 0.5 * (1.0 - theta) * (qu + qd)) - GRAVITY * hf * width * dt * slope) /
-               (1.0 + GRAVITY * dt * nsq * wfm::fabs_(q0) / (pow_hf * width));
-    if (froude) {
-        const double fr = (q / width / hf) / wfm::sqrt_(GRAVITY * hf);
-        if (wfm::fabs_(fr) > 1.0 && q > 0.0)
-            q = hf * wfm::sqrt_(GRAVITY * hf) * width;
-        else if (wfm::fabs_(fr) > 1.0 && q < 0.0)
-            q = -hf * wfm::sqrt_(GRAVITY * hf) * width;
+    double q = wfm::div_((theta * q0 + 0.5 * (1.0 - theta) * (qu + qd)) - GRAVITY * hf * width * dt * slope,
+                         1.0 + wfm::div_(GRAVITY * dt * nsq * wfm::fabs_(q0), pow_hf * width));
+    if (!froude) return q;
+    const int above = supercritical(q, width * hf, hf);
+    if (above == 0) return q;
+    const double c = wfm::sqrt_(GRAVITY * hf);
+    if (above > 0 || wfm::gt_(wfm::fabs_(wfm::div_(wfm::div_(wfm::div_(q, width), hf), c)), 1.0)) {
+        if (wfm::gt0_(q)) q = hf * c * width;
+        else if (wfm::lt_(q, 0.0)) q = -hf * c * width;
     }
     return q;
 }
@@ -193,12 +231,17 @@ WF_HD void land_direction(const LiLand& L, int64_t i, double dt, bool x_dir) {
     const double zs_max = wfm::jmax(zs_current, zs_upstream);
     const double hf = zs_max - (x_dir ? L.zx_max[i] : L.zy_max[i]);
     double qi = 0.0;
-    if (hf > L.h_thresh) {
+    if (wfm::gt_(hf, L.h_thresh)) {
         const double length_e = 0.5 * (len[i] + len[u]);
-        qi = flow_rect(L.theta, q0[i], q0[dn], q0[u], zs_current, zs_upstream, hf, width, length_e, L.nsq[i],
+#ifdef __CUDA_ARCH__
+        const double rlen = x_dir ? L.rlx[i] : L.rly[i];
+#else
+        const double rlen = 0.0;
+#endif
+        qi = flow_rect(L.theta, q0[i], q0[dn], q0[u], zs_current, zs_upstream, hf, width, length_e, rlen, L.nsq[i],
                        L.froude != 0, dt);
-        if (L.h[i] <= 0.0) qi = wfm::jmin(qi, 0.0);
-        if (L.h[u] <= 0.0) qi = wfm::jmax(qi, 0.0);
+        if (wfm::le0_(L.h[i])) qi = wfm::jmin(qi, 0.0);
+        if (wfm::le0_(L.h[u])) qi = wfm::jmax(qi, 0.0);
     }
     q[i] = qi;
     (x_dir ? L.qx_cum : L.qy_cum)[i] += qi * dt;
@@ -213,12 +256,16 @@ WF_HD void land_depth(const LiLand& L, const LiNet& R, const LiRiverBC& B, int64
     const int64_t xd = L.ixd[i], yd = L.iyd[i];
     if (r < 0) {
         double s = L.storage[i] + (L.qx[xd] - L.qx[i] + L.qy[yd] - L.qy[i] + L.runoff[i]) * dt;
-        if (s < 0.0) {
+        if (wfm::lt_(s, 0.0)) {
             L.error[i] += wfm::fabs_(s);
             s = 0.0;
         }
         L.storage[i] = s;
+#ifdef __CUDA_ARCH__
+        L.h[i] = wfm::div_by_(s, L.xl[i] * L.yl[i], L.rarea[i]);
+#else
         L.h[i] = s / (L.xl[i] * L.yl[i]);
+#endif
         return;
     }
     double s_in = 0.0, s_out = 0.0;
@@ -228,27 +275,31 @@ WF_HD void land_depth(const LiLand& L, const LiNet& R, const LiRiverBC& B, int64
     const double net_land = L.qx[xd] - L.qx[i] + L.qy[yd] - L.qy[i];
     const double net = net_river + net_land + L.runoff[i] - B.abstraction[r];
     double s = L.storage[i] + net * dt;
-    if (s < 0.0) {
+    if (wfm::lt_(s, 0.0)) {
         L.error[i] += wfm::fabs_(s);
         s = 0.0;
     }
     const double ext = B.external_inflow[r];
     double inflow = ext, taken = 0.0;
-    if (ext < 0.0) {
-        const double available = s >= B.bankfull_storage[r] ? B.bankfull_storage[r] : R.storage[r];
-        taken = wfm::jmin(-ext, available / dt * 0.80);
+    if (wfm::lt_(ext, 0.0)) {
+        const double available = wfm::le_(B.bankfull_storage[r], s) ? B.bankfull_storage[r] : R.storage[r];
+        taken = wfm::jmin(-ext, wfm::div_(available, dt) * 0.80);
         inflow = -taken;
+        B.abstraction_cum[r] += taken * dt;
     }
-    s += inflow * dt;
-    B.abstraction_cum[r] += taken * dt;
+    if (!wfm::is_zero_(inflow)) s += inflow * dt;
     L.storage[i] = s;
-    if (s >= B.bankfull_storage[r]) {
-        const double river_h = B.bankfull_depth[r] + (s - B.bankfull_storage[r]) / (L.xl[i] * L.yl[i]);
+    if (wfm::le_(B.bankfull_storage[r], s)) {
+        const double river_h = B.bankfull_depth[r] + wfm::div_(s - B.bankfull_storage[r], L.xl[i] * L.yl[i]);
         R.h[r] = river_h;
         L.h[i] = river_h - B.bankfull_depth[r];
         R.storage[r] = river_h * R.flow_length[r] * R.flow_width[r];
     } else {
+#ifdef __CUDA_ARCH__
+        R.h[r] = wfm::div_by_(s, R.flow_length[r] * R.flow_width[r], R.rplan[r]);
+#else
         R.h[r] = s / (R.flow_length[r] * R.flow_width[r]);
+#endif
         L.h[i] = 0.0;
         R.storage[r] = s;
     }
@@ -256,9 +307,19 @@ WF_HD void land_depth(const LiLand& L, const LiNet& R, const LiRiverBC& B, int64
 
 // the stable sub-step of land cell i: cells without a river only (:1022-1040)
 WF_HD double land_timestep(const LiLand& L, int64_t i) {
-    return L.river[i] < 0 ? L.alpha * wfm::jmin(L.xl[i], L.yl[i]) / wfm::sqrt_(GRAVITY * L.h[i])
+    return L.river[i] < 0 ? wfm::div_(L.alpha * wfm::jmin(L.xl[i], L.yl[i]), wfm::sqrt_(GRAVITY * L.h[i]))
                           : wfm::from_bits(0x7ff0000000000000ULL);
 }
+
+#ifdef __CUDACC__
+// FP32 rank of a cell's stable sub-step alpha l / sqrt(g h): h / l^2, the larger the shorter, to
+// within 1e-6. A depth that is NaN or negative ranks first, so that its NaN is found.
+__device__ __forceinline__ float timestep_rank(double h, double l) {
+    if (wfm::isnan_(h) || (wfm::signbit_(h) && !wfm::is_zero_(h))) return __int_as_float(0x7f800000);
+    const float l32 = wfm::f32_of(l);
+    return __fdividef(__fdividef(wfm::f32_of(h), l32), l32);
+}
+#endif
 
 // Edge elevations of the land grid as LocalInertialOverlandFlowParameters derives them
 // (surface_staggered_scheme.jl:929-939): the higher elevation of a cell and its upstream
