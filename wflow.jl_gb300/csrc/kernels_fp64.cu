@@ -22,6 +22,7 @@
 #include "snow_scheme.cuh"
 #include "wf_ff.cuh"
 #include "wf_walker.cuh"
+#include "wf_wave64.cuh"
 
 using wfm::div_;
 using wfm::div_by_;
@@ -36,10 +37,7 @@ using wfm::lt_;
 namespace {
 
 constexpr double KIN_WAVE_MIN_FLOW = 1e-30;                       // routing/utils.jl:1
-constexpr double KIN_WAVE_MIN_FLOW_QROOT = 0x1.0c6f7a0b5ed8ap-20;  // 1e-30^0.2 (routing/utils.jl:2)
-constexpr double BETA = 0.6;                                      // surface_kinwave.jl:2
 constexpr double MM_PER_DAY = (1.0 / 86400.0) * 1e-3;             // units.jl MM_PER_DAY factor
-constexpr double PERCENT = 1e-2;                                  // units.jl PERCENTAGE factor
 constexpr double NANV = __builtin_nan("");
 
 // ------------------------------------------------------------------ process functions ----
@@ -207,38 +205,6 @@ __device__ __forceinline__ double rwu_layer(double vwc, double ts, double tr, do
 
 __device__ __forceinline__ double lb_drainable(double ts, double tfc) { return jmax(ts - tfc, 0.02); }
 
-// kinematic wave for surface flow (routing/surface/surface_process.jl:24-70)
-__device__ void kinematic_wave(double q_in, double q_prev, double q_lat, double alpha, double dt, double dx,
-                               double& q, double& area) {
-    if (q_in + q_prev + q_lat == 0.0) {
-        q = 0.0;
-        area = 0.0;
-        return;
-    }
-    const double dt_dx = dt / dx;
-    const double u_prev = q_prev >= 0.0 ? wfm::pow(q_prev, 0.2) : 0.0;
-    const double cterm = dt_dx * q_in + alpha * u_prev * u_prev * u_prev + dt * q_lat;
-    double u = u_prev > 0.0 ? u_prev : wfm::cbrt(cterm / alpha);
-    const double c1 = 5.0 * dt_dx, c2 = 3.0 * alpha;
-    for (int it = 0; it < 3000; ++it) {
-        const double u2 = u * u;
-        const double u3 = u2 * u;
-        const double fu = u3 * (dt_dx * u2 + alpha) - cterm;
-        if (wfm::fabs_(fu) <= 1.0e-12) break;
-        const double df = u2 * (c1 * u2 + c2);
-        const double u_old = u;
-        u -= fu / df;
-        if (wfm::isnan_(u) || u <= 0.0) u = KIN_WAVE_MIN_FLOW_QROOT;
-        // an iterate that no longer changes repeats itself until max_iters: stop here with the
-        // identical result (e.g. no positive root when the lateral inflow is negative)
-        if (u == u_old) break;
-    }
-    u = jmax(u, KIN_WAVE_MIN_FLOW_QROOT);
-    const double u3 = u * u * u;
-    area = alpha * u3;
-    q = u3 * u * u;
-}
-
 // ------------------------------------------------------------------ soil column ---------
 
 template <int MAXN>
@@ -347,27 +313,36 @@ __device__ __forceinline__ double ssf_celerity(double zi, double slope, double s
                                                double zexp) {
     double z = zi;
     if (profile == WF_KV_EXPONENTIAL_CONSTANT) z = zi < zexp ? zi : zexp;
-    return (kh0 * wfm::exp(-f * z) * slope) / sy;
+    return div_(kh0 * wfm::exp(-f * z) * slope, sy);
 }
 
-// routing/subsurface/subsurface_process.jl:57-78
-__device__ double kw_ssf_newton(double q, double cterm, double celerity, double dt, double dx) {
+// routing/subsurface/subsurface_process.jl:57-78, with dt_dx = dt / dx, cinv = 1 / celerity, df their
+// sum and rdf = 1 / df
+__device__ __forceinline__ double kw_ssf_newton(double q, double cterm, double dt_dx, double cinv, double df, double rdf) {
     int count = 0;
-    const double dt_dx = dt / dx;
-    const double cinv = 1.0 / celerity;
-    const double df = dt_dx + cinv;
     while (true) {
         const double fq = dt_dx * q + cinv * q - cterm;
         const double q_old = q;
-        q -= (fq / df);
+        q -= div_by_(fq, df, rdf);
         if (wfm::isnan_(q)) q = 0.0;
         q = jmax(q, KIN_WAVE_MIN_FLOW);
-        if ((wfm::fabs_(fq) <= 1.0e-12) || (count >= 3000)) break;
-        if (q == q_old) break;  // fixed point: the remaining iterations repeat this one
+        if (wfz::converged(fq) || (count >= 3000)) break;
+        if (wfm::to_bits(q) == wfm::to_bits(q_old)) break;  // fixed point: the remaining iterations repeat this one
         count += 1;
     }
     return q;
 }
+
+// (a + b) / 2
+__device__ __forceinline__ double mean2(double a, double b) {
+    const double t = a + b;
+    const unsigned hx = (unsigned)__double2hiint(t) & 0x7fffffffu;
+    return hx - 0x00200000u < 0x7fd00000u ? wfm::from_bits(wfm::to_bits(t) - 0x0010000000000000ULL) : t / 2.0;
+}
+
+// Largest change of the water table of a sub-step that needs no sub-iterations: the reference takes
+// ceil(round(|dz| / 0.1, 12 digits)) of them, one or none up to 0.1 m.
+__device__ __forceinline__ bool one_iteration(double dz) { return lt_(wfm::fabs_(dz), 0.0999); }
 
 // routing/subsurface/subsurface_process.jl:89-172
 template <int MAXN>
@@ -383,34 +358,40 @@ __device__ void kinematic_wave_ssf(double q_in, double q_prev, double zi_prev, d
         return;
     }
     const double f = col.f;
-    double q = (q_prev + q_in) / 2.0;
     double cel = ssf_celerity(zi_prev, slope, sy, kh0, f, col.profile, col.zexp);
-    double cterm = (dt / dx) * (q_in + q_net) + q_prev / cel;
-    q = kw_ssf_newton(q, cterm, cel, dt, dx);
+    double dt_dx = div_(dt, dx), cinv = div_(1.0, cel);
+    double df = dt_dx + cinv;
+    double cterm = dt_dx * (q_in + q_net) + div_by_(q_prev, cel, cinv);
+    double q = kw_ssf_newton(mean2(q_prev, q_in), cterm, dt_dx, cinv, df, div_(1.0, df));
     q = jmin(q, (q_max * dw));
-    double net_flux = (q_in + q_net - q) / (dw * dx);
+    double net_flux = div_(q_in + q_net - q, dw * dx);
     double dh, exfilt;
     col.water_table_change(net_flux, sy, dt, dh, exfilt);
     double zi = zi_prev - dh;
-    if (zi > d) {
-        const double q_excess = (dw * dx) * sy * (zi - d) / dt;
+    if (gt_(zi, d)) {
+        const double q_excess = div_((dw * dx) * sy * (zi - d), dt);
         q = jmax(q - q_excess, KIN_WAVE_MIN_FLOW);
     }
     zi = jclamp(zi, 0.0, d);
-    const long its = (long)wfm::ceil_(wfm::round_sigdigits(wfm::fabs_(zi - zi_prev) / 0.1, 12));
+    const long its = one_iteration(zi - zi_prev)
+                         ? 1
+                         : (long)wfm::ceil_(wfm::round_sigdigits(wfm::fabs_(zi - zi_prev) / 0.1, 12));
     if (its > 1) {
         const double dt_s = dt / (double)its;
         double q_sum = 0.0, exfilt_sum = 0.0, net_flux_sum = 0.0;
         for (long i = 0; i < its; ++i) {
             cel = ssf_celerity(zi_prev, slope, sy, kh0, f, col.profile, col.zexp);
-            cterm = (dt_s / dx) * q_in + q_prev / cel + q_net * (dt_s / dx);
-            q = kw_ssf_newton(q_prev, cterm, cel, dt_s, dx);
+            dt_dx = div_(dt_s, dx);
+            cinv = div_(1.0, cel);
+            df = dt_dx + cinv;
+            cterm = dt_dx * q_in + div_by_(q_prev, cel, cinv) + q_net * dt_dx;
+            q = kw_ssf_newton(q_prev, cterm, dt_dx, cinv, df, div_(1.0, df));
             q = jmin(q, (q_max * dw));
-            net_flux = (q_in + q_net - q) / (dw * dx);
+            net_flux = div_(q_in + q_net - q, dw * dx);
             col.water_table_change(net_flux, sy, dt_s, dh, exfilt);
             zi = zi_prev - dh;
-            if (zi > d) {
-                const double q_excess = (dw * dx) * sy * (zi - d) / dt_s;
+            if (gt_(zi, d)) {
+                const double q_excess = div_((dw * dx) * sy * (zi - d), dt_s);
                 q = jmax(q - q_excess, KIN_WAVE_MIN_FLOW);
             }
             zi = jclamp(zi, 0.0, d);
@@ -766,8 +747,113 @@ __global__ void __launch_bounds__(256) vertical_kernel(WfDevFields F) {
     }
 }
 
-// ------------------------------------------------------------------ SSF wavefront -------
+// ------------------------------------------------------------------ subsurface ----------
 
+// Recharge flux of a cell (boundary_conditions.jl:219-236, check_flux :12-21)
+__device__ __forceinline__ double ssf_flux(const WfDevFields& F, int64_t e, double area, double zi_ssf, double d) {
+    const double flux = F.Mf[RECHARGE][e] * area;
+    return wfm::le_(d, zi_ssf) ? jmax(0.0, flux) : flux;
+}
+
+// The soil column of a cell as the subsurface update finds it
+template <int MAXN>
+__device__ __forceinline__ void ssf_column(const WfDevFields& F, int64_t slot, int64_t e, Column<MAXN>& col) {
+    col.load_static(F, slot);
+    col.kv0 = F.Mf[KV0][e];
+    col.f = F.Mf[FSCALE][e];
+#pragma unroll
+    for (int k = 0; k < MAXN; ++k) col.usld[k] = k < col.N ? F.LY[LY_USLD][k][e] : 0.0;
+}
+
+// One sub-step of a cell for the upstream inflow qin (tr: what of the upstream discharge goes to the
+// river): discharge, water table, storages and cumulative fluxes, after the model step's last sub-step
+// the averages and update_soil_water_storage!. Returns the discharge.
+template <int MAXN>
+__device__ double ssf_cell(const WfDevFields& F, int64_t slot, int64_t e, double qin, double tr, double dt_s, bool first,
+                           bool last, double dt) {
+    double* const* Mf = F.Mf;
+    double* const* L = F.L;
+    const double area = L[AREA][slot];
+    const double d = L[SOIL_THICKNESS][slot];
+    const double zi_ssf = Mf[SSF_ZI][e];
+    const double flux = ssf_flux(F, e, area, zi_ssf, d);
+    const double q_net = 0.0 + flux;
+    Column<MAXN> col;
+    ssf_column(F, slot, e, col);
+    const double zi_soil = Mf[ZI][e];
+    col.set_thickness(zi_soil);
+    const double q_prev = Mf[SSF_Q][e];
+    const double kh0 = L[KH_RATIO][slot] * col.kv0;
+    double q, zi_new, exfilt, netflux;
+    kinematic_wave_ssf<MAXN>(qin, q_prev, zi_ssf, q_net, L[SLOPE][slot], L[SY][slot], d, dt_s, L[FLOW_LENGTH][slot],
+                             L[FLOW_WIDTH][slot], Mf[Q_MAX][e], kh0, col, q, zi_new, exfilt, netflux);
+    const bool early = (qin + q_prev == 0.0 && q_net <= 0.0);
+    Mf[SSF_Q][e] = q;
+    Mf[SSF_ZI][e] = zi_new;
+    Mf[SSF_STORAGE][e] = L[SY][slot] * (d - zi_new) * area;
+    // cumulative fluxes (set_flux_vars! zeroes them at the start of the model step)
+    double c_tr = (first ? 0.0 : Mf[SSF_TR_CUM][e]) + tr * dt_s;
+    double c_rf = (first ? 0.0 : Mf[RCH_FLUX_CUM][e]) + flux * dt_s;
+    double c_qin = (first ? 0.0 : Mf[SSF_QIN_CUM][e]) + qin * dt_s;
+    double c_q = (first ? 0.0 : Mf[SSF_Q_CUM][e]) + q * dt_s;
+    double c_ex = (first ? 0.0 : Mf[SSF_EXF_CUM][e]) + exfilt * dt_s;
+    double c_nf = (first ? 0.0 : Mf[SSF_QNET_CUM][e]) + netflux * area * dt_s;
+    if (!early) {
+#pragma unroll
+        for (int k = 0; k < MAXN; ++k)
+            if (k < col.N) F.LY[LY_USLD][k][e] = col.usld[k];
+        Mf[ZI][e] = zi_new;
+    }
+    if (!last) {
+        Mf[SSF_TR_CUM][e] = c_tr;
+        Mf[RCH_FLUX_CUM][e] = c_rf;
+        Mf[SSF_QIN_CUM][e] = c_qin;
+        Mf[SSF_Q_CUM][e] = c_q;
+        Mf[SSF_EXF_CUM][e] = c_ex;
+        Mf[SSF_QNET_CUM][e] = c_nf;
+        return q;
+    }
+    // averages (groundwater.jl:622-638, lateral_subsurface_flow.jl:182-196)
+    const double rdt = div_(1.0, dt);
+    const double exf_avg = div_by_(c_ex, dt, rdt);
+    Mf[RCH_FLUX_AVG][e] = div_by_(c_rf, dt, rdt);
+    Mf[SSF_QIN_AVG][e] = div_by_(c_qin, dt, rdt);
+    Mf[SSF_Q_AVG][e] = div_by_(c_q, dt, rdt);
+    Mf[SSF_QNET_AVG][e] = div_by_(c_nf, dt, rdt);
+    Mf[SSF_EXF_AVG][e] = exf_avg;
+    Mf[SSF_TR_AVG][e] = div_by_(c_tr, dt, rdt);
+    // ---- update_soil_water_storage! (soil.jl:1294-1392), soil state after the sweep
+    if (early) {
+        // the soil column kept its state: reload it
+#pragma unroll
+        for (int k = 0; k < MAXN; ++k) col.usld[k] = k < col.N ? F.LY[LY_USLD][k][e] : 0.0;
+        col.set_thickness(zi_soil);
+    }
+    const double zi_s = early ? zi_soil : zi_new;
+    const double ts = col.ts, tr_ = col.tr;
+    double usd = 0.0;
+#pragma unroll
+    for (int k = 0; k < MAXN; ++k)
+        if (k < col.nu) usd += col.usld[k];
+    const double runoff =
+        jmax(0.0, exf_avg + Mf[SATEX][e] + Mf[RUNOFF_LAND][e] + Mf[INFEX][e]);
+    const double sat = (d - zi_s) * (ts - tr_);
+    Mf[SAT][e] = sat;
+    Mf[USTOREDEPTH][e] = usd;
+    Mf[TSWS][e] = sat + usd;
+    Mf[EXFILT][e] = exf_avg;
+    Mf[RUNOFF][e] = runoff;
+    const double net_runoff = runoff - Mf[AE_LAND][e];
+    Mf[NET_RUNOFF][e] = net_runoff;
+    // overland lateral inflow (surface_kinwave.jl:740-766, :365)
+    const double inwater = (net_runoff + 0.0) * area + 0.0;
+    Mf[OL_INWATER][e] = inwater;
+    Mf[OL_QLAT][e] = div_(inwater, L[FLOW_LENGTH][slot]);
+    return q;
+}
+
+// Subsurface sweep of several sub-steps (fixed ones shorter than the model step, or adaptive): the
+// whole cell update in the wavefront walker, since each sub-step needs the column of the last.
 template <int MAXN>
 struct SsfPhys {
     WfDevFields F;
@@ -776,238 +862,438 @@ struct SsfPhys {
 
     __device__ bool node(int64_t slot, int64_t e, int m, int s, uint32_t ep, int64_t chain, bool is_end,
                          double& hq) {
-        double* const* Mf = F.Mf;
-        double* const* L = F.L;
         double dt_s;
         bool first, last;
         if (!wf_substep(sw, m, s, dt_s, first, last)) return true;
-        const double area = L[AREA][slot];
-        const double d = L[SOIL_THICKNESS][slot];
-        double zi_ssf = Mf[SSF_ZI][e];
-        // recharge flux (boundary_conditions.jl:219-236, check_flux :12-21)
-        double flux = Mf[RECHARGE][e] * area;
-        if (zi_ssf >= d) flux = jmax(0.0, flux);
-        const double q_net = 0.0 + flux;
         // upstream inflow (lateral_subsurface_flow.jl:236-242)
         double qin = 0.0, tr = 0.0;
         for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
             double qu;
             if (!wfw::upstream_q(g, sw, hq, o, m, s, ep, F.status, qu)) return false;
-            const double fr = L[FRAC_TO_RIVER][g.up_slot[o]];
+            const double fr = g.up_fr[o];
             qin = qin + qu * (1.0 - fr);
             tr = tr + qu * fr;
         }
-        Column<MAXN> col;
-        col.load_static(F, slot);
-        col.kv0 = Mf[KV0][e];
-        col.f = Mf[FSCALE][e];
-#pragma unroll
-        for (int k = 0; k < MAXN; ++k) col.usld[k] = k < col.N ? F.LY[LY_USLD][k][e] : 0.0;
-        const double zi_soil = Mf[ZI][e];
-        col.set_thickness(zi_soil);
+        hq = ssf_cell<MAXN>(F, slot, e, qin, tr, dt_s, first, last, sw.dt);
+        if (is_end) wfw::publish(g, chain, m, s, ep, hq);
+        return true;
+    }
+};
+
+// ---- one sub-step per model step: terms per cell | slim wavefront | cell update
+
+// The sweep's discharge follows from the inflow alone unless the water table moves by the
+// sub-iteration threshold or below the soil bottom. Falling, it moves by |net| dt / (dw dx sy). Rising,
+// it fills the unsaturated layers from below: W_RISE is the volume that raises it by 0.0989 m
+// (water_table_change's fluxes up to that height), over dt. Both with 1 % in hand of the 0.1 m of
+// the reference's threshold, so a net flux below them takes no sub-iteration, whatever the roundings.
+template <int MAXN>
+__global__ void __launch_bounds__(128) ssf_prep64_kernel(WfDevFields F, WfSweep sw) {
+    const int M = F.M;
+    const int64_t E = F.land_slots * M;
+    double* const* Mf = F.Mf;
+    double* const* L = F.L;
+    const double dt = sw.dt_s, rdt = div_(1.0, dt);
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t slot = e / M;
+        if (F.land_node_of_slot[slot] < 0) continue;
+        const double d = L[SOIL_THICKNESS][slot], zi = Mf[SSF_ZI][e];
+        const double dx = L[FLOW_LENGTH][slot], dw = L[FLOW_WIDTH][slot], sy = L[SY][slot];
         const double q_prev = Mf[SSF_Q][e];
+        Column<MAXN> col;
+        ssf_column(F, slot, e, col);
+        col.set_thickness(Mf[ZI][e]);
         const double kh0 = L[KH_RATIO][slot] * col.kv0;
-        double q, zi_new, exfilt, netflux;
-        kinematic_wave_ssf<MAXN>(qin, q_prev, zi_ssf, q_net, L[SLOPE][slot], L[SY][slot], d, dt_s, L[FLOW_LENGTH][slot],
-                                 L[FLOW_WIDTH][slot], Mf[Q_MAX][e], kh0, col, q, zi_new, exfilt, netflux);
-        const bool early = (qin + q_prev == 0.0 && q_net <= 0.0);
-        Mf[SSF_Q][e] = q;
-        hq = q;
-        Mf[SSF_ZI][e] = zi_new;
-        Mf[SSF_STORAGE][e] = L[SY][slot] * (d - zi_new) * area;
-        // cumulative fluxes (set_flux_vars! zeroes them at the start of the model step)
-        double c_tr = (first ? 0.0 : Mf[SSF_TR_CUM][e]) + tr * dt_s;
-        double c_rf = (first ? 0.0 : Mf[RCH_FLUX_CUM][e]) + flux * dt_s;
-        double c_qin = (first ? 0.0 : Mf[SSF_QIN_CUM][e]) + qin * dt_s;
-        double c_q = (first ? 0.0 : Mf[SSF_Q_CUM][e]) + q * dt_s;
-        double c_ex = (first ? 0.0 : Mf[SSF_EXF_CUM][e]) + exfilt * dt_s;
-        double c_nf = (first ? 0.0 : Mf[SSF_QNET_CUM][e]) + netflux * area * dt_s;
-        if (!early) {
+        const double cel = ssf_celerity(zi, L[SLOPE][slot], sy, kh0, col.f, col.profile, col.zexp);
+        const double dt_dx = div_(dt, dx), cinv = div_(1.0, cel);
+        const double df = dt_dx + cinv;
+        F.W[W_SDTDX][e] = dt_dx;
+        F.W[W_CINV][e] = cinv;
+        F.W[W_SDF][e] = df;
+        F.W[W_SRDF][e] = div_(1.0, df);
+        F.W[W_QPC][e] = div_by_(q_prev, cel, cinv);
+        F.W[W_QNET][e] = 0.0 + ssf_flux(F, e, L[AREA][slot], zi, d);
+        F.W[W_QLIM][e] = Mf[Q_MAX][e] * dw;
+        const double te = col.ts - col.tr;
+        double x = 0.0, h = 0.0;
+        bool reached = false;
 #pragma unroll
-            for (int k = 0; k < MAXN; ++k)
-                if (k < col.N) F.LY[LY_USLD][k][e] = col.usld[k];
-            Mf[ZI][e] = zi_new;
+        for (int k = MAXN; k >= 1; --k) {
+            if (k > col.nu || reached) continue;
+            const double t = col.thick[k - 1], cap = jmax(t * te - col.usld[k - 1], 0.0);
+            if (gt_(h + t, 0.0989)) {
+                const double need = jmax((0.0989 - h) * (te - div_(col.usld[k - 1], t)), 0.0);
+                x += jmin(need, cap);
+                reached = true;
+            } else {
+                x += cap;
+                h += t;
+            }
         }
-        if (is_end) wfw::publish(g, chain, m, s, ep, q);
-        if (!last) {
-            Mf[SSF_TR_CUM][e] = c_tr;
-            Mf[RCH_FLUX_CUM][e] = c_rf;
-            Mf[SSF_QIN_CUM][e] = c_qin;
-            Mf[SSF_Q_CUM][e] = c_q;
-            Mf[SSF_EXF_CUM][e] = c_ex;
-            Mf[SSF_QNET_CUM][e] = c_nf;
-            return true;
-        }
-        // averages (groundwater.jl:622-638, lateral_subsurface_flow.jl:182-196)
-        const double dt = sw.dt;
-        const double exf_avg = c_ex / dt;
-        Mf[RCH_FLUX_AVG][e] = c_rf / dt;
-        Mf[SSF_QIN_AVG][e] = c_qin / dt;
-        Mf[SSF_Q_AVG][e] = c_q / dt;
-        Mf[SSF_QNET_AVG][e] = c_nf / dt;
-        Mf[SSF_EXF_AVG][e] = exf_avg;
-        Mf[SSF_TR_AVG][e] = c_tr / dt;
-        // ---- update_soil_water_storage! (soil.jl:1294-1392), soil state after the sweep
-        if (early) {
-            // the soil column kept its state: reload it
-#pragma unroll
-            for (int k = 0; k < MAXN; ++k) col.usld[k] = k < col.N ? F.LY[LY_USLD][k][e] : 0.0;
-            col.set_thickness(zi_soil);
-        }
-        const double zi_s = early ? zi_soil : Mf[ZI][e];
-        const double ts = col.ts, tr_ = col.tr;
-        double usd = 0.0;
-#pragma unroll
-        for (int k = 0; k < MAXN; ++k)
-            if (k < col.nu) usd += col.usld[k];
-        const double runoff =
-            jmax(0.0, exf_avg + Mf[SATEX][e] + Mf[RUNOFF_LAND][e] + Mf[INFEX][e]);
-        const double sat = (d - zi_s) * (ts - tr_);
-        Mf[SAT][e] = sat;
-        Mf[USTOREDEPTH][e] = usd;
-        Mf[TSWS][e] = sat + usd;
-        Mf[EXFILT][e] = exf_avg;
-        Mf[RUNOFF][e] = runoff;
-        const double net_runoff = runoff - Mf[AE_LAND][e];
-        Mf[NET_RUNOFF][e] = net_runoff;
-        // overland lateral inflow (surface_kinwave.jl:740-766, :365)
-        const double inwater = (net_runoff + 0.0) * area + 0.0;
-        Mf[OL_INWATER][e] = inwater;
-        Mf[OL_QLAT][e] = inwater / L[FLOW_LENGTH][slot];
-        return true;
+        const double per_dt = dw * dx * rdt * (1.0 - 1e-6);
+        F.W[W_RISE][e] = reached ? x * per_dt : wfm::from_bits(0x7ff0000000000000ULL);
+        F.W[W_FALL][e] = jmin(0.0989, d - zi - 1e-9) * sy * per_dt;
     }
-};
+}
 
-// --------------------------------------------------------------- overland wavefront -----
-
-struct OverlandPhys {
+template <int MAXN>
+struct SsfWave64 {
     WfDevFields F;
     WfDevGraph g;
     WfSweep sw;
 
-    __device__ bool node(int64_t slot, int64_t e, int m, int s, uint32_t ep, int64_t chain, bool is_end,
-                         double& hq) {
-        double* const* Mf = F.Mf;
+    struct In {
+        double dt_dx, cinv, df, rdf, qpc, q_net, q_lim, rise, fall, q_prev;
+    };
+    struct St {
+        double q;
+    };
+    __device__ __forceinline__ void load(int64_t slot, int64_t e, int m, bool fresh, bool resumed, In& x) const {
+        double* const* W = F.W;
+        x.dt_dx = W[W_SDTDX][e];
+        x.cinv = W[W_CINV][e];
+        x.df = W[W_SDF][e];
+        x.rdf = W[W_SRDF][e];
+        x.qpc = W[W_QPC][e];
+        x.q_net = W[W_QNET][e];
+        x.q_lim = W[W_QLIM][e];
+        x.rise = W[W_RISE][e];
+        x.fall = W[W_FALL][e];
+        x.q_prev = F.Mf[SSF_Q][e];
+    }
+    __device__ __forceinline__ void start(const In&, St&) const {}
+    // The discharge of a cell whose water table moves across the threshold or the soil bottom
+    __device__ __noinline__ double full(int64_t slot, int64_t e, double qin, double q_net) const {
         double* const* L = F.L;
-        double dt_s;
-        bool first, last;
-        if (!wf_substep(sw, m, s, dt_s, first, last)) return true;
-        if (first && F.mass_balance) Mf[BO_PREV][e] = Mf[OL_STORAGE][e];
-        const double sfw = L[SFW][slot];
-        double tr = 0.0, qin = 0.0;
-        for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
-            double qu;
-            if (!wfw::upstream_q(g, sw, hq, o, m, s, ep, F.status, qu)) return false;
-            const double fr = L[FRAC_TO_RIVER][g.up_slot[o]];
-            tr = tr + qu * fr;
-            qin = qin + qu * (1.0 - fr);
+        Column<MAXN> col;
+        ssf_column(F, slot, e, col);
+        col.set_thickness(F.Mf[ZI][e]);
+        double q, zi_new, exfilt, netflux;
+        kinematic_wave_ssf<MAXN>(qin, F.Mf[SSF_Q][e], F.Mf[SSF_ZI][e], q_net, L[SLOPE][slot], L[SY][slot],
+                                 L[SOIL_THICKNESS][slot], sw.dt_s, L[FLOW_LENGTH][slot], L[FLOW_WIDTH][slot],
+                                 F.Mf[Q_MAX][e], L[KH_RATIO][slot] * col.kv0, col, q, zi_new, exfilt, netflux);
+        return q;
+    }
+    __device__ __forceinline__ bool sub(const In& x, St& st, const wfz::Rec& r, unsigned long long w0,
+                                        unsigned long long w1, int64_t slot, int64_t e, int m, int s, int64_t chain,
+                                        bool is_end, bool heavy, double& hq, bool more) {
+        double qin, tr;
+        if (!wfz::gather<true, false>(g, sw, r, w0, w1, slot, m, s, heavy, hq, F.status, qin, tr)) return false;
+        double q;
+        // the early-out of kinematic_wave_ssf; its full form decides when a discharge is negative
+        const bool none = wfm::is_zero_(qin) && wfm::is_zero_(x.q_prev);
+        if (none && le0_(x.q_net)) {
+            q = 0.0;
+        } else if (lt_(qin, 0.0) || lt_(x.q_prev, 0.0)) {
+            q = full(slot, e, qin, x.q_net);
+        } else {
+            const double in_net = qin + x.q_net;
+            q = kw_ssf_newton(mean2(x.q_prev, qin), x.dt_dx * in_net + x.qpc, x.dt_dx, x.cinv, x.df, x.rdf);
+            q = jmin(q, x.q_lim);
+            const double net = in_net - q;
+            if (!(gt0_(net) ? lt_(net, x.rise) : lt_(-net, x.fall))) q = full(slot, e, qin, x.q_net);
         }
-        if (!(sfw > 0.0)) qin = 0.0;
-        const double fl = L[FLOW_LENGTH][slot];
-        double q, a;
-        kinematic_wave(qin, Mf[OL_Q][e], Mf[OL_QLAT][e], L[OL_ALPHA][slot], dt_s, fl, q, a);
-        double h = Mf[OL_H][e];
-        if (sfw > 0.0) h = a / sfw;
-        Mf[OL_Q][e] = q;
+        st.q = q;
         hq = q;
-        Mf[OL_H][e] = h;
-        Mf[OL_STORAGE][e] = fl * sfw * h;
-        if (is_end) wfw::publish(g, chain, m, s, ep, q);
-        const double c_tr = (first ? 0.0 : Mf[OL_TR_CUM][e]) + tr * dt_s;
-        const double c_q = (first ? 0.0 : Mf[OL_Q_CUM][e]) + q * dt_s;
-        const double c_qin = (first ? 0.0 : Mf[OL_QIN_CUM][e]) + qin * dt_s;
-        if (!last) {
-            Mf[OL_TR_CUM][e] = c_tr;
-            Mf[OL_Q_CUM][e] = c_q;
-            Mf[OL_QIN_CUM][e] = c_qin;
-            return true;
-        }
-        const double dt = sw.dt;
-        Mf[OL_Q_AVG][e] = c_q / dt;
-        Mf[OL_TR_AVG][e] = c_tr / dt;
-        Mf[OL_QIN_AVG][e] = c_qin / dt;
+        if (is_end) wfz::publish(g, chain, m, s, q);
         return true;
     }
+    __device__ __forceinline__ void finish(const St& st, int64_t e, bool) const { F.W[W_Q][e] = st.q; }
 };
 
-// ------------------------------------------------------------------ river wavefront ------
+// The cell update from the sweep's discharges (ssf_cell repeats the cell's own solve: its water table
+// and column need the discharge before the soil-bottom limit).
+template <int MAXN>
+__global__ void __launch_bounds__(128) ssf_post64_kernel(WfDevFields F, WfDevGraph g, WfSweep sw) {
+    const int M = F.M;
+    const int64_t E = F.land_slots * M;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t slot = e / M;
+        if (F.land_node_of_slot[slot] < 0) continue;
+        const int m = (int)(e - slot * M);
+        double qin = 0.0, tr = 0.0;
+        for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
+            const double qu = F.W[W_Q][g.up_slot[o] * M + m], fr = g.up_fr[o];
+            qin = qin + qu * (1.0 - fr);
+            tr = tr + qu * fr;
+        }
+        ssf_cell<MAXN>(F, slot, e, qin, tr, sw.dt_s, true, true, sw.dt);
+    }
+}
 
-// RES: the model has reservoirs. A reservoir cell hands its reservoir's outflow, not its river
-// discharge, to the downstream cell: published for a light child, in the walker's hand-off
-// register for the heavy child.
-template <bool RES>
-struct RiverPhys {
+// ------------------------------------------- overland and river kinematic waves ---------
+
+// Terms of a sweep launch per cell: storage_prev! at the first sub-step of the model step, the river's
+// lateral inflow, and the solve's terms of the state before the launch.
+template <bool LAND>
+__global__ void __launch_bounds__(128) kw_prep64_kernel(WfDevFields F, WfSweep sw) {
+    const int M = F.M;
+    const int64_t E = (LAND ? F.land_slots : F.river_slots) * M;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t slot = e / M;
+        if ((LAND ? F.land_node_of_slot : F.river_node_of_slot)[slot] < 0) continue;
+        const int m = (int)(e - slot * M);
+        bool first = sw.first == 0;
+        double dt_s = sw.dt_s;
+        if (sw.aflag) {
+            bool last;
+            if (!wf_substep(sw, m, 0, dt_s, first, last)) continue;
+        }
+        double dx, alpha, q_prev, q_lat;
+        if (LAND) {
+            if (first && F.mass_balance) F.Mf[BO_PREV][e] = F.Mf[OL_STORAGE][e];
+            dx = F.L[FLOW_LENGTH][slot];
+            alpha = F.L[OL_ALPHA][slot];
+            q_prev = F.Mf[OL_Q][e];
+            q_lat = F.Mf[OL_QLAT][e];
+        } else {
+            double* const* RM = F.RM;
+            double* const* R = F.R;
+            dx = R[R_LENGTH][slot];
+            const double rlen = div_(1.0, dx);
+            if (first) {
+                if (F.mass_balance) RM[BR_PREV][e] = RM[RV_STORAGE][e];
+                // update_lateral_inflow! (surface_kinwave.jl:710-734)
+                const int64_t le = F.river_land_slot[slot] * M + m;
+                const double inw = F.Mf[SSF_TR_AVG][le] + F.Mf[OL_TR_AVG][le] +
+                                   F.Mf[NET_RUNOFF_RIVER][le] * R[R_AREA][slot] + 0.0;
+                RM[RV_INWATER][e] = inw;
+                q_lat = div_by_(inw, dx, rlen);
+                RM[RV_QLAT][e] = q_lat;
+            } else {
+                q_lat = RM[RV_QLAT][e];
+            }
+            // external inflow (surface_kinwave.jl:523-532); the wavefront adds an abstraction itself
+            const double ext = R[R_EXT_INFLOW][slot];
+            if (!lt_(ext, 0.0)) q_lat = q_lat + (div_by_(ext, dx, rlen) - 0.0);
+            alpha = R[R_ALPHA][slot];
+            q_prev = RM[RV_Q][e];
+        }
+        const double dt_dx = div_(dt_s, dx), c1 = 5.0 * dt_dx, c2 = 3.0 * alpha;
+        wfz::KwState k;
+        wfz::kw_state(q_prev, dt_dx, alpha, c1, c2, k);
+        double* const* W = F.W;
+        W[W_U][e] = k.u;
+        W[W_A][e] = k.A;
+        W[W_P][e] = k.P;
+        W[W_DF][e] = k.df;
+        W[W_RDF][e] = k.rdf;
+        W[W_B][e] = dt_s * q_lat;
+        W[W_DTDX][e] = dt_dx;
+        W[W_C1][e] = c1;
+        W[W_C2][e] = c2;
+    }
+}
+
+// The wavefront. CUM: the walker sums the discharges, inflows (land: and flows to the river) over the
+// launch's sub-steps; a launch of one sub-step leaves the sums to the completion kernel, which finds
+// the upstream discharges in the discharge array (not with RES). RES: the model has reservoirs; a
+// reservoir cell hands its reservoir's outflow, not its river discharge, to the downstream cell.
+template <bool LAND, bool CUM, bool RES>
+struct KwWave64 {
     WfDevFields F;
     WfDevGraph g;
     WfSweep sw;
 
-    __device__ bool node(int64_t slot, int64_t e, int m, int s, uint32_t ep, int64_t chain, bool is_end,
-                         double& hq) {
-        double* const* RM = F.RM;
-        double* const* R = F.R;
-        const int M = F.M;
-        double dt_s;
-        bool first, last;
-        if (!wf_substep(sw, m, s, dt_s, first, last)) return true;
-        const double len = R[R_LENGTH][slot];
-        double qlat;
-        if (first) {
-            if (F.mass_balance) RM[BR_PREV][e] = RM[RV_STORAGE][e];
-            // update_lateral_inflow! (surface_kinwave.jl:710-734)
-            const int64_t le = F.river_land_slot[slot] * M + m;
-            const double inw = F.Mf[SSF_TR_AVG][le] + F.Mf[OL_TR_AVG][le] +
-                               F.Mf[NET_RUNOFF_RIVER][le] * R[R_AREA][slot] + 0.0;
-            RM[RV_INWATER][e] = inw;
-            qlat = inw / len;
-            RM[RV_QLAT][e] = qlat;
+    struct In {
+        wfz::KwState k;
+        double b, dt_dx, c1, c2, alpha, q_prev;
+        double u;                // river: final iterate of this launch's last sub-step (0: none yet)
+        double c_q, c_qin, c_x;  // cumulative discharge, inflow, flow to the river (abstraction)
+    };
+    struct St {
+        wfz::KwState k;
+        double q_prev, u;
+        double c_q, c_qin, c_x;
+    };
+    __device__ __forceinline__ double* q_of() const { return LAND ? F.Mf[OL_Q] : F.RM[RV_Q]; }
+    __device__ __forceinline__ double* cq_of() const { return LAND ? F.Mf[OL_Q_CUM] : F.RM[RV_Q_CUM]; }
+    __device__ __forceinline__ double* cqin_of() const { return LAND ? F.Mf[OL_QIN_CUM] : F.RM[RV_QIN_CUM]; }
+    __device__ __forceinline__ double* cx_of() const { return LAND ? F.Mf[OL_TR_CUM] : F.RM[RV_ABS_CUM]; }
+
+    __device__ __forceinline__ void load(int64_t slot, int64_t e, int m, bool fresh, bool resumed, In& x) const {
+        double* const* W = F.W;
+        x.k.u = W[W_U][e];
+        x.k.A = W[W_A][e];
+        x.k.P = W[W_P][e];
+        x.k.df = W[W_DF][e];
+        x.k.rdf = W[W_RDF][e];
+        x.b = W[W_B][e];
+        x.dt_dx = W[W_DTDX][e];
+        x.c1 = W[W_C1][e];
+        x.c2 = W[W_C2][e];
+        x.alpha = LAND ? F.L[OL_ALPHA][slot] : F.R[R_ALPHA][slot];
+        x.q_prev = q_of()[e];
+        x.u = !LAND && resumed ? W[W_UEND][e] : 0.0;
+        x.c_q = x.c_qin = x.c_x = 0.0;
+        if (CUM) {
+            if (sw.aflag) fresh = (sw.aflag[m] & WF_SUB_FIRST) != 0;
+            if (!fresh) {
+                x.c_q = cq_of()[e];
+                x.c_qin = cqin_of()[e];
+                x.c_x = cx_of()[e];
+            }
+        }
+    }
+    __device__ __forceinline__ void start(const In& x, St& st) const {
+        st.k = x.k;
+        st.q_prev = x.q_prev;
+        st.u = x.u;
+        st.c_q = x.c_q;
+        st.c_qin = x.c_qin;
+        st.c_x = x.c_x;
+    }
+    __device__ __forceinline__ bool sub(const In& x, St& st, const wfz::Rec& r, unsigned long long w0,
+                                        unsigned long long w1, int64_t slot, int64_t e, int m, int s, int64_t chain,
+                                        bool is_end, bool heavy, double& hq, bool more) {
+        double dt_s = sw.dt_s;
+        if (sw.aflag) {  // a member that has reached the end of the step takes no further sub-step
+            if (!(sw.aflag[m] & WF_SUB_ACTIVE)) {
+                st.u = -1.0;
+                return true;
+            }
+            dt_s = sw.adt[m];
+        }
+        double qin, tr;
+        if (!wfz::gather<LAND, CUM>(g, sw, r, w0, w1, slot, m, s, heavy, hq, F.status, qin, tr)) return false;
+        if (LAND && (r.flags & wfz::REC_NO_INFLOW)) qin = 0.0;
+        const float r_dt32 = __frcp_rn(wfm::f32_of(dt_s));
+        double b = x.b, q_lat = 0.0, taken = 0.0;
+        const bool draws = !LAND && (r.flags & wfz::REC_ABSTRACTION);
+        if (draws) {  // abstraction up to 80 % of the storage (surface_kinwave.jl:523-532)
+            const double len = F.R[R_LENGTH][slot], ext = F.R[R_EXT_INFLOW][slot];
+            // the storage that the previous sub-step left (of this launch: its final iterate in st.u)
+            const double storage =
+                gt0_(st.u) ? len * (wfm::is_zero_(st.q_prev) ? 0.0 : x.alpha * (st.u * st.u * st.u)) : F.RM[RV_STORAGE][e];
+            taken = jmin(-ext, div_(storage, dt_s) * 0.80);
+            q_lat = F.RM[RV_QLAT][e] + (div_(-taken, len) - 0.0);
+            b = dt_s * q_lat;
+        }
+        double q, u;
+        bool zero = false;
+        // q_in + q_prev + q_lat == 0: only without a positive previous discharge or with a negative term,
+        // and then not where FP32 sees a difference
+        const float in32 = wfm::f32_of(qin) + wfm::f32_of(st.q_prev), lat32 = wfm::f32_of(b) * r_dt32;
+        if (!(gt0_(st.q_prev) && !lt_(b, 0.0) && !lt_(qin, 0.0)) &&
+            !(fabsf(in32 + lat32) > 1e-4f * (fabsf(in32) + fabsf(lat32)))) {
+            if (!draws)
+                q_lat = LAND ? F.Mf[OL_QLAT][e]
+                             : F.RM[RV_QLAT][e] + (div_(F.R[R_EXT_INFLOW][slot], F.R[R_LENGTH][slot]) - 0.0);
+            zero = wfm::is_zero_(qin + st.q_prev + q_lat);
+        }
+        if (zero) {
+            q = u = 0.0;
         } else {
-            qlat = RM[RV_QLAT][e];
+            q = wfz::kw_solve(st.k, x.dt_dx * qin + st.k.A + b, x.dt_dx, x.alpha, x.c1, x.c2, u);
         }
-        double qs = 0.0;
-        for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
-            double qu;
-            if (!wfw::upstream_q(g, sw, hq, o, m, s, ep, F.status, qu)) return false;
-            qs = qs + qu;
-        }
-        const double qin = 0.0 + qs;
-        // external inflow / abstraction (surface_kinwave.jl:523-532)
-        const double ext = R[R_EXT_INFLOW][slot];
-        double inflow, absd = 0.0;
-        if (ext < 0.0) {
-            absd = jmin(-ext, (RM[RV_STORAGE][e] / dt_s) * 0.80);
-            inflow = -absd / len;
-        } else {
-            inflow = ext / len;
-        }
-        inflow -= 0.0 / len;
-        double q, a;
-        kinematic_wave(qin, RM[RV_Q][e], qlat + inflow, R[R_ALPHA][slot], dt_s, len, q, a);
-        RM[RV_Q][e] = q;
-        double q_down = q;  // what the downstream cell receives
+        double q_down = q;
         if (RES) {
-            const int32_t r = F.res_of_rslot[slot];
-            if (r >= 0) q_down = wfr::reservoir_node(F, r, m, q, dt_s);
+            const int32_t res = F.res_of_rslot[slot];
+            if (res >= 0) q_down = wfr::reservoir_node(F, res, m, q, dt_s);
         }
         hq = q_down;
-        RM[RV_H][e] = a / R[R_WIDTH][slot];
-        RM[RV_STORAGE][e] = len * a;
-        if (is_end) wfw::publish(g, chain, m, s, ep, q_down);
-        const double c_q = (first ? 0.0 : RM[RV_Q_CUM][e]) + q * dt_s;
-        const double c_qin = (first ? 0.0 : RM[RV_QIN_CUM][e]) + qin * dt_s;
-        const double c_ab = (first ? 0.0 : RM[RV_ABS_CUM][e]) + absd * dt_s;
-        if (!last) {
-            RM[RV_Q_CUM][e] = c_q;
-            RM[RV_QIN_CUM][e] = c_qin;
-            RM[RV_ABS_CUM][e] = c_ab;
-            return true;
+        if (is_end) wfz::publish(g, chain, m, s, q_down);
+        if (CUM) {
+            st.c_q = st.c_q + q * dt_s;
+            st.c_qin = st.c_qin + qin * dt_s;
+            if (LAND ? (r.flags & wfz::REC_WEIGHTED) != 0 : draws) st.c_x = st.c_x + (LAND ? tr : taken) * dt_s;
         }
-        const double dt = sw.dt;
-        RM[RV_Q_AVG][e] = c_q / dt;
-        RM[RV_ABS_AVG][e] = c_ab / dt;
-        RM[RV_QIN_AVG][e] = c_qin / dt;
+        st.q_prev = q;
+        st.u = u;
+        if (more) wfz::kw_state(q, x.dt_dx, x.alpha, x.c1, x.c2, st.k);
         return true;
     }
+    __device__ __forceinline__ void finish(const St& st, int64_t e, bool last_round) const {
+        if (lt_(st.u, 0.0)) return;  // no sub-step taken
+        q_of()[e] = st.q_prev;
+        F.W[W_UEND][e] = st.u;
+        if (CUM) {
+            cq_of()[e] = st.c_q;
+            cqin_of()[e] = st.c_qin;
+            cx_of()[e] = st.c_x;
+        }
+        if (!last_round) {
+            F.W[W_U][e] = st.k.u;
+            F.W[W_A][e] = st.k.A;
+            F.W[W_P][e] = st.k.P;
+            F.W[W_DF][e] = st.k.df;
+            F.W[W_RDF][e] = st.k.rdf;
+        }
+    }
 };
+
+// After a sweep launch: depth and storage of every cell, its sums when the walker has not kept them
+// (CUM), and after the model step's last sub-step the averages.
+template <bool LAND, bool CUM>
+__global__ void __launch_bounds__(128) kw_post64_kernel(WfDevFields F, WfDevGraph g, WfSweep sw) {
+    const int M = F.M;
+    const int64_t E = (LAND ? F.land_slots : F.river_slots) * M;
+    const double dt = sw.dt, rdt = div_(1.0, dt);
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t slot = e / M;
+        if ((LAND ? F.land_node_of_slot : F.river_node_of_slot)[slot] < 0) continue;
+        const int m = (int)(e - slot * M);
+        bool first = sw.first == 0, last = sw.last_of_step != 0;
+        double dt_s = sw.dt_s;
+        if (sw.aflag && !wf_substep(sw, m, 0, dt_s, first, last)) continue;
+        const double u = F.W[W_UEND][e];
+        const double* q_all = LAND ? F.Mf[OL_Q] : F.RM[RV_Q];
+        const double q = q_all[e];
+        const double area = wfm::is_zero_(q) ? 0.0 : (LAND ? F.L[OL_ALPHA][slot] : F.R[R_ALPHA][slot]) * (u * u * u);
+        const int32_t flags = g.up_rec64[slot].z;
+        double* cq = LAND ? F.Mf[OL_Q_CUM] : F.RM[RV_Q_CUM];
+        double* cqin = LAND ? F.Mf[OL_QIN_CUM] : F.RM[RV_QIN_CUM];
+        double* cx = LAND ? F.Mf[OL_TR_CUM] : F.RM[RV_ABS_CUM];
+        double c_q, c_qin, c_x;
+        if (CUM) {
+            c_q = cq[e];
+            c_qin = cqin[e];
+            c_x = cx[e];
+        } else {
+            double qin = 0.0, tr = 0.0, taken = 0.0;
+            for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
+                const double qu = q_all[g.up_slot[o] * M + m];
+                if (LAND) {
+                    tr = tr + qu * g.up_fr[o];
+                    qin = qin + qu * g.up_w[o];
+                } else {
+                    qin = qin + qu;
+                }
+            }
+            if (flags & wfz::REC_NO_INFLOW) qin = 0.0;
+            // the storage before the sub-step: this kernel overwrites it below
+            if (!LAND && (flags & wfz::REC_ABSTRACTION))
+                taken = jmin(-F.R[R_EXT_INFLOW][slot], div_(F.RM[RV_STORAGE][e], dt_s) * 0.80);
+            c_q = (first ? 0.0 : cq[e]) + q * dt_s;
+            c_qin = (first ? 0.0 : cqin[e]) + qin * dt_s;
+            c_x = (first ? 0.0 : cx[e]) + (LAND ? tr : taken) * dt_s;
+            if (!last) {
+                cq[e] = c_q;
+                cqin[e] = c_qin;
+                cx[e] = c_x;
+            }
+        }
+        if (LAND) {
+            const double sfw = F.L[SFW][slot];
+            double h = F.Mf[OL_H][e];
+            if (gt0_(sfw)) h = div_(area, sfw);
+            F.Mf[OL_H][e] = h;
+            F.Mf[OL_STORAGE][e] = F.L[FLOW_LENGTH][slot] * sfw * h;
+        } else {
+            F.RM[RV_H][e] = div_(area, F.R[R_WIDTH][slot]);
+            F.RM[RV_STORAGE][e] = F.R[R_LENGTH][slot] * area;
+        }
+        if (!last) continue;
+        (LAND ? F.Mf[OL_Q_AVG] : F.RM[RV_Q_AVG])[e] = div_by_(c_q, dt, rdt);
+        (LAND ? F.Mf[OL_TR_AVG] : F.RM[RV_ABS_AVG])[e] = div_by_(c_x, dt, rdt);
+        (LAND ? F.Mf[OL_QIN_AVG] : F.RM[RV_QIN_AVG])[e] = div_by_(c_qin, dt, rdt);
+    }
+}
+
+template <class Phys, bool MULTI>
+__global__ void __launch_bounds__(128) wave64_kernel(Phys phys, int64_t p_chunks, int SLp, int SLr, int batch) {
+    wfz::walk<Phys, MULTI>(phys, p_chunks, SLp, SLr, batch, phys.F.status);
+}
 
 // --------------------------------------------------------- gravitational snow transport ----
 
@@ -1332,13 +1618,84 @@ cudaError_t wf_fp64_li_couple_out(const WfDevFields& F, const WfLiCoupleView& v,
     return cudaGetLastError();
 }
 
+namespace {
+
+// Launch of a slim wavefront. Long chains (as many as half of the resident warps take) go first, each
+// in a warp of its own; the lanes beyond a chain's sub-steps stay idle, because one lane's long solve
+// (a drained cell that gets water again takes up to 75 iterations) holds up its whole warp. The other
+// chains are packed as loosely as their number allows: the plan's packing lanes (wave64_lanes).
+template <class Phys, bool MULTI>
+cudaError_t launch_wave64(const Phys& phys, const WfLaunchCfg& c) {
+    const int threads = 32 * (c.walk_warps > 0 ? std::min(c.walk_warps, 4) : 4);
+    const size_t smem = wfz::walk_smem(threads);
+    const WfDevGraph& g = phys.g;
+    const int SLp = g.M == 1 ? 32 : 1 << (31 - __builtin_clz(32 / std::min(g.M, 32) | 1));
+    int SLr = g.lanes64;
+    if (MULTI) {
+        const int cap = c.sub_lanes > 0 ? std::min(c.sub_lanes, 32) : 32;
+        int need = 1;
+        while (need < phys.sw.S && need < cap) need <<= 1;
+        SLr = c.sub_lanes > 0 ? need : std::max(SLr, std::min(need, g.lanes64_multi));
+    }
+    int per_sm = 0;
+    const cudaError_t err =
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wave64_kernel<Phys, MULTI>, threads, smem);
+    if (err != cudaSuccess) return err;
+    if (per_sm < 1) per_sm = 1;
+    // one or two warps per scheduler: a scheduler issues one FP64 instruction per 64 cycles, which one warp
+    // keeps busy, and more warps only slow the long chains down
+    const int fill = std::min(per_sm, 2);
+    int blocks = c.walk_blocks > 0 ? c.walk_blocks : c.num_sms * fill;
+    const int wpb = threads / 32;
+    const int64_t ipp = wf_items_per_chunk(1, g.M, SLp);
+    const int64_t items = g.n_chunks * wf_items_per_chunk(g.G, g.M, SLr);
+    const int64_t need = std::max<int64_t>((items + wpb - 1) / wpb, 1);
+    if (blocks > need) blocks = (int)need;
+    const int64_t resident = (int64_t)std::min(blocks, c.num_sms * per_sm) * wpb;
+    const int64_t p_chunks = std::min<int64_t>(g.n_long_chunks, resident / 2 / ipp);
+    // batches of short chains only where there are more items than warps
+    const int batch = (int)std::max<int64_t>(1, std::min<int64_t>(wfv::BATCH, items / (4 * resident)));
+    wave64_kernel<Phys, MULTI><<<blocks, threads, smem, c.stream>>>(phys, p_chunks, SLp, SLr, batch);
+    return cudaGetLastError();
+}
+
+template <int MAXN>
+cudaError_t launch_ssf_wave(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c) {
+    const int grid = grid_for(F.land_slots * F.M, 128, c.num_sms);
+    ssf_prep64_kernel<MAXN><<<grid, 128, 0, c.stream>>>(F, sw);
+    const cudaError_t err = launch_wave64<SsfWave64<MAXN>, false>(SsfWave64<MAXN>{F, g, sw}, c);
+    if (err != cudaSuccess) return err;
+    ssf_post64_kernel<MAXN><<<grid, 128, 0, c.stream>>>(F, g, sw);
+    return cudaGetLastError();
+}
+
+template <bool LAND, bool CUM, bool RES, bool MULTI>
+cudaError_t launch_kw(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c) {
+    const int grid = grid_for((LAND ? F.land_slots : F.river_slots) * F.M, 128, c.num_sms);
+    kw_prep64_kernel<LAND><<<grid, 128, 0, c.stream>>>(F, sw);
+    const cudaError_t err = launch_wave64<KwWave64<LAND, CUM, RES>, MULTI>(KwWave64<LAND, CUM, RES>{F, g, sw}, c);
+    if (err != cudaSuccess) return err;
+    kw_post64_kernel<LAND, CUM><<<grid, 128, 0, c.stream>>>(F, g, sw);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t wf_fp64_ssf_wave(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c) {
+    return F.N <= 4 ? launch_ssf_wave<4>(F, g, sw, c) : launch_ssf_wave<WF_MAX_LAYERS>(F, g, sw, c);
+}
+
 cudaError_t wf_fp64_overland(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c) {
-    return launch_walk(OverlandPhys{F, g, sw}, c);
+    return sw.S > 1 ? launch_kw<true, true, false, true>(F, g, sw, c)
+                    : launch_kw<true, false, false, false>(F, g, sw, c);
 }
 
 cudaError_t wf_fp64_river(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c) {
-    if (F.n_res > 0) return launch_walk(RiverPhys<true>{F, g, sw}, c);
-    return launch_walk(RiverPhys<false>{F, g, sw}, c);
+    if (F.n_res > 0)
+        return sw.S > 1 ? launch_kw<false, true, true, true>(F, g, sw, c)
+                        : launch_kw<false, true, true, false>(F, g, sw, c);
+    return sw.S > 1 ? launch_kw<false, true, false, true>(F, g, sw, c)
+                    : launch_kw<false, false, false, false>(F, g, sw, c);
 }
 
 // ------------------------------------------------------------------ reservoirs -----------

@@ -22,6 +22,7 @@
 #include "wf_kernels.h"
 #include "wf_li_couple.cuh"
 #include "wf_wave.cuh"
+#include "wf_wave64.cuh"
 #include "wf_math.cuh"
 #include "wf_plan.h"
 #include "wflow_gb300.h"
@@ -42,6 +43,9 @@ struct DevGraphAlloc {
     float* up_whv = nullptr;
     uint8_t* up_nlt = nullptr;
     float4* up_frec = nullptr;
+    int4* up_rec64 = nullptr;
+    double* up_w64 = nullptr;
+    int32_t lanes64 = 1, lanes64_multi = 1;
     uint32_t* flags = nullptr;
     double* end_q = nullptr;
     unsigned long long* ticket = nullptr;
@@ -251,12 +255,30 @@ WfDevGraph dev_graph(const DevGraphAlloc& G, int M) {
     g.up_whv = G.up_whv;
     g.up_nlt = G.up_nlt;
     g.up_frec = G.up_frec;
+    g.up_rec64 = G.up_rec64;
+    g.up_w64 = G.up_w64;
+    g.lanes64 = G.lanes64;
+    g.lanes64_multi = G.lanes64_multi;
     g.flags = G.flags;
     g.end_q = G.end_q;
     g.ticket = G.ticket;
     g.s_cap = G.s_cap;
     g.snow_up = G.snow_up;
     return g;
+}
+
+// Packing lanes per chain-member pair of the FP64 form's slim wavefronts, for launches of S sub-steps: the
+// most (fewest pairs per warp) for which the chains outside the first-dispatched group take at most
+// a quarter of the longest chain's time steps on the schedulers of the device.
+int wave64_lanes(const WfRoutingPlan& P, int M, int S, int num_sms) {
+    for (int SL = 32; SL > 1; SL >>= 1) {
+        const int SU = std::min(SL, S);
+        const int64_t rounds = (S + SU - 1) / SU, ipc = wf_items_per_chunk(P.G, M, SL);
+        int64_t steps = 0;
+        for (int64_t k = 0; k < P.n_chunks - P.n_long_chunks; ++k) steps += rounds * (P.chunk_len[k] + SU) * ipc;
+        if (steps / (num_sms * 4) <= rounds * (P.max_len + SU) / 4) return SL;
+    }
+    return 1;
 }
 
 // Graphs.jl v1.14 topological_sort_by_dfs (Wflow's network.order, network.jl:99) of a graph of
@@ -1330,6 +1352,38 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         CKR(upload(h, &G.up_whv, whv));
         CKR(upload(h, &G.up_nlt, nlt));
         CKR(upload(h, &G.up_frec, frec));
+        if (!F.split) {  // records of the FP64 form's slim wavefronts
+            std::vector<int4> r64(rec.size(), int4{-1, -1, 0, 0});
+            std::vector<double> w64(g == 0 ? rec.size() * 6 : 1, 0.0);
+            for (int64_t sl = 0; sl < P.n_slots; ++sl) {
+                const int64_t node = P.node_of_slot[sl];
+                if (node < 0) continue;
+                int4& q = r64[sl];
+                int entries = 0, heavy_at = -1;
+                for (int32_t o = P.up_ptr[sl]; o < P.up_ptr[sl + 1]; ++o, ++entries) {
+                    const bool heavy = P.up_chain[o] < 0;
+                    if (heavy) heavy_at = entries;
+                    const int at = heavy ? 0 : q.w + 1;  // heavy child, light child 0, light child 1
+                    if (!heavy) {
+                        if (q.w == 0) q.x = P.up_chain[o];
+                        if (q.w == 1) q.y = P.up_chain[o];
+                        q.w += 1;
+                    }
+                    if (g == 0 && at < 3) {
+                        w64[sl * 6 + 2 * at] = w[o];
+                        w64[sl * 6 + 2 * at + 1] = fr[o];
+                    }
+                    if (g == 0 && fr[o] != 0.0) q.z |= wfz::REC_WEIGHTED;
+                }
+                if (heavy_at >= 0 && heavy_at == entries - 1) q.z |= wfz::REC_HEAVY_LAST;
+                if (g == 0 && !(d->surface_flow_width[node] > 0.0)) q.z |= wfz::REC_NO_INFLOW;
+                if (g == 1 && r_ext[node] < 0.0) q.z |= wfz::REC_ABSTRACTION;
+            }
+            G.lanes64 = wave64_lanes(P, M, 1, h->num_sms);
+            G.lanes64_multi = wave64_lanes(P, M, G.s_cap, h->num_sms);
+            CKR(upload(h, &G.up_rec64, r64));
+            CKR(upload(h, &G.up_w64, w64));
+        }
     }
     // ---- split form: FP32 copies of the static fields and FP32 member fields
     if (F.split) {
@@ -1470,7 +1524,9 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
     // split form: the vertical kernel prepares the terms of a single subsurface sub-step; with
     // adaptive sub-steps that sub-step is the whole model step (used when every member's first
     // Courant sub-step reaches the end of the step, the usual case)
-    F.ssf_single = F.split && h->h_dts_ssf.size() == 1;
+    F.ssf_single = h->h_dts_ssf.size() == 1 && (F.split || !h->adaptive);
+    if (!F.split)
+        for (int k = 0; k < 10; ++k) CKR(dalloc(h, &F.W[k], (size_t)std::max(PL.n_slots, PR.n_slots) * M));
     if (F.split && PR.n_slots > 0) CKR(dalloc(h, &F.rv_lat_pub, (size_t)PR.n_slots * M));
     F.dt_ssf = h->h_dts_ssf[0];
     F.inv_dt_ssf = 1.0 / h->h_dts_ssf[0];
@@ -2030,6 +2086,35 @@ int enqueue_vertical(WfHandle* h, const WfLaunchCfg& lc, const WfDevGraph& gl, i
     return WF_OK;
 }
 
+// One FP64 sweep (0 subsurface, 1 overland, 2 river) with the slim wavefronts: launches of up to s_cap
+// sub-steps of one size, each with its per-cell kernels before and after it.
+int sweep_wave64(WfHandle* h, const DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts,
+                 const double* d_dts, int which, const WfLaunchCfg& lc, int64_t& nl) {
+    const int total = (int)dts.size();
+    for (int first = 0; first < total;) {
+        WfSweep sw{};
+        sw.S = 1;
+        while (sw.S < G.s_cap && first + sw.S < total && dts[first + sw.S] == dts[first]) ++sw.S;
+        sw.first = first;
+        sw.last_of_step = (first + sw.S == total);
+        sw.total = total;
+        sw.epoch0 = 1;
+        sw.dt = h->cfg.dt;
+        sw.dts = d_dts + first;
+        sw.dt_s = dts[first];
+        sw.wait_ns = h->wait_ns;
+        sw.wait_offset = h->wait_offset;
+        CK(cudaMemsetAsync(g.end_q, 0xFF, (size_t)G.plan.n_chains * h->M * G.s_cap * sizeof(double), h->stream));
+        CK(cudaMemsetAsync(g.ticket, 0, sizeof(unsigned long long), h->stream));
+        CK(which == 0   ? wf_fp64_ssf_wave(h->F, g, sw, lc)
+           : which == 1 ? wf_fp64_overland(h->F, g, sw, lc)
+                        : wf_fp64_river(h->F, g, sw, lc));
+        nl += 3;
+        first += sw.S;
+    }
+    return WF_OK;
+}
+
 // Enqueue one model step on the handle's stream (with adaptive sub-steps the host waits for
 // the device after every sub-step, see below).
 int enqueue_step(WfHandle* h, int64_t* launches) {
@@ -2045,8 +2130,8 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
     int rcv = enqueue_vertical(h, lc, gl, nl);
     if (rcv) return rcv;
     mark(1);
-    auto sweep = [&](DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts, double* d_dts,
-                     int which) -> int {
+    // subsurface sweeps of several sub-steps
+    auto sweep = [&](DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts, double* d_dts) -> int {
         const int total = (int)dts.size();
         for (int first = 0; first < total; first += G.s_cap) {
             WfSweep sw{};
@@ -2062,14 +2147,15 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
             CK(cudaMemsetAsync(G.flags, 0, (size_t)G.plan.n_chains * h->M * sizeof(uint32_t), h->stream));
             CK(cudaMemsetAsync(G.ticket, 0, sizeof(unsigned long long), h->stream));
             cudaError_t e;
-            if (which == 0) e = split ? wf_split_ssf(h->F, g, sw, lc) : wf_fp64_ssf(h->F, g, sw, lc);
-            else if (which == 1) e = wf_fp64_overland(h->F, g, sw, lc);
-            else e = wf_fp64_river(h->F, g, sw, lc);
+            e = split ? wf_split_ssf(h->F, g, sw, lc) : wf_fp64_ssf(h->F, g, sw, lc);
             CK(e);
             ++nl;
         }
         return WF_OK;
     };
+    // FP64 form: slim wavefronts between their per-cell kernels
+    auto wave64 = [&](DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts, double* d_dts,
+                      int which) -> int { return sweep_wave64(h, G, g, dts, d_dts, which, lc, nl); };
     // split form: slim wavefronts (end_q sentinel hand-off, node-major sub-step groups)
     // followed by their per-cell completion kernels
     auto wave_sw = [&](const DevGraphAlloc& G, const std::vector<double>& dts, double* d_dts, int first) {
@@ -2147,15 +2233,18 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
             sw.wait_offset = h->wait_offset;
             CK(cudaMemsetAsync(G.ticket, 0, sizeof(unsigned long long), h->stream));
             cudaError_t e;
-            if (slim) {
+            if (!split && kind != WF_ADAPT_SSF) {
+                CK(cudaMemsetAsync(G.end_q, 0xFF, (size_t)G.plan.n_chains * h->M * G.s_cap * sizeof(double),
+                                   h->stream));
+                e = kind == WF_ADAPT_LAND ? wf_fp64_overland(h->F, g, sw, lc) : wf_fp64_river(h->F, g, sw, lc);
+                nl += 2;
+            } else if (slim) {
                 CK(cudaMemsetAsync(G.end_q, 0xFF, (size_t)G.plan.n_chains * h->M * G.s_cap * sizeof(double),
                                    h->stream));
                 e = kind == WF_ADAPT_LAND ? wf_split_overland_wave(h->F, g, sw, lc) : wf_split_river_wave(h->F, g, sw, lc);
             } else {
                 CK(cudaMemsetAsync(G.flags, 0, (size_t)G.plan.n_chains * h->M * sizeof(uint32_t), h->stream));
-                if (kind == WF_ADAPT_SSF) e = split ? wf_split_ssf(h->F, g, sw, lc) : wf_fp64_ssf(h->F, g, sw, lc);
-                else if (kind == WF_ADAPT_LAND) e = wf_fp64_overland(h->F, g, sw, lc);
-                else e = wf_fp64_river(h->F, g, sw, lc);
+                e = split ? wf_split_ssf(h->F, g, sw, lc) : wf_fp64_ssf(h->F, g, sw, lc);
             }
             CK(e);
             ++nl;
@@ -2196,7 +2285,7 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
         mark(4);
     } else if (split) {
         if (h->F.ssf_single) rc = wave(h->land, gl, h->h_dts_ssf, h->dts_ssf, 0);
-        else rc = sweep(h->land, gl, h->h_dts_ssf, h->dts_ssf, 0);
+        else rc = sweep(h->land, gl, h->h_dts_ssf, h->dts_ssf);
         if (rc) return rc;
         mark(2);
         // the overland sweep and the river's first sub-step group in one launch (the river cells
@@ -2232,7 +2321,9 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
         }
     } else if (h->li) {
         // local-inertial land and river routing (surface_routing.jl:62-89) after the subsurface
-        if ((rc = sweep(h->land, gl, h->h_dts_ssf, h->dts_ssf, 0))) return rc;
+        rc = h->F.ssf_single ? wave64(h->land, gl, h->h_dts_ssf, h->dts_ssf, 0)
+                             : sweep(h->land, gl, h->h_dts_ssf, h->dts_ssf);
+        if (rc) return rc;
         mark(2);
         CK(wf_fp64_li_couple_in(h->F, h->liv, lc));
         ++nl;
@@ -2244,12 +2335,14 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
         ++nl;
         mark(4);
     } else {
-        if ((rc = sweep(h->land, gl, h->h_dts_ssf, h->dts_ssf, 0))) return rc;
+        rc = h->F.ssf_single ? wave64(h->land, gl, h->h_dts_ssf, h->dts_ssf, 0)
+                             : sweep(h->land, gl, h->h_dts_ssf, h->dts_ssf);
+        if (rc) return rc;
         mark(2);
-        if ((rc = sweep(h->land, gl, h->h_dts_land, h->dts_land, 1))) return rc;
+        if ((rc = wave64(h->land, gl, h->h_dts_land, h->dts_land, 1))) return rc;
         mark(3);
         if ((rc = res_prep())) return rc;
-        if (h->nr > 0 && (rc = sweep(h->river, gr, h->h_dts_river, h->dts_river, 2))) return rc;
+        if (h->nr > 0 && (rc = wave64(h->river, gr, h->h_dts_river, h->dts_river, 2))) return rc;
         if ((rc = res_post())) return rc;
         mark(4);
     }
@@ -2417,6 +2510,7 @@ int enqueue_step_static(WfHandle* h, unsigned char* base, int64_t* launches) {
     };
     auto sweep = [&](const DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts, double* d_dts,
                      int which, bool wave) -> int {
+        if (!split && (which != 0 || h->F.ssf_single)) return sweep_wave64(h, G, g, dts, d_dts, which, lc, nl);
         const int total = (int)dts.size();
         const int group = wave ? std::min<int>(G.s_cap, wfv::MAX_GROUP) : G.s_cap;
         for (int first = 0; first < total; first += group) {
@@ -2438,12 +2532,8 @@ int enqueue_step_static(WfHandle* h, unsigned char* base, int64_t* launches) {
                 if (which == 0) e = wf_split_ssf_wave(h->F, g, sw, lc);
                 else if (which == 1) e = wf_split_overland_wave(h->F, g, sw, lc);
                 else e = wf_split_river_wave(h->F, g, sw, lc);
-            } else if (which == 0) {
-                e = split ? wf_split_ssf(h->F, g, sw, lc) : wf_fp64_ssf(h->F, g, sw, lc);
-            } else if (which == 1) {
-                e = wf_fp64_overland(h->F, g, sw, lc);
             } else {
-                e = wf_fp64_river(h->F, g, sw, lc);
+                e = split ? wf_split_ssf(h->F, g, sw, lc) : wf_fp64_ssf(h->F, g, sw, lc);
             }
             CK(e);
             ++nl;

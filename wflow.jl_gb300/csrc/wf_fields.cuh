@@ -177,7 +177,18 @@ struct WfDevFields {
     // word, published by the overland wavefront for a river wavefront sharing its launch
     // (filled with the sentinel pattern before such a launch)
     unsigned long long* rv_lat_pub;  // [river slots * M]
+    // FP64 form: terms of the sweep in hand, per element of its graph, written by the per-cell kernel
+    // before the slim wavefront and read by it (WfW64Kw, WfW64Ssf); [max(land, river slots) * M] each
+    double* W[10];
 };
+
+// Surface kinematic wave: KwState of the previous discharge, dt q_lat, dt / dx, 5 dt / dx, 3 alpha, and
+// (written by the wavefront) the final iterate.
+enum WfW64Kw { W_U = 0, W_A, W_P, W_DF, W_RDF, W_B, W_DTDX, W_C1, W_C2, W_UEND };
+// Subsurface kinematic wave: dt / dx, 1 / celerity, their sum and its reciprocal, q_prev / celerity, the
+// net flux, the discharge limit, the net fluxes up to which the water table rises (falls) by less
+// than the sub-iteration threshold and stays above the soil bottom, and the sweep's discharge.
+enum WfW64Ssf { W_SDTDX = 0, W_CINV, W_SDF, W_SRDF, W_QPC, W_QNET, W_QLIM, W_RISE, W_FALL, W_Q };
 
 // Routing graph on the device (one per land / river graph).
 struct WfDevGraph {
@@ -210,6 +221,12 @@ struct WfDevGraph {
     // land graph: per slot, the fractions to the river of the heavy child and of light children
     // 0 and 1 (up_frf of those entries; 0 where absent)
     const float4* up_frec;
+    // FP64 form: upstream records of the slim wavefronts (wf_wave64.cuh Rec), and per land slot
+    // {1 - fraction to the river, fraction} of the heavy child and of light children 0 and 1
+    const int4* up_rec64;
+    const double* up_w64;
+    int32_t lanes64;        // FP64 form: packing lanes per chain-member pair of the slim wavefronts,
+    int32_t lanes64_multi;  // and the most of them that a launch of several sub-steps is worth
     uint32_t* flags;      // [n_chains * M] epoch of the last published sub-step
     double* end_q;        // [n_chains * M * s_cap] q of each chain end per sub-step
     unsigned long long* ticket;  // work counter of the current launch
@@ -238,6 +255,7 @@ struct WfSweep {
     uint32_t epoch0;      // epoch of sub-step 0 of this launch
     double dt;            // model step
     const double* dts;    // [S] sub-step sizes (device)
+    double dt_s;          // FP64 slim wavefronts, fixed sub-steps: their common size
     int64_t prio_items;   // work items dispatched first (the longest chains), set at launch
     float dts_f[16];      // FP32 copy of the first 16 sub-step sizes (split form's slim walkers)
     uint64_t wait_ns;     // spin-wait budget per wait [ns]

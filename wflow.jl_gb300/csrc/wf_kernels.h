@@ -20,6 +20,9 @@ struct WfLaunchCfg {
 // FP64 plain form (kernels_fp64.cu)
 cudaError_t wf_fp64_vertical(const WfDevFields& F, const WfLaunchCfg& c);
 cudaError_t wf_fp64_ssf(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c);
+// slim wavefronts (wf_wave64.cuh), each with its per-cell kernels before and after it; the subsurface
+// one takes a single sub-step per model step
+cudaError_t wf_fp64_ssf_wave(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c);
 cudaError_t wf_fp64_overland(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c);
 cudaError_t wf_fp64_river(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c);
 cudaError_t wf_fp64_balance(const WfDevFields& F, const WfLaunchCfg& c);
