@@ -1291,8 +1291,9 @@ __global__ void __launch_bounds__(128) kw_post64_kernel(WfDevFields F, WfDevGrap
 }
 
 template <class Phys, bool MULTI>
-__global__ void __launch_bounds__(128) wave64_kernel(Phys phys, int64_t p_chunks, int SLp, int SLr, int batch) {
-    wfz::walk<Phys, MULTI>(phys, p_chunks, SLp, SLr, batch, phys.F.status);
+__global__ void __launch_bounds__(128) wave64_kernel(Phys phys, int64_t p_chunks, int SLp, int SLs, int SLr,
+                                                     int batch) {
+    wfz::walk<Phys, MULTI>(phys, p_chunks, SLp, SLs, SLr, batch, phys.F.status);
 }
 
 // --------------------------------------------------------- gravitational snow transport ----
@@ -1623,19 +1624,20 @@ namespace {
 // Launch of a slim wavefront. Long chains (as many as half of the resident warps take) go first, each
 // in a warp of its own; the lanes beyond a chain's sub-steps stay idle, because one lane's long solve
 // (a drained cell that gets water again takes up to 75 iterations) holds up its whole warp. The other
-// chains are packed as loosely as their number allows: the plan's packing lanes (wave64_lanes).
+// chains are packed as loosely as their number allows (wave_lanes).
 template <class Phys, bool MULTI>
 cudaError_t launch_wave64(const Phys& phys, const WfLaunchCfg& c) {
     const int threads = 32 * (c.walk_warps > 0 ? std::min(c.walk_warps, 4) : 4);
     const size_t smem = wfz::walk_smem(threads);
     const WfDevGraph& g = phys.g;
     const int SLp = g.M == 1 ? 32 : 1 << (31 - __builtin_clz(32 / std::min(g.M, 32) | 1));
-    int SLr = g.lanes64;
+    int SLr = g.lanes, SLs = SLr;
     if (MULTI) {
         const int cap = c.sub_lanes > 0 ? std::min(c.sub_lanes, 32) : 32;
         int need = 1;
         while (need < phys.sw.S && need < cap) need <<= 1;
-        SLr = c.sub_lanes > 0 ? need : std::max(SLr, std::min(need, g.lanes64_multi));
+        SLr = c.sub_lanes > 0 ? need : std::max(SLr, std::min(need, g.lanes_multi));
+        SLs = SLr;
     }
     int per_sm = 0;
     const cudaError_t err =
@@ -1647,15 +1649,14 @@ cudaError_t launch_wave64(const Phys& phys, const WfLaunchCfg& c) {
     const int fill = std::min(per_sm, 2);
     int blocks = c.walk_blocks > 0 ? c.walk_blocks : c.num_sms * fill;
     const int wpb = threads / 32;
-    const int64_t ipp = wf_items_per_chunk(1, g.M, SLp);
     const int64_t items = g.n_chunks * wf_items_per_chunk(g.G, g.M, SLr);
     const int64_t need = std::max<int64_t>((items + wpb - 1) / wpb, 1);
     if (blocks > need) blocks = (int)need;
     const int64_t resident = (int64_t)std::min(blocks, c.num_sms * per_sm) * wpb;
-    const int64_t p_chunks = std::min<int64_t>(g.n_long_chunks, resident / 2 / ipp);
+    const int64_t p_chunks = first_chunks(g, SLp, resident);
     // batches of short chains only where there are more items than warps
     const int batch = (int)std::max<int64_t>(1, std::min<int64_t>(wfv::BATCH, items / (4 * resident)));
-    wave64_kernel<Phys, MULTI><<<blocks, threads, smem, c.stream>>>(phys, p_chunks, SLp, SLr, batch);
+    wave64_kernel<Phys, MULTI><<<blocks, threads, smem, c.stream>>>(phys, p_chunks, SLp, SLs, SLr, batch);
     return cudaGetLastError();
 }
 

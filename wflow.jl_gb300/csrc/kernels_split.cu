@@ -1025,14 +1025,13 @@ __global__ void __launch_bounds__(256, 2) vertical_split_kernel(WfDevFields F) {
             ff flux = wff::mul(recharge, WS ? ff{W32[VW_AREA_HI], W32[VW_AREA_LO]} : lds(F, AREA, slot));  // recharge flux of the subsurface model
             if (zi >= d_soil) flux = wff::fmax0(flux);
             stm(F, SSF_QNET, e, flux);
-            Mh[SSF_QNETF][e] = wff::to_f(flux);
-            Mh[SSF_ZIF][e] = zif;
             float z = zif;
             if (kv_const && !(z < zexp)) z = zexp;
             const float cel = p_kh_ratio * kv0 * expf(-fsc * z) * p_slope / p_sy;
             const float cinv = 1.0f / cel;
-            Mh[SSF_T2][e] = wff::to_f(VF(VS_SSFQ_H, VS_SSFQ_L)) * cinv;
-            Mh[SSF_RDF][e] = 1.0f / (p_ssf_dtdx + cinv);
+            const ff ssfq = VF(VS_SSFQ_H, VS_SSFQ_L);
+            const float rdf = 1.0f / (p_ssf_dtdx + cinv);
+            F.ssf_dyn[e] = make_float4(wff::to_f(flux), wff::to_f(ssfq) * cinv, ssfq.hi == 0.0f ? -rdf : rdf, zif);
             // deepest unsaturated layer: what a rising water table fills first
             float rth = 0.0f, rcap = 0.0f, rrho = 0.0f;
             const float dts = (float)F.dt_ssf;
@@ -1044,9 +1043,7 @@ __global__ void __launch_bounds__(256, 2) vertical_split_kernel(WfDevFields F) {
                 rcap = fmaxf(rth * te - uk, 0.0f) / dts;
                 rrho = dts / (te - uk / rth);
             }
-            Mh[SSF_RTH][e] = rth;
-            Mh[SSF_RCAP][e] = rcap;
-            Mh[SSF_RRHO][e] = rrho;
+            F.ssf_dyn[F.land_slots * M + e] = make_float4(rth, rcap, rrho, Mh[Q_MAX][e]);
         }
     }
 }
@@ -1242,7 +1239,8 @@ struct SsfSplitPhys {
         const double inwater = net_runoff * area;
         Mf[OL_INWATER][e] = inwater;
         const double qlat = inwater / L[FLOW_LENGTH][slot];
-        Mf[OL_QLAT][e] = qlat;
+        const wff::ff ql = wff::from_d(qlat);
+        F.ol_lat[e] = make_float2(ql.hi, ql.lo);
         return true;
     }
 };
@@ -1254,8 +1252,9 @@ struct SsfSplitPhys {
 
 // Root of dt_dx u^5 + alpha u^3 = cterm for the kinematic wave in u = Q^0.2 (the reference's
 // Newton-Raphson on Q, surface_process.jl:24-70, written for u), in double-FP32: Newton
-// iterations in FP32 from the upper bound min((cterm/alpha)^(1/3), (cterm/dt_dx)^(1/5)) (or
-// from the previous u when it lies below that bound) until |du| <= 3e-7 u, then one Newton
+// iterations in FP32 from the previous u, held below the upper bound min((cterm/alpha)^(1/3),
+// (cterm/dt_dx)^(1/5)) (computed beside the first iteration; the start without a previous u), until
+// |du| <= 1e-4 u (an error below 2 du^2 / u, less than the rounding of FP32), then one Newton
 // correction with the residual evaluated in double-FP32, which leaves |f(u)| at about 1e-13 of
 // cterm. Q = u^5 is formed from the correction du as v^5 - 5 v^4 du (the dropped terms are of
 // relative size (du/v)^2). Results below the reference's floor (u = QROOT) are raised to it, as
@@ -1280,7 +1279,7 @@ __device__ __forceinline__ void kw_solve_ff(wff::ff cterm, wff::ff dt_dx, float 
     }
     const float a = dt_dx.hi, b = alpha, c = cterm.hi;
     const float ub = 1.00001f * fminf(__powf(__fdividef(c, b), 1.0f / 3.0f), __powf(__fdividef(c, a), 0.2f));
-    float v = (u_prev > 0.0f && u_prev < ub) ? u_prev : ub;
+    float v = u_prev > 0.0f ? u_prev : ub;
     const float a5 = 5.0f * a, b3 = 3.0f * b;
 #pragma unroll 1
     for (int it = 0; it < 12; ++it) {
@@ -1289,7 +1288,7 @@ __device__ __forceinline__ void kw_solve_ff(wff::ff cterm, wff::ff dt_dx, float 
         const float dg = v2 * fmaf(a5, v2, b3);
         const float dv = __fdividef(g, dg);
         v = fminf(v - dv, ub);
-        if (!(fabsf(dv) > 3e-7f * v)) break;
+        if (!(fabsf(dv) > 1e-4f * v)) break;
     }
     const wff::ff v2 = wff::two_prod(v, v);
     const wff::ff v3 = wff::mul(v2, v);
@@ -1445,7 +1444,6 @@ enum SsfFlag { SSF_FAST = 0, SSF_EARLY = 1, SSF_FULL = 2, SSF_CUT = 3 };
 
 template <int MAXN>
 struct SsfWave {
-    static constexpr int kDepth = 1;  // the per-node inputs are many: one position ahead
     WfDevFields F;
     WfDevGraph g;
     WfSweep sw;
@@ -1454,69 +1452,47 @@ struct SsfWave {
         bool qprev_zero;
         wfv::UpRec up;
     };
-    __device__ __forceinline__ void load(int64_t slot, int64_t e, int m, In& x) const {
-        float* const* Mh = F.Mh;
-        float* const* Lf = F.Lf;
-        x.qnet = Mh[SSF_QNETF][e];
-        x.t2 = Mh[SSF_T2][e];
-        x.rdf = Mh[SSF_RDF][e];
-        x.zi = Mh[SSF_ZIF][e];
-        x.rth = Mh[SSF_RTH][e];
-        x.rcap = Mh[SSF_RCAP][e];
-        x.rrho = Mh[SSF_RRHO][e];
-        x.qmaxdw = Mh[Q_MAX][e] * Lf[FLOW_WIDTH][slot];
-        x.d = Lf[SOIL_THICKNESS][slot];
-        x.dtdx = Lf[SSF_DTDX][slot];
-        x.idwdx = Lf[SSF_IDWDX][slot];
-        x.dtsy = Lf[SSF_DTSY][slot];
-        x.k2 = Lf[SSF_K2][slot];
-        x.qprev_zero = F.Mh[SSF_Q][e] == 0.0f;
-        wfv::load_rec<true>(g, slot, x.up);
-    }
-    // the same inputs staged in shared memory (wfv::walk_ring)
-    static constexpr int kSweep = 0;  // bit of WfLaunchCfg::walk_inputs
-    static constexpr int kWords = 15;
+    static constexpr int kVecs = 4;
     static constexpr bool kWeighted = true;
-    __device__ __forceinline__ void sources(int64_t slot, int64_t e, const void** src) const {
-        float* const* Mh = F.Mh;
-        float* const* Lf = F.Lf;
-        src[0] = &Mh[SSF_QNETF][e];
-        src[1] = &Mh[SSF_T2][e];
-        src[2] = &Mh[SSF_RDF][e];
-        src[3] = &Mh[SSF_ZIF][e];
-        src[4] = &Mh[SSF_RTH][e];
-        src[5] = &Mh[SSF_RCAP][e];
-        src[6] = &Mh[SSF_RRHO][e];
-        src[7] = &Mh[Q_MAX][e];
-        src[8] = &Lf[FLOW_WIDTH][slot];
-        src[9] = &Lf[SOIL_THICKNESS][slot];
-        src[10] = &Lf[SSF_DTDX][slot];
-        src[11] = &Lf[SSF_IDWDX][slot];
-        src[12] = &Lf[SSF_DTSY][slot];
-        src[13] = &Lf[SSF_K2][slot];
-        src[14] = &Mh[SSF_Q][e];
+    __device__ __forceinline__ void copy(int64_t slot, int64_t e, float4* v) const {
+        wfv::cpa(v, &F.ssf_dyn[e]);
+        wfv::cpa(v + 32, &F.ssf_dyn[F.land_slots * g.M + e]);
+        wfv::cpa(v + 64, &F.ssf_st[slot]);
+        wfv::cpa(v + 96, &F.ssf_st[F.land_slots + slot]);
     }
-    __device__ __forceinline__ void from_words(const uint32_t* w, int st, In& x) const {
-        auto f = [&](int i) { return __uint_as_float(w[i * st]); };
-        x.qnet = f(0);
-        x.t2 = f(1);
-        x.rdf = f(2);
-        x.zi = f(3);
-        x.rth = f(4);
-        x.rcap = f(5);
-        x.rrho = f(6);
-        x.qmaxdw = f(7) * f(8);
-        x.d = f(9);
-        x.dtdx = f(10);
-        x.idwdx = f(11);
-        x.dtsy = f(12);
-        x.k2 = f(13);
-        x.qprev_zero = f(14) == 0.0f;
+    __device__ __forceinline__ void from_vecs(const float4* v, In& x) const {
+        const float4 a = v[0], b = v[32], c = v[64], d = v[96];
+        x.qnet = a.x;
+        x.t2 = a.y;
+        x.rdf = fabsf(a.z);
+        x.qprev_zero = __float_as_int(a.z) < 0;
+        x.zi = a.w;
+        x.rth = b.x;
+        x.rcap = b.y;
+        x.rrho = b.z;
+        x.qmaxdw = b.w * d.z;
+        x.d = c.x;
+        x.dtdx = c.y;
+        x.idwdx = c.z;
+        x.dtsy = c.w;
+        x.k2 = d.x;
+        x.up.w_hv = d.y;
+        x.up.n_lt = __float_as_int(d.w);
     }
-    __device__ __forceinline__ bool node(const In& x, const wfv::Ends& ends, int64_t slot, int64_t e, int m,
-                                         int64_t chain, bool is_end, bool heavy, unsigned long long* qh) {
+    struct Pass {
+        uint32_t none;
+    };
+    __device__ __forceinline__ void pack(const In&, Pass&) const {}
+    __device__ __forceinline__ void unpack(const Pass&, In&) const {}
+    struct St {};
+    __device__ __forceinline__ void start(const In&, St&) const {}
+    __device__ __forceinline__ bool active(int, bool& first) const { return true; }
+    __device__ __forceinline__ void finish(const St&, int64_t, bool) const {}
+    __device__ __forceinline__ bool sub(const In& x, St&, unsigned long long w0, unsigned long long w1, int64_t slot,
+                                        int64_t e, int m, int s, int64_t chain, bool is_end, bool heavy,
+                                        unsigned long long qh_in, unsigned long long& qh_out) const {
         wff::ff qinff;
-        if (!wfv::gather<true>(g, sw, x.up, ends, slot, m, 0, heavy, qh[0], F.status, qinff)) return false;
+        if (!wfv::gather_w<true>(g, sw, x.up, w0, w1, slot, m, 0, heavy, qh_in, F.status, qinff)) return false;
         const float qin = qinff.hi + qinff.lo;
         float q = 0.0f, qu = 0.0f;
         int flag;
@@ -1565,14 +1541,10 @@ struct SsfWave {
                 flag = SSF_FULL;
             }
         }
-        float* const* Mh = F.Mh;
         const wff::ff qf = {q, 0.0f};
-        qh[0] = wff::pack(qf);
+        qh_out = wff::pack(qf);
         if (is_end) wfv::publish(g, chain, m, 0, qf);
-        Mh[SSF_QF][e] = q;
-        Mh[SSF_QUF][e] = qu;
-        Mh[SSF_QINF][e] = qin;
-        Mh[SSF_FLAG][e] = (float)flag;
+        F.ssf_out[e] = make_float4(q, qu, qin, (float)flag);
         return true;
     }
 };
@@ -1580,8 +1552,7 @@ struct SsfWave {
 // The lateral inflow of river cell rs (element re) from the land cell of element le, with trsum
 // the step's sum of the overland flow to the river (update_lateral_inflow!,
 // surface_kinwave.jl:710-734): stores the river cell's inflow, lateral inflow and the lateral
-// inflow with the external inflow, and returns the latter. One function for the overland
-// wavefront and the per-cell completion kernel, so both give the same words.
+// inflow with the external inflow, and returns the latter. 
 __device__ __forceinline__ wff::ff river_lateral(const WfDevFields& F, int64_t le, int64_t rs, int64_t re,
                                                  wff::ff trsum) {
     using wff::ff;
@@ -1594,8 +1565,7 @@ __device__ __forceinline__ wff::ff river_lateral(const WfDevFields& F, int64_t l
     str(F, RV_QLAT, re, qlat);
     const float ext = F.Rf[R_EXT_INFLOW][rs];
     const ff qlt = ext < 0.0f ? qlat : wff::add(qlat, wff::mul(inv_len, ext));
-    F.RMh[RV_QLATTH][re] = qlt.hi;
-    F.RMh[RV_QLATTL][re] = qlt.lo;
+    F.rv_lat[re] = make_float2(qlt.hi, qlt.lo);
     return qlt;
 }
 
@@ -1605,77 +1575,61 @@ __device__ __forceinline__ wff::ff river_lateral(const WfDevFields& F, int64_t l
 // At the land cell of a river cell the walker also sums the upstream discharge that goes to the
 // river (q of each upstream cell times its flow fraction to the river, times the sub-step;
 // to_river_cumulative, surface_kinwave.jl:310-318), the only cells where it is not zero
-// (get_flow_fraction_to_river, utils.jl:485-505). FUSE: a river wavefront shares the launch;
-// after the step's last sub-step the walker publishes the river cell's lateral inflow for it
-// (F.rv_lat_pub).
-template <bool ADAPT, bool FUSE = false>
+// (get_flow_fraction_to_river, utils.jl:485-505).
+template <bool ADAPT>
 struct OlWave {
-    static constexpr int kDepth = 2;
     WfDevFields F;
     WfDevGraph g;
     WfSweep sw;
     struct In {
         wff::ff u, q, qlat, invdx;
-        float alpha;
-        bool sfw_pos;
+        float alpha;          // negative: no surface flow width
         int32_t rs;           // river slot of the cell, or -1
         float fr_hv, fr0, fr1;  // fractions to the river of the heavy child and light children 0, 1
         wfv::UpRec up;
     };
-    __device__ __forceinline__ void load_river(int64_t slot, In& x) const {
-        if (x.rs >= 0) {
-            const float4 f = g.up_frec[slot];
-            x.fr_hv = f.x;
-            x.fr0 = f.y;
-            x.fr1 = f.z;
-        } else {
-            x.fr_hv = x.fr0 = x.fr1 = 0.0f;
-        }
-    }
-    __device__ __forceinline__ void load(int64_t slot, int64_t e, int m, In& x) const {
-        float* const* Mh = F.Mh;
-        x.u = {Mh[OL_UH][e], Mh[OL_UL][e]};
-        x.q = ldm(F, OL_Q, e);
-        x.qlat = ldm(F, OL_QLAT, e);
-        x.invdx = {F.Lf[INV_FLOW_LENGTH][slot], F.Lf[INV_DX_LO][slot]};
-        x.alpha = F.Lf[OL_ALPHA][slot];
-        x.sfw_pos = F.Lf[SFW][slot] > 0.0f;
-        x.rs = (int32_t)F.land_river_slot[slot];
-        load_river(slot, x);
-        wfv::load_rec<true>(g, slot, x.up);
-    }
-    // the same inputs staged in shared memory (wfv::walk_ring)
-    static constexpr int kSweep = 1;
-    static constexpr int kWords = 14;
+    static constexpr int kVecs = 4;
     static constexpr bool kWeighted = true;
-    __device__ __forceinline__ void sources(int64_t slot, int64_t e, const void** src) const {
-        src[0] = &F.Mh[OL_UH][e];
-        src[1] = &F.Mh[OL_UL][e];
-        src[2] = &F.Mh[OL_Q][e];
-        src[3] = &F.Ml[OL_Q][e];
-        src[4] = &F.Mh[OL_QLAT][e];
-        src[5] = &F.Ml[OL_QLAT][e];
-        src[6] = &F.Lf[INV_FLOW_LENGTH][slot];
-        src[7] = &F.Lf[INV_DX_LO][slot];
-        src[8] = &F.Lf[OL_ALPHA][slot];
-        src[9] = &F.Lf[SFW][slot];
-        src[10] = &F.land_river_slot[slot];  // the low word (slots < 2^31; -1 stays -1)
-        src[11] = &g.up_frec[slot].x;
-        src[12] = &g.up_frec[slot].y;
-        src[13] = &g.up_frec[slot].z;
+    __device__ __forceinline__ void copy(int64_t slot, int64_t e, float4* v) const {
+        wfv::cpa(v, &F.ol_uq[e]);
+        wfv::cpa(v + 32, &F.ol_lat[e]);
+        wfv::cpa(v + 64, &F.ol_st[slot]);
+        wfv::cpa(v + 96, &F.ol_st[F.land_slots + slot]);
     }
-    __device__ __forceinline__ void from_words(const uint32_t* w, int st, In& x) const {
-        auto f = [&](int i) { return __uint_as_float(w[i * st]); };
-        x.u = {f(0), f(1)};
-        x.q = {f(2), f(3)};
-        x.qlat = {f(4), f(5)};
-        x.invdx = {f(6), f(7)};
-        x.alpha = f(8);
-        x.sfw_pos = f(9) > 0.0f;
-        x.rs = (int32_t)w[10 * st];
-        x.fr_hv = f(11);
-        x.fr0 = f(12);
-        x.fr1 = f(13);
+    __device__ __forceinline__ void from_vecs(const float4* v, In& x) const {
+        const float4 a = v[0], c = v[64], d = v[96];
+        const float2 b = *reinterpret_cast<const float2*>(v + 32);
+        x.u = {a.x, a.y};
+        x.q = {a.z, a.w};
+        x.qlat = {b.x, b.y};
+        x.invdx = {c.x, c.y};
+        x.alpha = c.z;
+        const int32_t rs = __float_as_int(c.w);
+        x.rs = (rs & 0x7fffffff) - 1;
+        x.up.n_lt = rs < 0 ? 3 : 0;
+        x.up.w_hv = d.x;
+        x.fr_hv = d.y;
+        x.fr0 = d.z;
+        x.fr1 = d.w;
+    }
+    // what the later sub-steps of a node need of its inputs
+    struct Pass {
+        wff::ff qlat, invdx;
+        float alpha, w_hv, fr_hv, fr0, fr1;
+        int32_t n_lt;
+    };
+    __device__ __forceinline__ void pack(const In& x, Pass& p) const {
+        p = {x.qlat, x.invdx, x.alpha, x.up.w_hv, x.fr_hv, x.fr0, x.fr1, x.up.n_lt};
+    }
+    __device__ __forceinline__ void unpack(const Pass& p, In& x) const {
+        x.qlat = p.qlat;
+        x.invdx = p.invdx;
+        x.alpha = p.alpha;
+        x.up.w_hv = p.w_hv;
+        x.fr_hv = p.fr_hv;
+        x.fr0 = p.fr0;
+        x.fr1 = p.fr1;
+        x.up.n_lt = p.n_lt;
     }
     struct St {
         wff::ff u, qp, qsum, trsum;
@@ -1688,14 +1642,18 @@ struct OlWave {
         st.trsum = {0.0f, 0.0f};
         st.rs = x.rs;
     }
-    // entry hook of the diagonal schedule (nothing to wait for)
-    __device__ __forceinline__ bool enter(St&, int64_t) const { return true; }
+    __device__ __forceinline__ bool active(int m, bool& first) const {
+        if (!ADAPT) return true;
+        const uint8_t f = sw.aflag[m];
+        first = (f & WF_SUB_FIRST) != 0;
+        return (f & WF_SUB_ACTIVE) != 0;
+    }
     // gather_w<true> with, at the land cell of a river cell, the upstream flow to the river
-    __device__ __forceinline__ bool gather_tr(const In& x, unsigned long long w0, unsigned long long w1, int64_t slot,
-                                              int m, int s, bool heavy, unsigned long long qh, wff::ff& qin,
+    __device__ __forceinline__ bool gather_tr(const In& x, int32_t rs, unsigned long long w0, unsigned long long w1,
+                                              int64_t slot, int m, int s, bool heavy, unsigned long long qh, wff::ff& qin,
                                               wff::ff& tr) const {
         const wfv::UpRec& r = x.up;
-        const bool riv = x.rs >= 0;
+        const bool riv = rs >= 0;
         wff::ff acc = {0.0f, 0.0f}, t = {0.0f, 0.0f};
         if (heavy) {
             const wff::ff q = wff::unpack(qh);
@@ -1748,26 +1706,24 @@ struct OlWave {
         if constexpr (ADAPT) dt_s = wff::ff{sw.adt_hi[m], sw.adt_lo[m]};
         else dt_s = sw.dts_f[s];
         wff::ff qin, tr;
-        if (!gather_tr(x, w0, w1, slot, m, s, heavy, qh_in, qin, tr)) return false;
-        if (!x.sfw_pos) qin = {0.0f, 0.0f};
+        if (!gather_tr(x, st.rs, w0, w1, slot, m, s, heavy, qh_in, qin, tr)) return false;
+        if (__float_as_int(x.alpha) < 0) qin = {0.0f, 0.0f};
         wff::ff un, qn;
-        kw_node_ff<ADAPT>(qin, st.qp, x.qlat, st.u, x.invdx, dt_s, x.alpha, un, qn);
+        kw_node_ff<ADAPT>(qin, st.qp, x.qlat, st.u, x.invdx, dt_s, fabsf(x.alpha), un, qn);
         st.u = un;
         st.qp = qn;
         qh_out = wff::pack(qn);
         if (is_end) wfv::publish(g, chain, m, s, qn);
         st.qsum = wff::add(st.qsum, mul_dt(qn, dt_s));
-        if (x.rs >= 0) st.trsum = wff::add(st.trsum, mul_dt(tr, dt_s));
+        if (st.rs >= 0) st.trsum = wff::add(st.trsum, mul_dt(tr, dt_s));
         return true;
     }
     // the node's state after the last sub-step of the launch (or of a round of the diagonal
     // schedule); add_stored: the step's cumulative discharge so far is added. At the land cell of
-    // a river cell, the flow to the river goes to the river cell's element; with FUSE, after the
-    // step's last sub-step, the river cell's lateral inflow is published.
+    // a river cell, the flow to the river goes to the river cell's element.
     __device__ __forceinline__ void finish(const St& st, int64_t e, bool add_stored) const {
         float* const* Mh = F.Mh;
-        Mh[OL_UH][e] = st.u.hi;
-        Mh[OL_UL][e] = st.u.lo;
+        F.ol_uq[e] = make_float4(st.u.hi, st.u.lo, st.qp.hi, st.qp.lo);
         stm(F, OL_Q, e, st.qp);
         wff::ff qsum = st.qsum;
         if (add_stored) qsum = wff::add(qsum, wff::ff{Mh[OL_QSUMH][e], Mh[OL_QSUML][e]});
@@ -1780,30 +1736,7 @@ struct OlWave {
             if (add_stored) trsum = wff::add(trsum, wff::ff{F.RMh[RV_TRSUMH][re], F.RMh[RV_TRSUML][re]});
             F.RMh[RV_TRSUMH][re] = trsum.hi;
             F.RMh[RV_TRSUML][re] = trsum.lo;
-            if (FUSE && sw.last_of_step)
-                wfv::st_relaxed(&F.rv_lat_pub[re], wff::pack(river_lateral(F, e, st.rs, re, trsum)));
         }
-    }
-    __device__ __forceinline__ bool node(const In& x, const wfv::Ends& ends, int64_t slot, int64_t e, int m,
-                                         int64_t chain, bool is_end, bool heavy, unsigned long long* qh) {
-        const int stride = blockDim.x;
-        bool first = sw.first == 0;
-        if (ADAPT) {
-            const uint8_t f = sw.aflag[m];
-            if (!(f & WF_SUB_ACTIVE)) return true;
-            first = (f & WF_SUB_FIRST) != 0;
-        }
-        St st;
-        start(x, st);
-        for (int s = 0; s < sw.S; ++s) {
-            unsigned long long out;
-            if (!sub(x, st, wfv::end_word0(ends, s), s == 0 ? ends.lq1 : wfv::SENTINEL, slot, e, m, s, chain, is_end,
-                     heavy, qh[s * stride], out))
-                return false;
-            qh[s * stride] = out;
-        }
-        finish(st, e, !first);
-        return true;
     }
 };
 
@@ -1813,12 +1746,8 @@ struct OlWave {
 // RES: the model has reservoirs. At a reservoir cell the reservoir update follows the cell's
 // kinematic wave in every sub-step (FP64, wf_reservoir.cuh) and the reservoir's outflow, not the
 // cell's discharge, is handed downstream (heavy hand-off row and published chain end alike).
-// FUSE: the overland wavefront shares the launch (its tickets first); a node takes its lateral
-// inflow from the word the overland walker publishes at the river cell's land cell
-// (F.rv_lat_pub), waiting for it like for a light child.
-template <bool ADAPT, bool RES, bool FUSE = false>
+template <bool ADAPT, bool RES>
 struct RvWave {
-    static constexpr int kDepth = 2;
     WfDevFields F;
     WfDevGraph g;
     WfSweep sw;
@@ -1828,47 +1757,44 @@ struct RvWave {
         int32_t res;  // reservoir at this cell (RES only), or -1
         wfv::UpRec up;
     };
-    __device__ __forceinline__ void load(int64_t slot, int64_t e, int m, In& x) const {
-        float* const* RMh = F.RMh;
-        x.u = {RMh[RV_UH][e], RMh[RV_UL][e]};
-        x.q = ldr(F, RV_Q, e);
-        x.qlatt = {RMh[RV_QLATTH][e], RMh[RV_QLATTL][e]};
-        x.invlen = {F.Rf[R_INV_LENGTH][slot], F.Rf[R_INV_LEN_LO][slot]};
-        x.alpha = F.Rf[R_ALPHA][slot];
-        x.len = F.Rf[R_LENGTH][slot];
-        x.ext = F.Rf[R_EXT_INFLOW][slot];
-        x.res = RES ? F.res_of_rslot[slot] : -1;
-        wfv::load_rec<false>(g, slot, x.up);
-    }
-    // the same inputs staged in shared memory (wfv::walk_ring)
-    static constexpr int kSweep = 2;
-    static constexpr int kWords = 12;
+    static constexpr int kVecs = 4;
     static constexpr bool kWeighted = false;
-    __device__ __forceinline__ void sources(int64_t slot, int64_t e, const void** src) const {
-        float* const* RMh = F.RMh;
-        src[0] = &RMh[RV_UH][e];
-        src[1] = &RMh[RV_UL][e];
-        src[2] = &F.RMh[RV_Q][e];
-        src[3] = &F.RMl[RV_Q][e];
-        src[4] = &RMh[RV_QLATTH][e];
-        src[5] = &RMh[RV_QLATTL][e];
-        src[6] = &F.Rf[R_INV_LENGTH][slot];
-        src[7] = &F.Rf[R_INV_LEN_LO][slot];
-        src[8] = &F.Rf[R_ALPHA][slot];
-        src[9] = &F.Rf[R_LENGTH][slot];
-        src[10] = &F.Rf[R_EXT_INFLOW][slot];
-        src[11] = RES ? (const void*)&F.res_of_rslot[slot] : (const void*)&F.Rf[R_ALPHA][slot];
+    __device__ __forceinline__ void copy(int64_t slot, int64_t e, float4* v) const {
+        wfv::cpa(v, &F.rv_uq[e]);
+        wfv::cpa(v + 32, &F.rv_lat[e]);
+        wfv::cpa(v + 64, &F.rv_st[slot]);
+        wfv::cpa(v + 96, &F.rv_st[F.river_slots + slot]);
     }
-    __device__ __forceinline__ void from_words(const uint32_t* w, int st, In& x) const {
-        auto f = [&](int i) { return __uint_as_float(w[i * st]); };
-        x.u = {f(0), f(1)};
-        x.q = {f(2), f(3)};
-        x.qlatt = {f(4), f(5)};
-        x.invlen = {f(6), f(7)};
-        x.alpha = f(8);
-        x.len = f(9);
-        x.ext = f(10);
-        x.res = RES ? (int32_t)w[11 * st] : -1;
+    __device__ __forceinline__ void from_vecs(const float4* v, In& x) const {
+        const float4 a = v[0], c = v[64], d = v[96];
+        const float2 b = *reinterpret_cast<const float2*>(v + 32);
+        x.u = {a.x, a.y};
+        x.q = {a.z, a.w};
+        x.qlatt = {b.x, b.y};
+        x.invlen = {c.x, c.y};
+        x.alpha = c.z;
+        x.len = c.w;
+        x.ext = d.x;
+        x.res = RES ? __float_as_int(d.y) : -1;
+        x.up.w_hv = 1.0f;
+        x.up.n_lt = __float_as_int(d.w);
+    }
+    // what the later sub-steps of a node need of its inputs
+    struct Pass {
+        wff::ff invlen;
+        float alpha, len, ext;
+        int32_t res, n_lt;
+    };
+    __device__ __forceinline__ void pack(const In& x, Pass& p) const {
+        p = {x.invlen, x.alpha, x.len, x.ext, x.res, x.up.n_lt};
+    }
+    __device__ __forceinline__ void unpack(const Pass& p, In& x) const {
+        x.invlen = p.invlen;
+        x.alpha = p.alpha;
+        x.len = p.len;
+        x.ext = p.ext;
+        x.res = RES ? p.res : -1;
+        x.up.n_lt = p.n_lt;
     }
     struct St {
         wff::ff u, qp, qsum, asum, qlatt;
@@ -1880,14 +1806,11 @@ struct RvWave {
         st.asum = {0.0f, 0.0f};
         st.qlatt = x.qlatt;
     }
-    // FUSE: the lateral inflow the overland walker publishes for element e (entry hook of both
-    // schedules); false when the wait ran out
-    __device__ __forceinline__ bool enter(St& st, int64_t e) const {
-        if (!FUSE) return true;
-        unsigned long long w;
-        if (!wfv::await_word(sw, &F.rv_lat_pub[e], F.status, w)) return false;
-        st.qlatt = wff::unpack(w);
-        return true;
+    __device__ __forceinline__ bool active(int m, bool& first) const {
+        if (!ADAPT) return true;
+        const uint8_t f = sw.aflag[m];
+        first = (f & WF_SUB_FIRST) != 0;
+        return (f & WF_SUB_ACTIVE) != 0;
     }
     // sub-step s of the node
     __device__ __forceinline__ bool sub(const In& x, St& st, unsigned long long w0, unsigned long long w1,
@@ -1930,8 +1853,7 @@ struct RvWave {
     // schedule); add_stored: the step's cumulative discharge and abstraction so far are added
     __device__ __forceinline__ void finish(const St& st, int64_t e, bool add_stored) const {
         float* const* RMh = F.RMh;
-        RMh[RV_UH][e] = st.u.hi;
-        RMh[RV_UL][e] = st.u.lo;
+        F.rv_uq[e] = make_float4(st.u.hi, st.u.lo, st.qp.hi, st.qp.lo);
         str(F, RV_Q, e, st.qp);
         wff::ff qsum = st.qsum, asum = st.asum;
         if (add_stored) {
@@ -1943,86 +1865,59 @@ struct RvWave {
         RMh[RV_ABSH][e] = asum.hi;
         RMh[RV_ABSL][e] = asum.lo;
     }
-    __device__ __forceinline__ bool node(const In& x, const wfv::Ends& ends, int64_t slot, int64_t e, int m,
-                                         int64_t chain, bool is_end, bool heavy, unsigned long long* qh) {
-        const int stride = blockDim.x;
-        bool first = sw.first == 0;
-        if (ADAPT) {
-            const uint8_t f = sw.aflag[m];
-            if (!(f & WF_SUB_ACTIVE)) return true;
-            first = (f & WF_SUB_FIRST) != 0;
-        }
-        St st;
-        start(x, st);
-        if (!enter(st, e)) return false;
-        for (int s = 0; s < sw.S; ++s) {
-            unsigned long long out;
-            if (!sub(x, st, wfv::end_word0(ends, s), s == 0 ? ends.lq1 : wfv::SENTINEL, slot, e, m, s, chain, is_end,
-                     heavy, qh[s * stride], out))
-                return false;
-            qh[s * stride] = out;
-        }
-        finish(st, e, !first);
-        return true;
-    }
 };
 
-template <class Phys>
-__global__ void __launch_bounds__(128) wave_kernel(Phys phys) {
-    wfv::walk(phys.g, phys.sw, phys, phys.F.status);
+template <class Phys, bool MULTI>
+__global__ void __launch_bounds__(128, 1) wave_kernel(Phys phys, int64_t p_chunks, int SLp, int SLs, int SLr,
+                                                   int batch) {
+    wfv::walk<Phys, MULTI>(phys, p_chunks, SLp, SLs, SLr, batch, phys.F.status);
 }
 
-template <class Phys>
-__global__ void __launch_bounds__(128) wave_diag_kernel(Phys phys) {
-    wfv::walk_diag(phys.g, phys.sw, phys, phys.F.status);
+// A sweep launch: as many long chains as half of the resident warps take go first, each in a warp of its
+// own, with a lane per sub-step (up to 32). Short chains are packed into full warps; those in between, on
+// whose ends the long ones wait, as loosely as their number allows (wave_lanes): a full warp takes two to
+// three times as long per position as a chain alone. In launches of one sub-step, whose positions are short,
+// eight of those chains share a warp at least.
+template <class Phys, bool MULTI>
+cudaError_t launch_wave_as(const Phys& phys, const WfLaunchCfg& c) {
+    const int threads = 32 * (c.walk_warps > 0 ? std::min(c.walk_warps, 4) : 4);
+    const WfDevGraph& g = phys.g;
+    const size_t smem = wfv::lean_smem(threads, Phys::kVecs);
+    auto kernel = wave_kernel<Phys, MULTI>;
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    int SLp = g.M == 1 ? 32 : 1, SLs = 1, SLr = std::min(g.lanes, 4);
+    if (MULTI) {
+        const int cap = c.sub_lanes > 0 ? std::min(c.sub_lanes, 32) : 32;
+        int need = 1;
+        while (need < phys.sw.S && need < cap) need <<= 1;
+        SLp = c.sub_lanes > 0 ? need : std::max(SLp, need);
+        SLs = std::min(need, c.sub_lanes > 0 ? 32 : 8);
+        SLr = c.sub_lanes > 0 ? need : std::max(g.lanes, std::min(need, g.lanes_multi));
+    }
+    int per_sm = 0;
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+    if (err != cudaSuccess) return err;
+    if (per_sm < 1) per_sm = 1;
+    int blocks = c.walk_blocks > 0 ? c.walk_blocks : c.num_sms * per_sm;
+    const int wpb = threads / 32;
+    const int64_t items = g.n_short_chunks * wf_items_per_chunk(g.G, g.M, SLs) +
+                          (g.n_chunks - g.n_short_chunks) * wf_items_per_chunk(g.G, g.M, SLr);
+    const int64_t need = std::max<int64_t>((items + wpb - 1) / wpb, 1);
+    if (blocks > need) blocks = (int)need;
+    const int64_t resident = (int64_t)std::min(blocks, c.num_sms * per_sm) * wpb;
+    const int64_t p_chunks = first_chunks(g, SLp, resident);
+    // Two short chunks a ticket where there are many more items than warps. Longer batches put a chunk's
+    // last chain behind those before it, and the chains that wait for it behind that. Hourly steps of a
+    // 1024 x 1024 domain: 8.7 ms with two and eight chains to a warp (SLr), 9.4 with eight and one.
+    const int batch = (int)std::max<int64_t>(1, std::min<int64_t>(wfv::BATCH, items / (2 * resident)));
+    kernel<<<blocks, threads, smem, c.stream>>>(phys, p_chunks, SLp, SLs, SLr, batch);
+    return cudaGetLastError();
 }
 
-template <class Phys>
-__global__ void __launch_bounds__(128) wave_ring_kernel(Phys phys) {
-    wfv::walk_ring(phys.g, phys.sw, phys, phys.F.status);
-}
-
-// Node-major sweeps: inputs staged in shared memory (walk_ring) unless the tuning asks for the
-// register pipeline (walk) for this sweep (bit Phys::kSweep of walk_inputs).
 template <class Phys>
 cudaError_t launch_wave(const Phys& phys, const WfLaunchCfg& c) {
-    const int threads = 32 * (c.walk_warps > 0 ? c.walk_warps : 4);
-    int blocks;
-    Phys p = phys;
-    p.sw.SL = 1;
-    if (!((c.walk_inputs >> Phys::kSweep) & 1)) {
-        const size_t smem = wfv::ring_smem(threads, phys.sw.S, Phys::kWords);
-        cudaError_t err = cudaFuncSetAttribute(wave_ring_kernel<Phys>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
-        if (err != cudaSuccess) return err;
-        err = wave_grid(wave_ring_kernel<Phys>, threads, smem, c, p.g, blocks, p.sw.prio_items);
-        if (err != cudaSuccess) return err;
-        wave_ring_kernel<Phys><<<blocks, threads, smem, c.stream>>>(p);
-        return cudaGetLastError();
-    }
-    const size_t smem = wfv::walk_smem(threads, phys.sw.S);
-    cudaError_t err = wave_grid(wave_kernel<Phys>, threads, smem, c, p.g, blocks, p.sw.prio_items);
-    if (err != cudaSuccess) return err;
-    wave_kernel<Phys><<<blocks, threads, smem, c.stream>>>(p);
-    return cudaGetLastError();
-}
-
-// Overland and river launches of several fixed sub-steps run on the diagonal schedule
-// (wfv::walk_diag); one sub-step per launch (and the subsurface sweep) node-major.
-template <class Phys>
-cudaError_t launch_wave_sub(const Phys& phys, const WfLaunchCfg& c) {
-    const int SL = wave_sub_lanes(phys.sw.S, c);
-    if (phys.sw.aflag || SL <= 1) return launch_wave(phys, c);
-    const int threads = 32 * (c.walk_warps > 0 ? c.walk_warps : 4);
-    const size_t smem = wfv::diag_smem(threads);
-    int blocks;
-    Phys p = phys;
-    p.sw.SL = SL;
-    cudaError_t err = wave_grid(wave_diag_kernel<Phys>, threads, smem, c, p.g, blocks, p.sw.prio_items,
-                                wf_items_per_chunk(p.g.G, p.g.M, SL));
-    if (err != cudaSuccess) return err;
-    wave_diag_kernel<Phys><<<blocks, threads, smem, c.stream>>>(p);
-    return cudaGetLastError();
+    return phys.sw.S > 1 ? launch_wave_as<Phys, true>(phys, c) : launch_wave_as<Phys, false>(phys, c);
 }
 
 // --------------------------------------------------------------- post-sweep kernels ------
@@ -2048,7 +1943,8 @@ __global__ void __launch_bounds__(256) ssf_post_kernel(WfDevFields F, WfDevGraph
         if (F.land_node_of_slot[slot] < 0) continue;
         const int m = (int)(e - slot * M);
         float* const* Mh = F.Mh;
-        const int flag = (int)Mh[SSF_FLAG][e];
+        const float4 swept = F.ssf_out[e];
+        const int flag = (int)swept.w;
         const double zi_soil = F.Mf[ZI][e];
         const ff zis = wff::from_d(zi_soil);
         const ff d = lds(F, SOIL_THICKNESS, slot);
@@ -2094,9 +1990,9 @@ __global__ void __launch_bounds__(256) ssf_post_kernel(WfDevFields F, WfDevGraph
 #pragma unroll
             for (int k = 0; k < MAXN; ++k) usld[k] = k < N ? ff{F.LYf[LY_USLD][k][e], F.LYl[k][e]} : ff{0.0f, 0.0f};
         } else {
-            q = wff::from_f(Mh[SSF_QF][e]);
-            qin = wff::from_f(Mh[SSF_QINF][e]);
-            const float qu = Mh[SSF_QUF][e];
+            q = wff::from_f(swept.x);
+            qin = wff::from_f(swept.z);
+            const float qu = swept.y;
             nf = wff::mul(wff::sub(wff::add(ldm(F, SSF_QNET, e), qin), qu), lds(F, SSF_IDWDX, slot));
             // water_table_change (subsurface_process.jl): falling by net flux / specific yield,
             // rising through the unsaturated layers from the deepest up
@@ -2155,7 +2051,7 @@ __global__ void __launch_bounds__(256) ssf_post_kernel(WfDevFields F, WfDevGraph
         const int nu = nu_at(zss);
         ff tr = {0.0f, 0.0f};
         for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o)
-            tr = wff::add(tr, wff::two_prod(Mh[SSF_QF][g.up_slot[o] * M + m], g.up_frf[o]));
+            tr = wff::add(tr, wff::two_prod(F.ssf_out[g.up_slot[o] * M + m].x, g.up_frf[o]));
         const ff area = lds(F, AREA, slot);
         const ff flux = ldm(F, SSF_QNET, e);
         stm(F, SSF_STORAGE, e, wff::mul(wff::mul(wff::sub(d, zin), F.Lf[SY][slot]), area));
@@ -2183,7 +2079,8 @@ __global__ void __launch_bounds__(256) ssf_post_kernel(WfDevFields F, WfDevGraph
         stm(F, NET_RUNOFF, e, net_runoff);
         const ff inwater = wff::mul(net_runoff, area);
         stm(F, OL_INWATER, e, inwater);
-        stm(F, OL_QLAT, e, wff::mul(inwater, lds(F, INV_FLOW_LENGTH, slot)));
+        const ff qlat = wff::mul(inwater, lds(F, INV_FLOW_LENGTH, slot));
+        F.ol_lat[e] = make_float2(qlat.hi, qlat.lo);
     }
 }
 
@@ -2202,7 +2099,8 @@ __global__ void __launch_bounds__(256) ol_post_kernel(WfDevFields F, WfDevGraph 
         float* const* Mh = F.Mh;
         const ff inv_sfw = lds(F, INV_SFW, slot);
         if (inv_sfw.hi > 0.0f) {
-            const ff u = {Mh[OL_UH][e], Mh[OL_UL][e]};
+            const float4 uq = F.ol_uq[e];
+            const ff u = {uq.x, uq.y};
             const ff a = wff::mul(wff::mul(wff::mul(u, u), u), F.Lf[OL_ALPHA][slot]);
             stm(F, OL_H, e, wff::mul(a, inv_sfw));
             stm(F, OL_STORAGE, e, wff::mul(a, lds(F, FLOW_LENGTH, slot)));
@@ -2241,7 +2139,8 @@ __global__ void __launch_bounds__(256) rv_post_kernel(WfDevFields F, WfDevGraph 
         if (F.river_node_of_slot[slot] < 0) continue;
         const int m = (int)(e - slot * M);
         float* const* RMh = F.RMh;
-        const ff u = {RMh[RV_UH][e], RMh[RV_UL][e]};
+        const float4 uq = F.rv_uq[e];
+        const ff u = {uq.x, uq.y};
         const ff a = wff::mul(wff::mul(wff::mul(u, u), u), F.Rf[R_ALPHA][slot]);
         str(F, RV_H, e, wff::mul(a, ldrs(F, R_INV_WIDTH, slot)));
         str(F, RV_STORAGE, e, wff::mul(a, ldrs(F, R_LENGTH, slot)));
@@ -2344,14 +2243,12 @@ __global__ void __launch_bounds__(256) sync_u_kernel(WfDevFields F) {
     const int64_t EL = F.land_slots * M, ER = F.river_slots * M;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < EL + ER; i += (int64_t)gridDim.x * blockDim.x) {
         if (i < EL) {
-            const wff::ff uf = wff::from_d(u_of_q(wff::to_d(ldm(F, OL_Q, i))));
-            F.Mh[OL_UH][i] = uf.hi;
-            F.Mh[OL_UL][i] = uf.lo;
+            const wff::ff q = ldm(F, OL_Q, i), uf = wff::from_d(u_of_q(wff::to_d(q)));
+            F.ol_uq[i] = make_float4(uf.hi, uf.lo, q.hi, q.lo);
         } else {
             const int64_t e = i - EL;
-            const wff::ff uf = wff::from_d(u_of_q(wff::to_d(ldr(F, RV_Q, e))));
-            F.RMh[RV_UH][e] = uf.hi;
-            F.RMh[RV_UL][e] = uf.lo;
+            const wff::ff q = ldr(F, RV_Q, e), uf = wff::from_d(u_of_q(wff::to_d(q)));
+            F.rv_uq[e] = make_float4(uf.hi, uf.lo, q.hi, q.lo);
         }
     }
 }
@@ -2458,93 +2355,23 @@ cudaError_t wf_split_balance(const WfDevFields& F, const WfLaunchCfg& c) {
 }
 
 cudaError_t wf_split_ssf_wave(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c) {
-    if (F.N <= 4) return launch_wave(SsfWave<4>{F, g, sw}, c);
-    return launch_wave(SsfWave<WF_MAX_LAYERS>{F, g, sw}, c);
+    if (F.N <= 4) return launch_wave_as<SsfWave<4>, false>(SsfWave<4>{F, g, sw}, c);
+    return launch_wave_as<SsfWave<WF_MAX_LAYERS>, false>(SsfWave<WF_MAX_LAYERS>{F, g, sw}, c);
 }
 
 cudaError_t wf_split_overland_wave(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw,
                                    const WfLaunchCfg& c) {
-    if (sw.aflag) return launch_wave(OlWave<true>{F, g, sw}, c);
-    return launch_wave_sub(OlWave<false>{F, g, sw}, c);
+    if (sw.aflag) return launch_wave_as<OlWave<true>, false>(OlWave<true>{F, g, sw}, c);
+    return launch_wave(OlWave<false>{F, g, sw}, c);
 }
 
 cudaError_t wf_split_river_wave(const WfDevFields& F, const WfDevGraph& g, const WfSweep& sw, const WfLaunchCfg& c) {
     if (F.n_res > 0) {
-        if (sw.aflag) return launch_wave(RvWave<true, true>{F, g, sw}, c);
-        return launch_wave_sub(RvWave<false, true>{F, g, sw}, c);
+        if (sw.aflag) return launch_wave_as<RvWave<true, true>, false>(RvWave<true, true>{F, g, sw}, c);
+        return launch_wave(RvWave<false, true>{F, g, sw}, c);
     }
-    if (sw.aflag) return launch_wave(RvWave<true, false>{F, g, sw}, c);
-    return launch_wave_sub(RvWave<false, false>{F, g, sw}, c);
-}
-
-namespace {
-template <class PA, class PB>
-__global__ void __launch_bounds__(128) wave_pair_kernel(PA pa, PB pb, int S_alloc) {
-    wfv::walk_pair(pa, pb, S_alloc, pa.F.status);
-}
-template <class PA, class PB>
-__global__ void __launch_bounds__(128) wave_pair_diag_kernel(PA pa, PB pb, int S_alloc, int64_t p_chunks, int SL) {
-    wfv::walk_pair_diag(pa, pb, S_alloc, p_chunks, SL, pa.F.status);
-}
-}  // namespace
-
-// The river's first-dispatched chunks run on the diagonal schedule when the river launch has
-// several sub-steps and the tuning's sub-step lanes (wave_sub_lanes) give more than one lane per
-// chain-member pair; the rest of both sweeps node-major.
-cudaError_t wf_split_overland_river_wave(const WfDevFields& F, const WfDevGraph& gl, const WfSweep& swl,
-                                         const WfDevGraph& gr, const WfSweep& swr, const WfLaunchCfg& c) {
-    using PA = OlWave<false, true>;
-    using PB = RvWave<false, false, true>;
-    PA pa{F, gl, swl};
-    PB pb{F, gr, swr};
-    pa.sw.SL = 1;
-    pb.sw.SL = 1;
-    const int threads = 32 * (c.walk_warps > 0 ? c.walk_warps : 4);
-    const int S_alloc = swl.S > swr.S ? swl.S : swr.S;
-    const int SL = wave_sub_lanes(swr.S, c);
-    int blocks_l, blocks_r;
-    // a persistent launch gains nothing from blocks beyond those resident at once (the shared
-    // launch holds more registers per thread than the separate sweeps the tuning was made for)
-    WfLaunchCfg cp = c;
-    cp.walk_blocks = 0;
-    if (SL <= 1) {
-        const size_t smem = wfv::walk_smem(threads, S_alloc);
-        auto kernel = wave_pair_kernel<PA, PB>;
-        int per_sm = 0;
-        cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-        if (err != cudaSuccess) return err;
-        if (c.walk_blocks > 0) cp.walk_blocks = std::min(c.walk_blocks, c.num_sms * std::max(per_sm, 1));
-        err = wave_grid(kernel, threads, smem, cp, gl, blocks_l, pa.sw.prio_items);
-        if (err != cudaSuccess) return err;
-        err = wave_grid(kernel, threads, smem, cp, gr, blocks_r, pb.sw.prio_items);
-        if (err != cudaSuccess) return err;
-        kernel<<<blocks_l > blocks_r ? blocks_l : blocks_r, threads, smem, c.stream>>>(pa, pb, S_alloc);
-        return cudaGetLastError();
-    }
-    const size_t smem = wfv::pair_diag_smem(threads, S_alloc);
-    auto kernel = wave_pair_diag_kernel<PA, PB>;
-    int64_t prio_r;
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
-    int per_sm = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-    if (err != cudaSuccess) return err;
-    if (c.walk_blocks > 0) cp.walk_blocks = std::min(c.walk_blocks, c.num_sms * std::max(per_sm, 1));
-    err = wave_grid(kernel, threads, smem, cp, gl, blocks_l, pa.sw.prio_items);
-    if (err != cudaSuccess) return err;
-    err = wave_grid(kernel, threads, smem, cp, gr, blocks_r, prio_r);
-    if (err != cudaSuccess) return err;
-    const int blocks = blocks_l > blocks_r ? blocks_l : blocks_r;
-    // at most half of the resident warps hold first-dispatched river tickets (diagonal items and
-    // node-major long chunks together), as in wave_grid
-    const int64_t resident = (int64_t)std::min(blocks, c.num_sms * std::max(per_sm, 1)) * (threads / 32);
-    const int64_t ipc_d = wf_items_per_chunk(gr.G, gr.M, SL);
-    const int64_t gpc = gr.M > 32 ? gr.M / 32 : 1;
-    const int64_t p_chunks = std::min<int64_t>(gr.n_long_chunks, (resident / 2) / ipc_d);
-    pb.sw.prio_items = std::max<int64_t>(0, std::min<int64_t>((gr.n_long_chunks - p_chunks) * gpc,
-                                                              resident / 2 - p_chunks * ipc_d));
-    kernel<<<blocks, threads, smem, c.stream>>>(pa, pb, S_alloc, p_chunks, SL);
-    return cudaGetLastError();
+    if (sw.aflag) return launch_wave_as<RvWave<true, false>, false>(RvWave<true, false>{F, g, sw}, c);
+    return launch_wave(RvWave<false, false>{F, g, sw}, c);
 }
 
 cudaError_t wf_split_ssf_post(const WfDevFields& F, const WfDevGraph& g, const WfLaunchCfg& c) {

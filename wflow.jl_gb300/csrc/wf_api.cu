@@ -40,12 +40,9 @@ struct DevGraphAlloc {
     double *up_w = nullptr, *up_fr = nullptr;
     float *up_wf = nullptr, *up_frf = nullptr;
     int4* up_rec = nullptr;
-    float* up_whv = nullptr;
-    uint8_t* up_nlt = nullptr;
-    float4* up_frec = nullptr;
     int4* up_rec64 = nullptr;
     double* up_w64 = nullptr;
-    int32_t lanes64 = 1, lanes64_multi = 1;
+    int32_t lanes = 1, lanes_multi = 1;
     uint32_t* flags = nullptr;
     double* end_q = nullptr;
     unsigned long long* ticket = nullptr;
@@ -202,6 +199,28 @@ int upload_slots_ff(WfHandle* h, float** hi, float** lo, const std::vector<doubl
     return rc ? rc : upload(h, lo, vl);
 }
 
+// Leading chunks of at most SHORT_LEN positions
+int64_t short_chunks(const WfRoutingPlan& P) {
+    int64_t ns = 0;
+    while (ns < P.n_chunks && P.chunk_len[ns] <= wfv::SHORT_LEN) ++ns;
+    return ns;
+}
+
+// Packing lanes per chain-member pair of the slim wavefronts, for launches of S sub-steps: the most
+// (fewest pairs per warp) for which the chunks from `from` up to the first-dispatched group take at most
+// a quarter of the longest chain's time steps on the device's schedulers. Measured on one 160 x 160 daily
+// FP64 domain (overland): 6.1 ms by this rule, 6.9 at a sixteenth, 17 at a 64th.
+int wave_lanes(const WfRoutingPlan& P, int M, int S, int num_sms, int64_t from) {
+    for (int SL = 32; SL > 1; SL >>= 1) {
+        const int SU = std::min(SL, S);
+        const int64_t rounds = (S + SU - 1) / SU, ipc = wf_items_per_chunk(P.G, M, SL);
+        int64_t steps = 0;
+        for (int64_t k = from; k < P.n_chunks - P.n_long_chunks; ++k) steps += rounds * (P.chunk_len[k] + SU) * ipc;
+        if (steps / (num_sms * 4) <= rounds * (P.max_len + SU) / 4) return SL;
+    }
+    return 1;
+}
+
 int plan_graph(WfHandle* h, DevGraphAlloc& G, int64_t n, const int32_t* ds, int M, int32_t s_cap,
                const int64_t* heavy_hint = nullptr) {
     std::string err;
@@ -219,6 +238,10 @@ int plan_graph(WfHandle* h, DevGraphAlloc& G, int64_t n, const int32_t* ds, int 
     if ((rc = upload(h, &G.is_chain_end, P.is_chain_end))) return rc;
     if ((rc = upload(h, &G.node_of_slot, P.node_of_slot))) return rc;
     G.s_cap = s_cap;
+    const int s_most = h->cfg.form == WF_FORM_SPLIT ? std::min<int>(s_cap, wfv::MAX_GROUP) : s_cap;
+    const int64_t from = h->cfg.form == WF_FORM_SPLIT ? short_chunks(P) : 0;
+    G.lanes = wave_lanes(P, M, 1, h->num_sms, from);
+    G.lanes_multi = wave_lanes(P, M, s_most, h->num_sms, from);
     if ((rc = dalloc(h, &G.flags, (size_t)P.n_chains * M))) return rc;
     if ((rc = dalloc(h, &G.end_q, (size_t)P.n_chains * M * s_cap))) return rc;
     if ((rc = dalloc(h, &G.ticket, 1))) return rc;
@@ -231,11 +254,7 @@ WfDevGraph dev_graph(const DevGraphAlloc& G, int M) {
     g.n_chunks = G.plan.n_chunks;
     g.n_chains = G.plan.n_chains;
     g.n_long_chunks = G.plan.n_long_chunks;
-    {
-        int64_t ns = 0;
-        while (ns < G.plan.n_chunks && G.plan.chunk_len[ns] <= wfv::SHORT_LEN) ++ns;
-        g.n_short_chunks = ns;
-    }
+    g.n_short_chunks = short_chunks(G.plan);
     g.G = G.plan.G;
     g.M = M;
     g.chunk_base = G.chunk_base;
@@ -252,33 +271,16 @@ WfDevGraph dev_graph(const DevGraphAlloc& G, int M) {
     g.up_wf = G.up_wf;
     g.up_frf = G.up_frf;
     g.up_rec = G.up_rec;
-    g.up_whv = G.up_whv;
-    g.up_nlt = G.up_nlt;
-    g.up_frec = G.up_frec;
     g.up_rec64 = G.up_rec64;
     g.up_w64 = G.up_w64;
-    g.lanes64 = G.lanes64;
-    g.lanes64_multi = G.lanes64_multi;
+    g.lanes = G.lanes;
+    g.lanes_multi = G.lanes_multi;
     g.flags = G.flags;
     g.end_q = G.end_q;
     g.ticket = G.ticket;
     g.s_cap = G.s_cap;
     g.snow_up = G.snow_up;
     return g;
-}
-
-// Packing lanes per chain-member pair of the FP64 form's slim wavefronts, for launches of S sub-steps: the
-// most (fewest pairs per warp) for which the chains outside the first-dispatched group take at most
-// a quarter of the longest chain's time steps on the schedulers of the device.
-int wave64_lanes(const WfRoutingPlan& P, int M, int S, int num_sms) {
-    for (int SL = 32; SL > 1; SL >>= 1) {
-        const int SU = std::min(SL, S);
-        const int64_t rounds = (S + SU - 1) / SU, ipc = wf_items_per_chunk(P.G, M, SL);
-        int64_t steps = 0;
-        for (int64_t k = 0; k < P.n_chunks - P.n_long_chunks; ++k) steps += rounds * (P.chunk_len[k] + SU) * ipc;
-        if (steps / (num_sms * 4) <= rounds * (P.max_len + SU) / 4) return SL;
-    }
-    return 1;
 }
 
 // Graphs.jl v1.14 topological_sort_by_dfs (Wflow's network.order, network.jl:99) of a graph of
@@ -1149,28 +1151,24 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         // per-cell constants of the slim wavefronts (split form): 1/dx and the subsurface terms
         // of a single sub-step dt_s
         const double dts = h->h_dts_ssf[0];
-        std::vector<double> inv_dx(n), dtdx(n), idwdx(n), dtsy(n), k2(n), inv_te(n), inv_area(n), inv_sfw(n), inv_dx_lo(n);
+        std::vector<double> inv_dx(n), dtdx(n), idwdx(n), dtsy(n), inv_te(n), inv_area(n), inv_sfw(n);
         for (int64_t i = 0; i < n; ++i) {
             const double dx = d->flow_length[i], dw = d->flow_width[i];
             inv_area[i] = 1.0 / d->area[i];
             inv_sfw[i] = d->surface_flow_width[i] > 0.0 ? 1.0 / d->surface_flow_width[i] : 0.0;
             inv_te[i] = 1.0 / (p->theta_s[i] - p->theta_r[i]);
             inv_dx[i] = 1.0 / dx;
-            inv_dx_lo[i] = inv_dx[i] - (double)(float)inv_dx[i];
             dtdx[i] = dts / dx;
             idwdx[i] = 1.0 / (dw * dx);
             dtsy[i] = dts / sy[i];
-            k2[i] = (dw * dx) * sy[i] / dts;
         }
         ls.push_back({INV_FLOW_LENGTH, inv_dx});
         ls.push_back({SSF_DTDX, dtdx});
         ls.push_back({SSF_IDWDX, idwdx});
         ls.push_back({SSF_DTSY, dtsy});
-        ls.push_back({SSF_K2, k2});
         ls.push_back({INV_TE, inv_te});
         ls.push_back({INV_AREA, inv_area});
         ls.push_back({INV_SFW, inv_sfw});
-        ls.push_back({INV_DX_LO, inv_dx_lo});
     }
     for (auto& x : ls) CKR(upload_slots(h, &F.L[x.idx], x.v, PL, M, n, false));
     for (int k = 0; k < N; ++k) {
@@ -1269,13 +1267,12 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         CKR(upload(h, &h->land.snow_up, su));
     }
     // ---- river fields
-    std::vector<double> r_width(nr), r_length(nr), r_alpha(nr), r_ext(nr), r_area(nr), r_inv_len(nr), r_inv_w(nr), r_inv_len_lo(nr);
+    std::vector<double> r_width(nr), r_length(nr), r_alpha(nr), r_ext(nr), r_area(nr), r_inv_len(nr), r_inv_w(nr);
     for (int64_t r = 0; r < nr; ++r) {
         r_width[r] = d->river_width[r];
         r_length[r] = d->river_length[r];
         r_inv_len[r] = 1.0 / d->river_length[r];
         r_inv_w[r] = 1.0 / d->river_width[r];
-        r_inv_len_lo[r] = r_inv_len[r] - (double)(float)r_inv_len[r];
         r_ext[r] = d->river_external_inflow ? d->river_external_inflow[r] : 0.0;
         r_area[r] = d->area[d->river_land_index[r]];
         h->river_land.push_back(d->river_land_index[r]);
@@ -1290,7 +1287,6 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
     CKR(upload_slots(h, &F.R[R_AREA], r_area, PR, M, nr, false));
     CKR(upload_slots(h, &F.R[R_INV_LENGTH], r_inv_len, PR, M, nr, false));
     CKR(upload_slots(h, &F.R[R_INV_WIDTH], r_inv_w, PR, M, nr, false));
-    CKR(upload_slots(h, &F.R[R_INV_LEN_LO], r_inv_len_lo, PR, M, nr, false));
     std::vector<double> zeros_r((size_t)std::max<int64_t>(nr, 1) * M, 0.0);
     for (int f = 0; f < RM_COUNT; ++f) {
         if (wf_split_only_river_member(f)) {
@@ -1300,6 +1296,18 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         if (F.split) CKR(upload_slots_ff(h, &F.RMh[f], &F.RMl[f], zeros_r, PR, M, nr, true));
         else CKR(upload_slots(h, &F.RM[f], zeros_r, PR, M, nr, true));
     }
+    std::vector<int32_t> river_of_land(n, -1);
+    for (int64_t r = 0; r < nr; ++r) river_of_land[d->river_land_index[r]] = (int32_t)PR.slot_of_node[r];
+    auto int_of = [](float v) {
+        int32_t i;
+        std::memcpy(&i, &v, sizeof(i));
+        return i;
+    };
+    auto float_of = [](int32_t v) {
+        float f;
+        std::memcpy(&f, &v, sizeof(f));
+        return f;
+    };
     // ---- upstream weights of the wavefront gathers: land discharge splits into the part that
     // goes to the river (flow_fraction_to_river) and the rest that flows downstream
     for (int g = 0; g < 2; ++g) {
@@ -1319,42 +1327,63 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         std::vector<float> wf(w.begin(), w.end()), frf(fr.begin(), fr.end());
         CKR(upload(h, &G.up_wf, wf));
         CKR(upload(h, &G.up_frf, frf));
-        // per-slot records of the slim wavefronts: the first two light children and the weights
-        std::vector<int4> rec(std::max<int64_t>(P.n_slots, 1), int4{-1, -1, 0, 0});
-        std::vector<float> whv(rec.size(), 0.0f);
-        std::vector<uint8_t> nlt(rec.size(), 0);
-        std::vector<float4> frec(rec.size(), float4{0.0f, 0.0f, 0.0f, 0.0f});
-        for (int64_t sl = 0; sl < P.n_slots; ++sl) {
-            int lights = 0;
-            for (int32_t o = P.up_ptr[sl]; o < P.up_ptr[sl + 1]; ++o) {
-                if (P.up_chain[o] < 0) {
-                    whv[sl] = wf[o];
-                    frec[sl].x = frf[o];
-                    continue;
+        if (F.split) {  // per-slot records and constants of the slim wavefronts
+            std::vector<int4> rec(std::max<int64_t>(P.n_slots, 1), int4{-1, -1, 0, 0});
+            std::vector<float4> st(2 * rec.size(), float4{0.0f, 0.0f, 0.0f, 0.0f}), ssf(st);
+            for (int64_t sl = 0; sl < P.n_slots; ++sl) {
+                const int64_t i = P.node_of_slot[sl];
+                if (i < 0) continue;
+                int lights = 0;
+                float whv = 0.0f, fhv = 0.0f, fl[2] = {0.0f, 0.0f};
+                for (int32_t o = P.up_ptr[sl]; o < P.up_ptr[sl + 1]; ++o) {
+                    if (P.up_chain[o] < 0) {
+                        whv = wf[o];
+                        fhv = frf[o];
+                        continue;
+                    }
+                    if (lights < 2) {
+                        (lights == 0 ? rec[sl].x : rec[sl].y) = P.up_chain[o];
+                        (lights == 0 ? rec[sl].z : rec[sl].w) = int_of(wf[o]);
+                        fl[lights] = frf[o];
+                    }
+                    ++lights;
                 }
-                float wo = wf[o];
-                int32_t bits;
-                std::memcpy(&bits, &wo, sizeof(bits));
-                if (lights == 0) {
-                    rec[sl].x = P.up_chain[o];
-                    rec[sl].z = bits;
-                    frec[sl].y = frf[o];
-                } else if (lights == 1) {
-                    rec[sl].y = P.up_chain[o];
-                    rec[sl].w = bits;
-                    frec[sl].z = frf[o];
+                const double dx = g == 0 ? d->flow_length[i] : d->river_length[i], inv = 1.0 / dx;
+                const float inv_hi = (float)inv, inv_lo = (float)(inv - (double)inv_hi);
+                const size_t lo = sl, hi = P.n_slots + sl;  // the two planes
+                if (g == 0) {
+                    const int32_t rs1 = river_of_land[i] + 1;
+                    const float a = (float)ol_alpha[i];
+                    st[lo] = {inv_hi, inv_lo, (float)d->surface_flow_width[i] > 0.0f ? a : -a,
+                              float_of(lights > 2 ? rs1 | INT32_MIN : rs1)};
+                    st[hi] = {whv, fhv, fl[0], fl[1]};
+                    const double dts = h->h_dts_ssf[0], dw = d->flow_width[i];
+                    ssf[lo] = {(float)p->soil_thickness[i], (float)(dts / dx), (float)(1.0 / (dw * dx)),
+                               (float)(dts / sy[i])};
+                    ssf[hi] = {(float)((dw * dx) * sy[i] / dts), whv, (float)dw, float_of(lights)};
+                } else {
+                    st[lo] = {inv_hi, inv_lo, (float)r_alpha[i], (float)dx};
+                    st[hi] = {(float)r_ext[i], float_of(nres > 0 ? res_of_river[i] : -1), 0.0f, float_of(lights)};
                 }
-                ++lights;
             }
-            nlt[sl] = (uint8_t)std::min(lights, 255);
+            CKR(upload(h, &G.up_rec, rec));
+            CKR(upload(h, g == 0 ? &F.ol_st : &F.rv_st, st));
+            if (g == 0) CKR(upload(h, &F.ssf_st, ssf));
+            const size_t E = rec.size() * M;
+            auto zeroed = [&](auto** dst, size_t count) -> int {
+                int rc = dalloc(h, dst, count);
+                if (rc) return rc;
+                CK(cudaMemset(*dst, 0, count * sizeof(**dst)));
+                return WF_OK;
+            };
+            CKR(zeroed(g == 0 ? &F.ol_uq : &F.rv_uq, E));
+            CKR(zeroed(g == 0 ? &F.ol_lat : &F.rv_lat, E));
+            if (g == 0) CKR(zeroed(&F.ssf_out, E));
+            if (g == 0) CKR(zeroed(&F.ssf_dyn, 2 * E));
         }
-        CKR(upload(h, &G.up_rec, rec));
-        CKR(upload(h, &G.up_whv, whv));
-        CKR(upload(h, &G.up_nlt, nlt));
-        CKR(upload(h, &G.up_frec, frec));
         if (!F.split) {  // records of the FP64 form's slim wavefronts
-            std::vector<int4> r64(rec.size(), int4{-1, -1, 0, 0});
-            std::vector<double> w64(g == 0 ? rec.size() * 6 : 1, 0.0);
+            std::vector<int4> r64(std::max<int64_t>(P.n_slots, 1), int4{-1, -1, 0, 0});
+            std::vector<double> w64(g == 0 ? r64.size() * 6 : 1, 0.0);
             for (int64_t sl = 0; sl < P.n_slots; ++sl) {
                 const int64_t node = P.node_of_slot[sl];
                 if (node < 0) continue;
@@ -1379,8 +1408,6 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
                 if (g == 0 && !(d->surface_flow_width[node] > 0.0)) q.z |= wfz::REC_NO_INFLOW;
                 if (g == 1 && r_ext[node] < 0.0) q.z |= wfz::REC_ABSTRACTION;
             }
-            G.lanes64 = wave64_lanes(P, M, 1, h->num_sms);
-            G.lanes64_multi = wave64_lanes(P, M, G.s_cap, h->num_sms);
             CKR(upload(h, &G.up_rec64, r64));
             CKR(upload(h, &G.up_w64, w64));
         }
@@ -1427,7 +1454,6 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         CKR(upload_slots_ff(h, &F.Rf[R_EXT_INFLOW], &F.Rl[R_EXT_INFLOW], r_ext, PR, M, nr, false));
         CKR(upload_slots_ff(h, &F.Rf[R_AREA], &F.Rl[R_AREA], r_area, PR, M, nr, false));
         CKR(upload_slots_ff(h, &F.Rf[R_INV_LENGTH], &F.Rl[R_INV_LENGTH], r_inv_len, PR, M, nr, false));
-        CKR(upload_slots_ff(h, &F.Rf[R_INV_LEN_LO], &F.Rl[R_INV_LEN_LO], r_inv_len_lo, PR, M, nr, false));
         CKR(upload_slots_ff(h, &F.Rf[R_INV_WIDTH], &F.Rl[R_INV_WIDTH], r_inv_w, PR, M, nr, false));
     }
     // ---- maps
@@ -1527,7 +1553,6 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
     F.ssf_single = h->h_dts_ssf.size() == 1 && (F.split || !h->adaptive);
     if (!F.split)
         for (int k = 0; k < 10; ++k) CKR(dalloc(h, &F.W[k], (size_t)std::max(PL.n_slots, PR.n_slots) * M));
-    if (F.split && PR.n_slots > 0) CKR(dalloc(h, &F.rv_lat_pub, (size_t)PR.n_slots * M));
     F.dt_ssf = h->h_dts_ssf[0];
     F.inv_dt_ssf = 1.0 / h->h_dts_ssf[0];
     F.inv_dt_hi = (float)F.inv_dt;
@@ -2174,11 +2199,10 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
         sw.wait_offset = h->wait_offset;
         return sw;
     };
-    auto wave = [&](DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts, double* d_dts, int which,
-                    int first0 = 0) -> int {
+    auto wave = [&](DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts, double* d_dts, int which) -> int {
         const int total = (int)dts.size();
         const int group = std::min<int>(G.s_cap, wfv::MAX_GROUP);
-        for (int first = first0; first < total; first += group) {
+        for (int first = 0; first < total; first += group) {
             const WfSweep sw = wave_sw(G, dts, d_dts, first);
             CK(cudaMemsetAsync(G.end_q, 0xFF, (size_t)G.plan.n_chains * h->M * G.s_cap * sizeof(double), h->stream));
             CK(cudaMemsetAsync(G.ticket, 0, sizeof(unsigned long long), h->stream));
@@ -2288,37 +2312,12 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
         else rc = sweep(h->land, gl, h->h_dts_ssf, h->dts_ssf);
         if (rc) return rc;
         mark(2);
-        // the overland sweep and the river's first sub-step group in one launch (the river cells
-        // take their lateral inflow from the overland walker as it passes them), unless the
-        // tuning asks for separate launches; models with reservoirs (whose inflow is the
-        // overland step average) and steps of more overland sub-steps than one launch holds
-        // keep them apart
-        const bool fuse = h->tuning.reserved[6] == 0 && h->nres == 0 && h->nr > 0 &&
-                          (int)h->h_dts_land.size() <= std::min<int>(h->land.s_cap, wfv::MAX_GROUP);
-        if (fuse) {
-            const WfSweep swl = wave_sw(h->land, h->h_dts_land, h->dts_land, 0);
-            const WfSweep swr = wave_sw(h->river, h->h_dts_river, h->dts_river, 0);
-            CK(cudaMemsetAsync(h->land.end_q, 0xFF,
-                               (size_t)h->land.plan.n_chains * h->M * h->land.s_cap * sizeof(double), h->stream));
-            CK(cudaMemsetAsync(h->river.end_q, 0xFF,
-                               (size_t)h->river.plan.n_chains * h->M * h->river.s_cap * sizeof(double), h->stream));
-            CK(cudaMemsetAsync(h->F.rv_lat_pub, 0xFF, (size_t)h->river.plan.n_slots * h->M * sizeof(double),
-                               h->stream));
-            CK(cudaMemsetAsync(h->land.ticket, 0, sizeof(unsigned long long), h->stream));
-            CK(wf_split_overland_river_wave(h->F, gl, swl, gr, swr, lc));
-            CK(wf_split_overland_post(h->F, gl, lc));
-            nl += 2;
-            mark(3);
-            if ((rc = wave(h->river, gr, h->h_dts_river, h->dts_river, 2, swr.S))) return rc;
-            mark(4);
-        } else {
-            if ((rc = wave(h->land, gl, h->h_dts_land, h->dts_land, 1))) return rc;
-            mark(3);
-            if ((rc = res_prep())) return rc;
-            if (h->nr > 0 && (rc = wave(h->river, gr, h->h_dts_river, h->dts_river, 2))) return rc;
-            if ((rc = res_post())) return rc;
-            mark(4);
-        }
+        if ((rc = wave(h->land, gl, h->h_dts_land, h->dts_land, 1))) return rc;
+        mark(3);
+        if ((rc = res_prep())) return rc;
+        if (h->nr > 0 && (rc = wave(h->river, gr, h->h_dts_river, h->dts_river, 2))) return rc;
+        if ((rc = res_post())) return rc;
+        mark(4);
     } else if (h->li) {
         // local-inertial land and river routing (surface_routing.jl:62-89) after the subsurface
         rc = h->F.ssf_single ? wave64(h->land, gl, h->h_dts_ssf, h->dts_ssf, 0)

@@ -19,7 +19,7 @@
     X(WHC) X(THETA_S) X(THETA_R) X(THETA_FC) X(SWC) X(SOIL_THICKNESS) X(PSI_B) X(H1) X(H2) X(H3_HIGH) \
     X(H3_LOW) X(H4) X(ALPHA_H1) X(CAP_COMP) X(COMPACT_FRAC) X(ROOTDISTPAR) X(CAP_HMAX) X(CAP_N)       \
     X(MAX_LEAKAGE) X(W_SOIL) X(CF_SOIL) X(ROOTING_DEPTH) X(Z_EXP) X(KH_RATIO) X(INV_FLOW_LENGTH)  \
-    X(SSF_DTDX) X(SSF_IDWDX) X(SSF_DTSY) X(SSF_K2) X(INV_TE) X(INV_AREA) X(INV_SFW) X(INV_DX_LO)
+    X(SSF_DTDX) X(SSF_IDWDX) X(SSF_DTSY) X(INV_TE) X(INV_AREA) X(INV_SFW)
 
 #define WF_M_FIELDS(X)                                                                             \
     X(KV0) X(FSCALE) X(Q_MAX) X(PRECIP) X(POTEVAP) X(TEMP) X(CANOPY) X(SNOW) X(SNOW_WATER) X(TSOIL) X(SAT) X(TSWS)    \
@@ -32,16 +32,14 @@
     X(EXFILT) X(BL_PREV) X(BO_PREV) X(TOTAL_STORAGE) X(BL_ERR) X(BL_REL) X(BO_ERR) X(BO_REL)          \
     X(BS_ERR) X(BS_REL)                                                                            \
     X(SSF_QNET) X(SSF_TQIN) X(SSF_TEXF) X(SSF_TNF)                                                 \
-    X(SSF_T2) X(SSF_RDF) X(SSF_RTH) X(SSF_RCAP) X(SSF_RRHO) X(SSF_FLAG) X(SSF_QNETF) X(SSF_ZIF)      \
-    X(SSF_QF) X(SSF_QUF) X(SSF_QINF) X(OL_UH) X(OL_UL) X(OL_QSUMH) X(OL_QSUML)
+    X(OL_QSUMH) X(OL_QSUML)
 
-#define WF_R_FIELDS(X) X(R_WIDTH) X(R_LENGTH) X(R_ALPHA) X(R_EXT_INFLOW) X(R_AREA) X(R_INV_LENGTH) X(R_INV_WIDTH) X(R_INV_LEN_LO)
+#define WF_R_FIELDS(X) X(R_WIDTH) X(R_LENGTH) X(R_ALPHA) X(R_EXT_INFLOW) X(R_AREA) X(R_INV_LENGTH) X(R_INV_WIDTH)
 
 #define WF_RM_FIELDS(X)                                                                            \
     X(RV_Q) X(RV_H) X(RV_STORAGE) X(RV_Q_AVG) X(RV_QIN_AVG) X(RV_INWATER) X(RV_QLAT) X(RV_ABS_AVG)    \
     X(RV_Q_CUM) X(RV_QIN_CUM) X(RV_ABS_CUM) X(BR_PREV) X(BR_ERR) X(BR_REL)                         \
-    X(RV_UH) X(RV_UL) X(RV_QSUMH) X(RV_QSUML) X(RV_ABSH) X(RV_ABSL) X(RV_QLATTH) X(RV_QLATTL)      \
-    X(RV_TRSUMH) X(RV_TRSUML)
+    X(RV_QSUMH) X(RV_QSUML) X(RV_ABSH) X(RV_ABSL) X(RV_TRSUMH) X(RV_TRSUML)
 
 // Reservoirs, per reservoir and member (element r * M + m), FP64 in both forms. The first
 // fifteen follow the order of the WF_F_RESERVOIR_* field ids (WF_F_RESERVOIR_STORAGE + i).
@@ -87,11 +85,11 @@ __host__ __device__ inline bool wf_split_f32_member(int f) {
 
 // Member fields only the split form's slim wavefronts use (not allocated by the FP64 form).
 __host__ __device__ inline bool wf_split_only_member(int f) { return f >= SSF_QNET; }
-__host__ __device__ inline bool wf_split_only_river_member(int f) { return f >= RV_UH; }
-// Of those, the ones held only in FP32 (Mh / RMh): walker inputs and the double-FP32 routing
-// state (pairs *H + *L).
-__host__ __device__ inline bool wf_split_f32_only(int f) { return f >= SSF_T2; }
-__host__ __device__ inline bool wf_split_f32_only_river(int f) { return f >= RV_UH; }
+__host__ __device__ inline bool wf_split_only_river_member(int f) { return f >= RV_QSUMH; }
+// Of those, the ones held only in FP32 (Mh / RMh): sums of the double-FP32 routing (pairs
+// *H + *L).
+__host__ __device__ inline bool wf_split_f32_only(int f) { return f >= OL_QSUMH; }
+__host__ __device__ inline bool wf_split_f32_only_river(int f) { return f >= RV_QSUMH; }
 // Split form: the large stores stay FP64 (saturated depth, water-table depths, total soil
 // water and the land balance's previous storage): a step changes them by as little as
 // 1e-15 of their size in dry cells, below the double-FP32 resolution.
@@ -134,6 +132,22 @@ struct WfDevFields {
     const int64_t* land_river_slot;       // [land slots], river slot or -1
     const int64_t* river_node_of_slot;    // [river slots], -1 padding
     const int64_t* river_land_slot;       // [river slots], land slot of the river cell
+    // Split form: what the slim wavefronts read and write, in vectors, so that a position takes a few wide
+    // copies. Per element, by the step's kernels; per slot (*_st, two planes of a vector a slot), at creation.
+    //   ssf_dyn  {net inflow, q_prev / celerity, 1 / (dt/dx + 1/celerity), negative where q_prev is 0,
+    //            water table}; then a plane {deepest unsaturated layer: thickness, capacity as a flux,
+    //            rise per flux; largest discharge per width}
+    //   ssf_st   {soil thickness, dt/dx, 1/(dw dx), dt/sy}, {dw dx sy/dt, heavy child's weight, flow
+    //            width, light children}
+    //   ssf_out  {q, q before the cut at the soil's bottom, inflow, case (SSF_EARLY..)}
+    //   *_uq     {u = Q^0.2, Q}, *_lat the lateral inflow (double-FP32 pairs)
+    //   ol_st    {1/dx, alpha, negative without surface flow width, river slot + 1, negative with more
+    //            than two light children}, {heavy child's weight; fractions to the river of the heavy
+    //            child and of light children 0 and 1}
+    //   rv_st    {1/dx, alpha, length}, {external inflow, reservoir, -, light children}
+    float4 *ssf_dyn, *ssf_out, *ol_uq, *rv_uq;
+    float2 *ol_lat, *rv_lat;
+    float4 *ssf_st, *ol_st, *rv_st;
     int64_t land_slots;
     int64_t river_slots;
     int32_t N;      // maximum_number_of_layers
@@ -173,10 +187,6 @@ struct WfDevFields {
     // local-inertial land and river routing in place of the kinematic waves (wf_li_couple.cuh):
     // the overland and river balances are the scheme's
     int32_t li_coupled;
-    // split form: the lateral inflow of each river cell and member as a packed double-FP32
-    // word, published by the overland wavefront for a river wavefront sharing its launch
-    // (filled with the sentinel pattern before such a launch)
-    unsigned long long* rv_lat_pub;  // [river slots * M]
     // FP64 form: terms of the sweep in hand, per element of its graph, written by the per-cell kernel
     // before the slim wavefront and read by it (WfW64Kw, WfW64Ssf); [max(land, river slots) * M] each
     double* W[10];
@@ -213,20 +223,14 @@ struct WfDevGraph {
     const float* up_wf;   // FP32 copies of up_w / up_fr (split form)
     const float* up_frf;
     // per-slot upstream records of the split form's slim wavefronts (wf_wave.cuh UpRec):
-    // {chain of light child 0, chain of light child 1, their weights as float bits}, the heavy
-    // child's weight and the number of light children
+    // {chain of light child 0, chain of light child 1, their weights as float bits}
     const int4* up_rec;
-    const float* up_whv;
-    const uint8_t* up_nlt;
-    // land graph: per slot, the fractions to the river of the heavy child and of light children
-    // 0 and 1 (up_frf of those entries; 0 where absent)
-    const float4* up_frec;
     // FP64 form: upstream records of the slim wavefronts (wf_wave64.cuh Rec), and per land slot
     // {1 - fraction to the river, fraction} of the heavy child and of light children 0 and 1
     const int4* up_rec64;
     const double* up_w64;
-    int32_t lanes64;        // FP64 form: packing lanes per chain-member pair of the slim wavefronts,
-    int32_t lanes64_multi;  // and the most of them that a launch of several sub-steps is worth
+    int32_t lanes;        // packing lanes per chain-member pair of the slim wavefronts,
+    int32_t lanes_multi;  // and the most of them that a launch of several sub-steps is worth
     uint32_t* flags;      // [n_chains * M] epoch of the last published sub-step
     double* end_q;        // [n_chains * M * s_cap] q of each chain end per sub-step
     unsigned long long* ticket;  // work counter of the current launch

@@ -35,6 +35,12 @@ cudaError_t wave_grid(Kernel kernel, int threads, size_t smem, const WfLaunchCfg
     return cudaSuccess;
 }
 
+// Chunks of the first-dispatched group that a slim wavefront (wf_wave.cuh) takes first with SL lanes per
+// pair: as many as half of the resident warps hold.
+inline int64_t first_chunks(const WfDevGraph& g, int SL, int64_t resident) {
+    return std::min<int64_t>(g.n_long_chunks, resident / 2 / wf_items_per_chunk(1, g.M, SL));
+}
+
 // Sub-step lanes of a diagonal-schedule launch of S sub-steps: the smallest power of two that
 // covers S, at most the cap (tuning; 8 by default) and at most 32.
 inline int wave_sub_lanes(int S, const WfLaunchCfg& c) {

@@ -9,7 +9,7 @@
 // soil column are finished by another after it. Every operation is the reference's, in its order,
 // wherever it runs, so the results are those of a plain sweep bit for bit.
 //
-// Schedule: the diagonal one of wf_wave.cuh (diag_ticket). SL lanes serve a chain-member pair, lane l
+// Schedule: the diagonal one of wf_wave.cuh. SL lanes serve a chain-member pair, lane l
 // takes sub-step r SL + l of round r and at time t works on position t - l; the node's state goes from
 // lane to lane by warp shuffles, the heavy child's discharge stays in the lane. Launches of one
 // sub-step (SL = 1) skip the hand-over. Chain ends publish their discharge's bits into end_q, filled
@@ -214,86 +214,27 @@ __device__ __forceinline__ double kw_solve(const KwState& k, double cterm, doubl
 //     return; more: the launch holds another sub-step after s. False to abort.
 //   void finish(const St&, e, bool last_round)   stores after the last sub-step of a round
 
-// A lane's chain in each item of the warp's ticket, resolved once per ticket (a position costs a
-// multiply-add then; resolving it from the item each time, with its divisions by the member count,
-// took most of a position's 780 instructions).
-struct Batch {
-    int64_t slot0[wfv::BATCH][32];
-    int32_t chain[wfv::BATCH][32], len[wfv::BATCH][32], m[wfv::BATCH][32];
-    int32_t L[wfv::BATCH], Gc[wfv::BATCH];
-};
+using wfv::Batch;
+using wfv::Cursor;
+using wfv::P_END;
+using wfv::P_HEAVY;
+using wfv::Pos;
 
 __host__ __device__ constexpr size_t walk_smem(int threads) { return (size_t)(threads / 32) * sizeof(Batch); }
-
-// A position of the lane's sequence
-struct Pos {
-    int64_t slot;
-    int32_t m, chain, flags;  // P_VALID: the lane has a node here
-};
-constexpr int32_t P_VALID = 1, P_END = 2, P_HEAVY = 4;
-
-// Walks over the positions (item, k) of a ticket
-struct Cursor {
-    int it, k, L;
-    __device__ __forceinline__ void reset(const Batch* b, int count) {
-        it = k = 0;
-        L = b->L[0];
-    }
-    __device__ __forceinline__ void advance(const Batch* b, int count) {
-        if (++k < L || it >= count) return;
-        k = 0;
-        if (++it < count) L = b->L[it];
-    }
-    __device__ __forceinline__ void resolve(const Batch* b, int count, unsigned lane, Pos& p) const {
-        p.flags = 0;
-        if (it >= count) return;
-        const int len = b->len[it][lane];
-        if (k >= len) return;
-        p.slot = b->slot0[it][lane] + (int64_t)(k * b->Gc[it]);
-        p.m = b->m[it][lane];
-        p.chain = b->chain[it][lane];
-        p.flags = P_VALID | (k == len - 1 ? P_END : 0) | (k > 0 ? P_HEAVY : 0);
-    }
-};
 
 // SL lanes per chain-member pair, of which the first SU = min(SL, S) work (more lanes than sub-steps
 // only keep other chains out of the warp).
 template <class Phys, bool MULTI>
-__device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, Phys& phys, int32_t* status,
-                                       int64_t first, int count, int SL, int64_t ipc, Batch* wb) {
+__device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, Phys& phys, int32_t* status, int count,
+                                       int SL, const wfv::LanePair& lp, int npos, Batch* wb) {
     using In = typename Phys::In;
     using St = typename Phys::St;
     const unsigned lane = threadIdx.x & 31u;
     const int M = g.M;
-    const int J = 32 / SL;
     const int sl = (int)lane & (SL - 1);
-    const int j = (int)lane / SL;
     const int SU = MULTI ? min(SL, sw.S) : 1;
     const int rounds = MULTI ? (sw.S + SU - 1) / SU : 1;
     if (wfv::status_ld(status) & WF_DEV_SPIN_TIMEOUT) return false;
-    int npos = 0, work = 0;
-    for (int it = 0; it < count; ++it) {
-        const int64_t item = first + it, chunk = item / ipc;
-        const int Gc = g.chunk_g[chunk], L = g.chunk_len[chunk];
-        const int p = (int)(item - chunk * ipc) * J + j;
-        const int gi = M == 1 ? p : (M <= 32 ? p / M : 0);
-        const int m = M == 1 ? 0 : (M <= 32 ? p - gi * M : p);
-        const int64_t chain = g.chunk_chain0[chunk] + gi;
-        int len = 0;
-        if ((M <= 32 ? gi < Gc : p < M) && (MULTI || sl == 0)) len = g.chain_len[chain];
-        wb->slot0[it][lane] = g.chunk_base[chunk] + gi;
-        wb->chain[it][lane] = (int32_t)chain;
-        wb->len[it][lane] = len;
-        wb->m[it][lane] = m;
-        if (lane == 0) {
-            wb->L[it] = L;
-            wb->Gc[it] = Gc;
-        }
-        work |= len;
-        npos += L;
-    }
-    __syncwarp();
-    if (!__any_sync(0xffffffffu, work > 0)) return true;  // items past their chunks' pairs
     const bool lead = sl == 0;
     for (int r = 0; r < rounds; ++r) {
         const int s = r * SU + sl;
@@ -309,14 +250,14 @@ __device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, P
         Cursor cur2;
         cur2.reset(wb, count);
         if (lead) {
-            cur2.resolve(wb, count, lane, pc);
+            cur2.resolve(wb, count, lp, pc);
             if (pc.flags) {
                 ucur = load_rec(g, pc.slot);
                 phys.load(pc.slot, pc.slot * M + pc.m, pc.m, fresh, r > 0, cur);
                 load_words(g, pc.m, ucur, s0, c0, c1);
             }
             cur2.advance(wb, count);
-            cur2.resolve(wb, count, lane, pn);
+            cur2.resolve(wb, count, lp, pn);
             if (pn.flags) unxt = load_rec(g, pn.slot);
         }
         In x;
@@ -341,7 +282,7 @@ __device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, P
                     load_words(g, pn.m, unxt, s0, n0, n1);
                 }
                 cur2.advance(wb, count);
-                cur2.resolve(wb, count, lane, pnn);
+                cur2.resolve(wb, count, lp, pnn);
                 if (pnn.flags) unn = load_rec(g, pnn.slot);
             }
             bool ok = true;
@@ -384,37 +325,40 @@ __device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, P
 }
 
 // Tickets: the last p_chunks chunks (one long chain each) longest first, with SLp lanes per pair, then
-// the other chunks in dependency order with SLr lanes, the short ones in batches of `batch`.
+// the other chunks in dependency order, the short ones with SLs lanes in batches of `batch`, the rest
+// with SLr lanes.
 template <class Phys, bool MULTI>
-__device__ __forceinline__ void walk(Phys& phys, int64_t p_chunks, int SLp, int SLr, int batch, int32_t* status) {
+__device__ __forceinline__ void walk(Phys& phys, int64_t p_chunks, int SLp, int SLs, int SLr, int batch, int32_t* status) {
     extern __shared__ unsigned long long wave_smem[];
     const WfDevGraph& g = phys.g;
     const WfSweep& sw = phys.sw;
     const unsigned lane = threadIdx.x & 31u;
     Batch* wb = reinterpret_cast<Batch*>(wave_smem) + (threadIdx.x >> 5);
-    const int64_t ipp = wf_items_per_chunk(1, g.M, SLp), ipr = wf_items_per_chunk(g.G, g.M, SLr);
+    const int64_t ipp = wf_items_per_chunk(1, g.M, SLp), ips = wf_items_per_chunk(g.G, g.M, SLs),
+                  ipr = wf_items_per_chunk(g.G, g.M, SLr);
     const int64_t nd = p_chunks * ipp, rest = g.n_chunks - p_chunks;
-    const int64_t n_short = min(g.n_short_chunks, rest) * ipr;
+    const int64_t short_chunks = min(g.n_short_chunks, rest), n_short = short_chunks * ips;
     const int64_t n_sb = (n_short + batch - 1) / batch;
-    const int64_t total = nd + n_sb + (rest * ipr - n_short);
+    const int64_t total = nd + n_sb + (rest - short_chunks) * ipr;
     while (true) {
         unsigned long long t0 = 0;
         if (lane == 0) t0 = atomicAdd(g.ticket, 1ULL);
         const int64_t t = (int64_t)__shfl_sync(0xffffffffu, t0, 0);
         if (t >= total) return;
-        int64_t first, ipc = ipr;
-        int count = 1, SL = SLr;
-        if (t < nd) {
-            first = g.n_chunks * ipp - 1 - t;
-            ipc = ipp;
-            SL = SLp;
-        } else {
+        int64_t first = g.n_chunks * ipp - 1 - t, ipc = ipp;
+        int count = 1, SL = SLp, npos;
+        if (t >= nd) {
             const int64_t v = t - nd;
-            first = v < n_sb ? v * batch : n_short + (v - n_sb);
-            if (v < n_sb) count = (int)min((int64_t)batch, n_short - first);
+            const bool is_short = v < n_sb;
+            first = is_short ? v * batch : short_chunks * ipr + (v - n_sb);
+            if (is_short) count = (int)min((int64_t)batch, n_short - first);
+            SL = is_short ? SLs : SLr;
+            ipc = is_short ? ips : ipr;
         }
+        wfv::LanePair lp;
         __syncwarp();
-        if (!ticket<Phys, MULTI>(g, sw, phys, status, first, count, SL, ipc, wb)) return;
+        if (!wfv::fill_batch(g, first, count, SL, ipc, MULTI || (lane & (SL - 1)) == 0, wb, lp, npos)) continue;
+        if (!ticket<Phys, MULTI>(g, sw, phys, status, count, SL, lp, npos, wb)) return;
     }
 }
 
