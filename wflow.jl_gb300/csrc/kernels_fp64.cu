@@ -938,6 +938,7 @@ __global__ void __launch_bounds__(128) ssf_prep64_kernel(WfDevFields F, WfSweep 
 
 template <int MAXN>
 struct SsfWave64 {
+    static constexpr bool kLand = true, kTr = false;
     WfDevFields F;
     WfDevGraph g;
     WfSweep sw;
@@ -974,11 +975,9 @@ struct SsfWave64 {
                                  F.Mf[Q_MAX][e], L[KH_RATIO][slot] * col.kv0, col, q, zi_new, exfilt, netflux);
         return q;
     }
-    __device__ __forceinline__ bool sub(const In& x, St& st, const wfz::Rec& r, unsigned long long w0,
-                                        unsigned long long w1, int64_t slot, int64_t e, int m, int s, int64_t chain,
-                                        bool is_end, bool heavy, double& hq, bool more) {
-        double qin, tr;
-        if (!wfz::gather<true, false>(g, sw, r, w0, w1, slot, m, s, heavy, hq, F.status, qin, tr)) return false;
+    __device__ __forceinline__ bool active(int, St&) const { return true; }
+    __device__ __forceinline__ void sub(const In& x, St& st, const wfz::Rec& r, double qin, double tr, int64_t slot,
+                                        int64_t e, int m, int s, int64_t chain, bool is_end, double& hq, bool more) {
         double q;
         // the early-out of kinematic_wave_ssf; its full form decides when a discharge is negative
         const bool none = wfm::is_zero_(qin) && wfm::is_zero_(x.q_prev);
@@ -996,7 +995,6 @@ struct SsfWave64 {
         st.q = q;
         hq = q;
         if (is_end) wfz::publish(g, chain, m, s, q);
-        return true;
     }
     __device__ __forceinline__ void finish(const St& st, int64_t e, bool) const { F.W[W_Q][e] = st.q; }
 };
@@ -1091,6 +1089,7 @@ __global__ void __launch_bounds__(128) kw_prep64_kernel(WfDevFields F, WfSweep s
 // reservoir cell hands its reservoir's outflow, not its river discharge, to the downstream cell.
 template <bool LAND, bool CUM, bool RES>
 struct KwWave64 {
+    static constexpr bool kLand = LAND, kTr = CUM;
     WfDevFields F;
     WfDevGraph g;
     WfSweep sw;
@@ -1143,19 +1142,15 @@ struct KwWave64 {
         st.c_qin = x.c_qin;
         st.c_x = x.c_x;
     }
-    __device__ __forceinline__ bool sub(const In& x, St& st, const wfz::Rec& r, unsigned long long w0,
-                                        unsigned long long w1, int64_t slot, int64_t e, int m, int s, int64_t chain,
-                                        bool is_end, bool heavy, double& hq, bool more) {
-        double dt_s = sw.dt_s;
-        if (sw.aflag) {  // a member that has reached the end of the step takes no further sub-step
-            if (!(sw.aflag[m] & WF_SUB_ACTIVE)) {
-                st.u = -1.0;
-                return true;
-            }
-            dt_s = sw.adt[m];
-        }
-        double qin, tr;
-        if (!wfz::gather<LAND, CUM>(g, sw, r, w0, w1, slot, m, s, heavy, hq, F.status, qin, tr)) return false;
+    // a member that has reached the end of the step takes no further sub-step
+    __device__ __forceinline__ bool active(int m, St& st) const {
+        if (!sw.aflag || (sw.aflag[m] & WF_SUB_ACTIVE)) return true;
+        st.u = -1.0;
+        return false;
+    }
+    __device__ __forceinline__ void sub(const In& x, St& st, const wfz::Rec& r, double qin, double tr, int64_t slot,
+                                        int64_t e, int m, int s, int64_t chain, bool is_end, double& hq, bool more) {
+        const double dt_s = sw.aflag ? sw.adt[m] : sw.dt_s;
         if (LAND && (r.flags & wfz::REC_NO_INFLOW)) qin = 0.0;
         const float r_dt32 = __frcp_rn(wfm::f32_of(dt_s));
         double b = x.b, q_lat = 0.0, taken = 0.0;
@@ -1201,7 +1196,6 @@ struct KwWave64 {
         st.q_prev = q;
         st.u = u;
         if (more) wfz::kw_state(q, x.dt_dx, x.alpha, x.c1, x.c2, st.k);
-        return true;
     }
     __device__ __forceinline__ void finish(const St& st, int64_t e, bool last_round) const {
         if (lt_(st.u, 0.0)) return;  // no sub-step taken

@@ -1488,11 +1488,13 @@ struct SsfWave {
     __device__ __forceinline__ void start(const In&, St&) const {}
     __device__ __forceinline__ bool active(int, bool& first) const { return true; }
     __device__ __forceinline__ void finish(const St&, int64_t, bool) const {}
-    __device__ __forceinline__ bool sub(const In& x, St&, unsigned long long w0, unsigned long long w1, int64_t slot,
-                                        int64_t e, int m, int s, int64_t chain, bool is_end, bool heavy,
-                                        unsigned long long qh_in, unsigned long long& qh_out) const {
-        wff::ff qinff;
-        if (!wfv::gather_w<true>(g, sw, x.up, w0, w1, slot, m, 0, heavy, qh_in, F.status, qinff)) return false;
+    __device__ __forceinline__ bool gather(const In& x, const St&, unsigned long long w0, unsigned long long w1,
+                                           int64_t slot, int m, int s, bool heavy, unsigned long long qh, wff::ff& qin,
+                                           wff::ff&) const {
+        return wfv::gather_w<true>(g, sw, x.up, w0, w1, slot, m, 0, heavy, qh, F.status, qin);
+    }
+    __device__ __forceinline__ void sub(const In& x, St&, wff::ff qinff, wff::ff, int64_t slot, int64_t e, int m, int s,
+                                        int64_t chain, bool is_end, unsigned long long& qh_out) const {
         const float qin = qinff.hi + qinff.lo;
         float q = 0.0f, qu = 0.0f;
         int flag;
@@ -1545,7 +1547,6 @@ struct SsfWave {
         qh_out = wff::pack(qf);
         if (is_end) wfv::publish(g, chain, m, 0, qf);
         F.ssf_out[e] = make_float4(q, qu, qin, (float)flag);
-        return true;
     }
 };
 
@@ -1649,48 +1650,41 @@ struct OlWave {
         return (f & WF_SUB_ACTIVE) != 0;
     }
     // gather_w<true> with, at the land cell of a river cell, the upstream flow to the river
-    __device__ __forceinline__ bool gather_tr(const In& x, int32_t rs, unsigned long long w0, unsigned long long w1,
-                                              int64_t slot, int m, int s, bool heavy, unsigned long long qh, wff::ff& qin,
+    __device__ __forceinline__ bool gather(const In& x, const St& st, unsigned long long w0, unsigned long long w1,
+                                           int64_t slot, int m, int s, bool heavy, unsigned long long qh, wff::ff& qin,
                                               wff::ff& tr) const {
         const wfv::UpRec& r = x.up;
-        const bool riv = rs >= 0;
+        const bool riv = st.rs >= 0;
         wff::ff acc = {0.0f, 0.0f}, t = {0.0f, 0.0f};
         if (heavy) {
             const wff::ff q = wff::unpack(qh);
             acc = wff::mul(q, r.w_hv);
             if (riv) t = wff::mul(q, x.fr_hv);
         }
+        if (!wfv::await_two(g, sw, r.lt0, r.lt1, m, s, w0, w1, F.status)) return false;
         if (r.lt0 >= 0) {
-            const int64_t idx = wfv::end_index(g, r.lt0, m, s);
-            unsigned long long first = w0;
-            if (first == wfv::SENTINEL) first = wfv::ld_relaxed(&g.end_q[idx]);
-            unsigned long long w;
-            if (!wfv::await_end(g, sw, idx, first, F.status, w)) return false;
-            const wff::ff q = wff::unpack(w);
+            const wff::ff q = wff::unpack(w0);
             acc = wff::add(acc, wff::mul(q, r.w_lt0));
             if (riv) t = wff::add(t, wff::mul(q, x.fr0));
         }
         if (r.lt1 >= 0) {
-            const int64_t idx = wfv::end_index(g, r.lt1, m, s);
-            unsigned long long first = w1;
-            if (first == wfv::SENTINEL) first = wfv::ld_relaxed(&g.end_q[idx]);
-            unsigned long long w;
-            if (!wfv::await_end(g, sw, idx, first, F.status, w)) return false;
-            const wff::ff q = wff::unpack(w);
+            const wff::ff q = wff::unpack(w1);
             acc = wff::add(acc, wff::mul(q, r.w_lt1));
             if (riv) t = wff::add(t, wff::mul(q, x.fr1));
         }
         if (r.n_lt > 2) {  // further light children, in up-list order after the first two
-            int seen = 0;
-            for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
-                const int32_t uc = g.up_chain[o];
-                if (uc < 0 || ++seen <= 2) continue;
-                const int64_t idx = wfv::end_index(g, uc, m, s);
-                unsigned long long w;
-                if (!wfv::await_end(g, sw, idx, wfv::ld_relaxed(&g.end_q[idx]), F.status, w)) return false;
-                const wff::ff q = wff::unpack(w);
-                acc = wff::add(acc, wff::mul(q, g.up_wf[o]));
-                if (riv) t = wff::add(t, wff::mul(q, g.up_frf[o]));
+            int skip = 2;
+            const int32_t o1 = __ldg(g.up_ptr + slot + 1);
+            for (int32_t o = __ldg(g.up_ptr + slot); o < o1; o += wfv::GROUP) {
+                wfv::UpGroup u;
+                if (!wfv::gather_group(g, sw, o, o1, skip, m, s, F.status, u)) return false;
+#pragma unroll
+                for (int i = 0; i < wfv::GROUP; ++i) {
+                    if (u.chain[i] < 0) continue;
+                    const wff::ff q = wff::unpack(u.word[i]);
+                    acc = wff::add(acc, wff::mul(q, __ldg(g.up_wf + o + i)));
+                    if (riv) t = wff::add(t, wff::mul(q, __ldg(g.up_frf + o + i)));
+                }
             }
         }
         qin = acc;
@@ -1698,15 +1692,12 @@ struct OlWave {
         return true;
     }
     // sub-step s of the node
-    __device__ __forceinline__ bool sub(const In& x, St& st, unsigned long long w0, unsigned long long w1,
-                                        int64_t slot, int64_t e, int m, int s, int64_t chain, bool is_end, bool heavy,
-                                        unsigned long long qh_in, unsigned long long& qh_out) const {
+    __device__ __forceinline__ void sub(const In& x, St& st, wff::ff qin, wff::ff tr, int64_t slot, int64_t e, int m,
+                                        int s, int64_t chain, bool is_end, unsigned long long& qh_out) const {
         using DT = typename std::conditional<ADAPT, wff::ff, float>::type;
         DT dt_s;
         if constexpr (ADAPT) dt_s = wff::ff{sw.adt_hi[m], sw.adt_lo[m]};
         else dt_s = sw.dts_f[s];
-        wff::ff qin, tr;
-        if (!gather_tr(x, st.rs, w0, w1, slot, m, s, heavy, qh_in, qin, tr)) return false;
         if (__float_as_int(x.alpha) < 0) qin = {0.0f, 0.0f};
         wff::ff un, qn;
         kw_node_ff<ADAPT>(qin, st.qp, x.qlat, st.u, x.invdx, dt_s, fabsf(x.alpha), un, qn);
@@ -1716,7 +1707,6 @@ struct OlWave {
         if (is_end) wfv::publish(g, chain, m, s, qn);
         st.qsum = wff::add(st.qsum, mul_dt(qn, dt_s));
         if (st.rs >= 0) st.trsum = wff::add(st.trsum, mul_dt(tr, dt_s));
-        return true;
     }
     // the node's state after the last sub-step of the launch (or of a round of the diagonal
     // schedule); add_stored: the step's cumulative discharge so far is added. At the land cell of
@@ -1812,10 +1802,14 @@ struct RvWave {
         first = (f & WF_SUB_FIRST) != 0;
         return (f & WF_SUB_ACTIVE) != 0;
     }
+    __device__ __forceinline__ bool gather(const In& x, const St&, unsigned long long w0, unsigned long long w1,
+                                           int64_t slot, int m, int s, bool heavy, unsigned long long qh, wff::ff& qin,
+                                           wff::ff&) const {
+        return wfv::gather_w<false>(g, sw, x.up, w0, w1, slot, m, s, heavy, qh, F.status, qin);
+    }
     // sub-step s of the node
-    __device__ __forceinline__ bool sub(const In& x, St& st, unsigned long long w0, unsigned long long w1,
-                                        int64_t slot, int64_t e, int m, int s, int64_t chain, bool is_end, bool heavy,
-                                        unsigned long long qh_in, unsigned long long& qh_out) const {
+    __device__ __forceinline__ void sub(const In& x, St& st, wff::ff qin, wff::ff tr, int64_t slot, int64_t e, int m,
+                                        int s, int64_t chain, bool is_end, unsigned long long& qh_out) const {
         using DT = typename std::conditional<ADAPT, wff::ff, float>::type;
         DT dt_s;
         float dt_f;
@@ -1826,8 +1820,6 @@ struct RvWave {
             dt_s = sw.dts_f[s];
             dt_f = dt_s;
         }
-        wff::ff qin;
-        if (!wfv::gather_w<false>(g, sw, x.up, w0, w1, slot, m, s, heavy, qh_in, F.status, qin)) return false;
         wff::ff ql = st.qlatt;
         if (x.ext < 0.0f) {  // abstraction: qlatt holds the lateral inflow alone
             const float storage = x.len * (x.alpha * (st.u.hi * st.u.hi * st.u.hi));
@@ -1847,7 +1839,6 @@ struct RvWave {
         qh_out = wff::pack(q_down);
         if (is_end) wfv::publish(g, chain, m, s, q_down);
         st.qsum = wff::add(st.qsum, mul_dt(qn, dt_s));
-        return true;
     }
     // the node's state after the last sub-step of the launch (or of a round of the diagonal
     // schedule); add_stored: the step's cumulative discharge and abstraction so far are added

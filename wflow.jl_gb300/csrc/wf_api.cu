@@ -1388,15 +1388,15 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
                 const int64_t node = P.node_of_slot[sl];
                 if (node < 0) continue;
                 int4& q = r64[sl];
-                int entries = 0, heavy_at = -1;
+                int entries = 0, heavy_at = -1, lights = 0;
                 for (int32_t o = P.up_ptr[sl]; o < P.up_ptr[sl + 1]; ++o, ++entries) {
                     const bool heavy = P.up_chain[o] < 0;
                     if (heavy) heavy_at = entries;
-                    const int at = heavy ? 0 : q.w + 1;  // heavy child, light child 0, light child 1
+                    const int at = heavy ? 0 : lights + 1;  // heavy child, light child 0, light child 1
                     if (!heavy) {
-                        if (q.w == 0) q.x = P.up_chain[o];
-                        if (q.w == 1) q.y = P.up_chain[o];
-                        q.w += 1;
+                        if (lights == 0) q.x = P.up_chain[o];
+                        if (lights == 1) q.y = P.up_chain[o];
+                        ++lights;
                     }
                     if (g == 0 && at < 3) {
                         w64[sl * 6 + 2 * at] = w[o];
@@ -1407,6 +1407,8 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
                 if (heavy_at >= 0 && heavy_at == entries - 1) q.z |= wfz::REC_HEAVY_LAST;
                 if (g == 0 && !(d->surface_flow_width[node] > 0.0)) q.z |= wfz::REC_NO_INFLOW;
                 if (g == 1 && r_ext[node] < 0.0) q.z |= wfz::REC_ABSTRACTION;
+                q.z |= lights << wfz::REC_LIGHTS;
+                q.w = P.up_ptr[sl];
             }
             CKR(upload(h, &G.up_rec64, r64));
             CKR(upload(h, &G.up_w64, w64));

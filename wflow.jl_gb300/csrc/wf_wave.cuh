@@ -60,34 +60,75 @@ __device__ __forceinline__ int64_t end_index(const WfDevGraph& g, int64_t chain,
     return (chain * g.s_cap + s) * g.M + m;
 }
 
-// Discharge word published at end_q[idx]; `first` is a value already loaded from that slot (or
-// the sentinel). False when the budget ran out or another lane aborted. A non-zero
-// sw.wait_offset (test hook, 0 in production) makes every wait run out.
-__device__ __forceinline__ bool await_end(const WfDevGraph& g, const WfSweep& sw, int64_t idx,
-                                          unsigned long long first, int32_t* status, unsigned long long& out) {
-    unsigned long long b = first;
-    if (b != SENTINEL && sw.wait_offset == 0) {
-        out = b;
-        return true;
-    }
+// Whether a wait since t0 goes on. Called after a poll that failed: the order matters, a poll takes a round
+// trip to L2 and so does the status word.
+__device__ __forceinline__ bool wait_goes_on(const WfSweep& sw, uint64_t t0, int32_t* status) {
+    if (status_ld(status) & WF_DEV_SPIN_TIMEOUT) return false;
+    if (now_ns() - t0 <= sw.wait_ns) return true;
+    atomicOr(status, WF_DEV_SPIN_TIMEOUT);
+    return false;
+}
+
+// The words of the chains lt0 and lt1 (negative: none) at sub-step s, waited for together; w0 / w1 hold
+// the values loaded earlier (or the sentinel). False when the budget ran out or another lane aborted. A
+// non-zero sw.wait_offset (test hook, 0 in production) makes every wait run out.
+__device__ __forceinline__ bool await_two(const WfDevGraph& g, const WfSweep& sw, int32_t lt0, int32_t lt1, int m, int s,
+                                          unsigned long long& w0, unsigned long long& w1, int32_t* status) {
+    auto missing = [&]() {
+        if (lt0 >= 0 && w0 == SENTINEL) w0 = ld_relaxed(&g.end_q[end_index(g, lt0, m, s)]);
+        if (lt1 >= 0 && w1 == SENTINEL) w1 = ld_relaxed(&g.end_q[end_index(g, lt1, m, s)]);
+        return (lt0 >= 0 && (w0 == SENTINEL || sw.wait_offset != 0)) ||
+               (lt1 >= 0 && (w1 == SENTINEL || sw.wait_offset != 0));
+    };
+    if (!missing()) return true;
     const uint64_t t0 = now_ns();
     while (true) {
         __nanosleep(32);
-        b = ld_relaxed(&g.end_q[idx]);
-        if (b != SENTINEL && sw.wait_offset == 0) {
-            out = b;
-            return true;
-        }
-        if (status_ld(status) & WF_DEV_SPIN_TIMEOUT) return false;
-        if (now_ns() - t0 > sw.wait_ns) {
-            atomicOr(status, WF_DEV_SPIN_TIMEOUT);
-            return false;
-        }
+        if (!missing()) return true;
+        if (!wait_goes_on(sw, t0, status)) return false;
     }
 }
 
 __device__ __forceinline__ void publish(const WfDevGraph& g, int64_t chain, int m, int s, wff::ff q) {
     st_relaxed(&g.end_q[end_index(g, chain, m, s)], wff::pack(q));
+}
+
+// Up to GROUP entries of a node's upstream list, for the nodes with more than two light children. Their
+// chains are loaded together, then their words, then waited for together: one at a time, each entry took
+// three dependent loads, and with 24 sub-steps in a warp some lane is at such a node in most steps of a
+// long chain (daily overland flow: 64 x 64 cells in FP64 3.15 -> 2.70 ms, 40 uneven catchments in the
+// split form 15.2 -> 12.4).
+constexpr int GROUP = 4;
+struct UpGroup {
+    int32_t chain[GROUP];  // -1: the heavy child, -2: no entry
+    unsigned long long word[GROUP];
+};
+// Entries from o on (o1: end of the list) at sub-step s; the first `skip` light children are left out.
+__device__ __forceinline__ bool gather_group(const WfDevGraph& g, const WfSweep& sw, int32_t o, int32_t o1, int& skip,
+                                             int m, int s, int32_t* status, UpGroup& u) {
+#pragma unroll
+    for (int i = 0; i < GROUP; ++i) u.chain[i] = o + i < o1 ? __ldg(g.up_chain + o + i) : -2;
+#pragma unroll
+    for (int i = 0; i < GROUP; ++i) {
+        if (u.chain[i] >= 0 && --skip >= 0) u.chain[i] = -2;
+        u.word[i] = u.chain[i] >= 0 ? ld_relaxed(&g.end_q[end_index(g, u.chain[i], m, s)]) : 0ull;
+    }
+    auto missing = [&]() {
+        bool any = sw.wait_offset != 0;
+#pragma unroll
+        for (int i = 0; i < GROUP; ++i) any |= u.word[i] == SENTINEL;
+        return any;
+    };
+    if (!missing()) return true;
+    const uint64_t t0 = now_ns();
+    while (true) {
+        __nanosleep(32);
+#pragma unroll
+        for (int i = 0; i < GROUP; ++i)
+            if (u.word[i] == SENTINEL) u.word[i] = ld_relaxed(&g.end_q[end_index(g, u.chain[i], m, s)]);
+        if (!missing()) return true;
+        if (!wait_goes_on(sw, t0, status)) return false;
+    }
 }
 
 // Upstream inflow record of one node. A node at chain position k > 0 has its heavy child at
@@ -115,34 +156,27 @@ __device__ __forceinline__ bool gather_w(const WfDevGraph& g, const WfSweep& sw,
         const wff::ff q = wff::unpack(qh);
         acc = WEIGHTED ? wff::mul(q, r.w_hv) : q;
     }
+    if (!await_two(g, sw, r.lt0, r.lt1, m, s, w0, w1, status)) return false;
     if (r.lt0 >= 0) {
-        const int64_t idx = end_index(g, r.lt0, m, s);
-        unsigned long long first = w0;
-        if (first == SENTINEL) first = ld_relaxed(&g.end_q[idx]);
-        unsigned long long w;
-        if (!await_end(g, sw, idx, first, status, w)) return false;
-        const wff::ff q = wff::unpack(w);
+        const wff::ff q = wff::unpack(w0);
         acc = WEIGHTED ? wff::add(acc, wff::mul(q, r.w_lt0)) : wff::add(acc, q);
     }
     if (r.lt1 >= 0) {
-        const int64_t idx = end_index(g, r.lt1, m, s);
-        unsigned long long first = w1;
-        if (first == SENTINEL) first = ld_relaxed(&g.end_q[idx]);
-        unsigned long long w;
-        if (!await_end(g, sw, idx, first, status, w)) return false;
-        const wff::ff q = wff::unpack(w);
+        const wff::ff q = wff::unpack(w1);
         acc = WEIGHTED ? wff::add(acc, wff::mul(q, r.w_lt1)) : wff::add(acc, q);
     }
     if (r.n_lt > 2) {  // further light children, in up-list order after the first two
-        int seen = 0;
-        for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
-            const int32_t uc = g.up_chain[o];
-            if (uc < 0 || ++seen <= 2) continue;
-            const int64_t idx = end_index(g, uc, m, s);
-            unsigned long long w;
-            if (!await_end(g, sw, idx, ld_relaxed(&g.end_q[idx]), status, w)) return false;
-            const wff::ff q = wff::unpack(w);
-            acc = WEIGHTED ? wff::add(acc, wff::mul(q, g.up_wf[o])) : wff::add(acc, q);
+        int skip = 2;
+        const int32_t o1 = __ldg(g.up_ptr + slot + 1);
+        for (int32_t o = __ldg(g.up_ptr + slot); o < o1; o += GROUP) {
+            UpGroup u;
+            if (!gather_group(g, sw, o, o1, skip, m, s, status, u)) return false;
+#pragma unroll
+            for (int i = 0; i < GROUP; ++i) {
+                if (u.chain[i] < 0) continue;
+                const wff::ff q = wff::unpack(u.word[i]);
+                acc = WEIGHTED ? wff::add(acc, wff::mul(q, __ldg(g.up_wf + o + i))) : wff::add(acc, q);
+            }
         }
     }
     qin = acc;
@@ -300,9 +334,11 @@ __device__ __forceinline__ void shfl_up_pod(T& v, int width) {
 //   void start(const In&, St&)                            state at the start of a round
 //   bool active(m, first)                                 whether member m takes the launch's sub-step;
 //                                                         adaptive sub-steps: first of the model step
-//   bool sub(const In&, St&, w0, w1, slot, e, m, s, chain, is_end, heavy, qh_in, qh_out)
-//     one sub-step: w0 / w1 the light children's end_q words of sub-step s (or SENTINEL),
-//     qh_in the heavy child's packed discharge of sub-step s, qh_out this node's. False to abort.
+//   bool gather(const In&, const St&, w0, w1, slot, m, s, heavy, qh_in, qin, tr)
+//     the inflow of sub-step s: w0 / w1 the light children's end_q words (or SENTINEL), qh_in the
+//     heavy child's packed discharge. False to abort.
+//   void sub(const In&, St&, qin, tr, slot, e, m, s, chain, is_end, qh_out)
+//     the sub-step after its gather; qh_out the node's packed discharge
 //   void finish(const St&, e, add_stored)                 stores after the last sub-step of a round
 //                                                         (add_stored: add the stored cumulative sums)
 // The copies and their commit carry no compiler memory clobber (it would force every shared
@@ -426,24 +462,27 @@ __device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, P
             }
             stage();
             unsigned long long v0 = SENTINEL, v1 = SENTINEL;  // words of sub-step s + 1 for the next lane
-            if (ps.y && works) {
-                const int flags = (unsigned)ps.y >> 28, m = ps.z, chain = ps.w;
-                const int64_t slot = ((int64_t)(ps.y & 0x0fffffff) << 32) | (uint32_t)ps.x;
-                const int64_t e = slot * M + m;
-                if (MULTI && sl + 1 < SU && s + 1 < sw.S) load_words(g, m, x.up.lt0, x.up.lt1, s + 1, v0, v1);
-                bool first_of_step = sw.first == 0;
-                if (phys.active(m, first_of_step)) {
-                    unsigned long long out = 0ull;
-                    ok = phys.sub(x, st, w0, w1, slot, e, m, s, chain, (flags & P_END) != 0, (flags & P_HEAVY) != 0, hq,
-                                  out);
-                    hq = out;
-                    if (ok && last_lane) phys.finish(st, e, r > 0 || !first_of_step);
-                }
-            }
+            const bool here = ps.y && works;
+            const int flags = (unsigned)ps.y >> 28, m = ps.z, chain = ps.w;
+            const int64_t slot = ((int64_t)(ps.y & 0x0fffffff) << 32) | (uint32_t)ps.x;
+            bool first_of_step = sw.first == 0;
+            const bool acts = here && phys.active(m, first_of_step);
+            if (here && MULTI && sl + 1 < SU && s + 1 < sw.S) load_words(g, m, x.up.lt0, x.up.lt1, s + 1, v0, v1);
+            wff::ff qin = {0.0f, 0.0f}, tr = {0.0f, 0.0f};
+            if (acts) ok = phys.gather(x, st, w0, w1, slot, m, s, (flags & P_HEAVY) != 0, hq, qin, tr);
+            // The lanes meet after their waits: lanes that wait differently would otherwise run the rest of
+            // the step group by group (daily steps of 40 uneven catchments: overland 12.4 -> 9.1 ms, river
+            // 12.4 -> 9.5).
             if (__any_sync(0xffffffffu, !ok)) {
                 ok = false;
                 return false;
             }
+            if (acts) {
+                const int64_t e = slot * M + m;
+                phys.sub(x, st, qin, tr, slot, e, m, s, chain, (flags & P_END) != 0, hq);
+                if (last_lane) phys.finish(st, e, r > 0 || !first_of_step);
+            }
+            __syncwarp();
             if constexpr (MULTI) {
                 if (SL > 1) {  // hand the node to the next lane
                     typename Phys::Pass pass;

@@ -13,7 +13,7 @@
 // takes sub-step r SL + l of round r and at time t works on position t - l; the node's state goes from
 // lane to lane by warp shuffles, the heavy child's discharge stays in the lane. Launches of one
 // sub-step (SL = 1) skip the hand-over. Chain ends publish their discharge's bits into end_q, filled
-// with a sentinel before the launch (wf_wave.cuh await_end).
+// with a sentinel before the launch (wf_wave.cuh await_two).
 //
 // The loads of a position (inputs, light children's words) are issued one position ahead, its
 // upstream record two ahead: a position takes 3000 cycles and more, several times a memory round
@@ -27,36 +27,45 @@ namespace wfz {
 
 using wfv::SENTINEL;
 
-// Upstream record of a node (up_rec64): the chains of the first two light children (-1 none), flags,
-// and the number of light children. The reference adds the inflows in ascending cell order: with up
-// to two light children that order only matters when the heavy child is the last of three.
-struct Rec {
-    int32_t lt0, lt1, flags, n_lt;
-};
+// Upstream record of a node (up_rec64): the chains of the first two light children (-1 none), flags
+// with the number of light children, and where its upstream list starts. The reference adds the inflows
+// in ascending cell order: with up to two light children that order only matters when the heavy child is
+// the last of three.
 constexpr int32_t REC_HEAVY_LAST = 1;
 constexpr int32_t REC_WEIGHTED = 2;     // land: some child sends a fraction of its discharge to the river
 constexpr int32_t REC_NO_INFLOW = 4;    // land: no surface flow width, the overland inflow does not count
 constexpr int32_t REC_ABSTRACTION = 8;  // river: a negative external inflow, limited by the storage
+constexpr int REC_LIGHTS = 8;           // flags: number of light children from this bit on
+struct Rec {
+    int32_t lt0, lt1, flags, list;
+    __device__ __forceinline__ int n_lt() const { return flags >> REC_LIGHTS; }
+};
 
 __device__ __forceinline__ Rec load_rec(const WfDevGraph& g, int64_t slot) {
     const int4 v = g.up_rec64[slot];
     return {v.x, v.y, v.z, v.w};
 }
 
+// What the gather of the position after the next reads besides the words, into L1
+template <bool LAND>
+__device__ __forceinline__ void prefetch_lists(const WfDevGraph& g, int64_t slot, const Rec& r) {
+    auto l1 = [](const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); };
+    if (r.n_lt() > 2) {
+        l1(g.up_chain + r.list);
+        if (LAND) {
+            l1(g.up_w + r.list);
+            l1(g.up_fr + r.list);
+        }
+    } else if (LAND && (r.flags & REC_WEIGHTED)) {
+        l1(g.up_w64 + slot * 6);
+        l1(g.up_w64 + slot * 6 + 5);
+    }
+}
+
 __device__ __forceinline__ void load_words(const WfDevGraph& g, int m, const Rec& r, int s, unsigned long long& w0,
                                            unsigned long long& w1) {
     w0 = r.lt0 >= 0 ? wfv::ld_relaxed(&g.end_q[wfv::end_index(g, r.lt0, m, s)]) : SENTINEL;
     w1 = r.lt1 >= 0 ? wfv::ld_relaxed(&g.end_q[wfv::end_index(g, r.lt1, m, s)]) : SENTINEL;
-}
-
-__device__ __forceinline__ bool await(const WfDevGraph& g, const WfSweep& sw, int32_t chain, int m, int s,
-                                      unsigned long long first, int32_t* status, double& q) {
-    const int64_t idx = wfv::end_index(g, chain, m, s);
-    if (first == SENTINEL) first = wfv::ld_relaxed(&g.end_q[idx]);
-    unsigned long long w;
-    if (!wfv::await_end(g, sw, idx, first, status, w)) return false;
-    q = wfm::from_bits(w);
-    return true;
 }
 
 __device__ __forceinline__ void publish(const WfDevGraph& g, int64_t chain, int m, int s, double q) {
@@ -79,31 +88,46 @@ __device__ __forceinline__ bool gather(const WfDevGraph& g, const WfSweep& sw, c
                                        unsigned long long w1, int64_t slot, int m, int s, bool heavy, double hq,
                                        int32_t* status, double& qin, double& tr) {
     tr = 0.0;
-    if (r.n_lt > 2) {
+    if (r.n_lt() > 2) {
         double acc = 0.0;
-        for (int32_t o = g.up_ptr[slot]; o < g.up_ptr[slot + 1]; ++o) {
-            const int32_t uc = g.up_chain[o];
-            double q = hq;
-            if (uc >= 0 && !await(g, sw, uc, m, s, SENTINEL, status, q)) return false;
-            if (LAND) {
-                acc = acc + q * g.up_w[o];
-                if (TR) tr = tr + q * g.up_fr[o];
-            } else {
-                acc = acc + q;
+        int skip = 0;
+        const int32_t o1 = r.list + r.n_lt() + (heavy ? 1 : 0);
+        for (int32_t o = r.list; o < o1; o += wfv::GROUP) {
+            double wt[wfv::GROUP] = {}, fr[wfv::GROUP] = {};
+            if (LAND)
+#pragma unroll
+                for (int i = 0; i < wfv::GROUP; ++i)
+                    if (o + i < o1) {
+                        wt[i] = __ldg(g.up_w + o + i);
+                        if (TR) fr[i] = __ldg(g.up_fr + o + i);
+                    }
+            wfv::UpGroup u;
+            if (!wfv::gather_group(g, sw, o, o1, skip, m, s, status, u)) return false;
+#pragma unroll
+            for (int i = 0; i < wfv::GROUP; ++i) {
+                if (u.chain[i] < -1) continue;
+                const double q = u.chain[i] < 0 ? hq : wfm::from_bits(u.word[i]);
+                if (LAND) {
+                    acc = acc + q * wt[i];
+                    if (TR) tr = tr + q * fr[i];
+                } else {
+                    acc = acc + q;
+                }
             }
         }
         qin = acc;
         return true;
     }
-    double a = 0.0, b = 0.0;
-    if (r.lt0 >= 0 && !await(g, sw, r.lt0, m, s, w0, status, a)) return false;
-    if (r.lt1 >= 0 && !await(g, sw, r.lt1, m, s, w1, status, b)) return false;
+    if (!wfv::await_two(g, sw, r.lt0, r.lt1, m, s, w0, w1, status)) return false;
+    double a = wfm::from_bits(w0), b = wfm::from_bits(w1);  // read only where there is a child
     if (LAND && (r.flags & REC_WEIGHTED)) {
-        const double* w = g.up_w64 + slot * 6;  // {1 - fr, fr} of the heavy child and light children 0 and 1
-        if (TR) tr = sum_up(r, heavy, hq * w[1], a * w[3], b * w[5]);
-        hq = hq * w[0];
-        if (r.lt0 >= 0) a = a * w[2];
-        if (r.lt1 >= 0) b = b * w[4];
+        // {1 - fr, fr} of the heavy child and light children 0 and 1
+        const double2* w = reinterpret_cast<const double2*>(g.up_w64 + slot * 6);
+        const double2 wh = __ldg(w), wa = __ldg(w + 1), wb = __ldg(w + 2);
+        if (TR) tr = sum_up(r, heavy, hq * wh.y, a * wa.y, b * wb.y);
+        hq = hq * wh.x;
+        if (r.lt0 >= 0) a = a * wa.x;
+        if (r.lt1 >= 0) b = b * wb.x;
     }
     qin = sum_up(r, heavy, hq, a, b);
     return true;
@@ -209,9 +233,11 @@ __device__ __forceinline__ double kw_solve(const KwState& k, double cterm, doubl
 //   void load(slot, e, m, fresh, resumed, In&)   issues the loads (fresh: before the model step's first
 //                                                sub-step; resumed: after another round of the launch)
 //   void start(const In&, St&)
-//   bool sub(const In&, St&, rec, w0, w1, slot, e, m, s, chain, is_end, heavy, hq, more)
-//     one sub-step; hq the heavy child's discharge on entry, what the node hands downstream on
-//     return; more: the launch holds another sub-step after s. False to abort.
+//   static constexpr bool kLand, kTr             arguments of gather
+//   bool active(m, St&)                          whether member m takes the sub-step
+//   void sub(const In&, St&, rec, qin, tr, slot, e, m, s, chain, is_end, hq, more)
+//     one sub-step after its gather; on return hq is what the node hands downstream; more: the launch
+//     holds another sub-step after s.
 //   void finish(const St&, e, bool last_round)   stores after the last sub-step of a round
 
 using wfv::Batch;
@@ -280,6 +306,7 @@ __device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, P
                 if (pn.flags) {
                     phys.load(pn.slot, pn.slot * M + pn.m, pn.m, fresh, r > 0, nxt);
                     load_words(g, pn.m, unxt, s0, n0, n1);
+                    prefetch_lists<Phys::kLand>(g, pn.slot, unxt);
                 }
                 cur2.advance(wb, count);
                 cur2.resolve(wb, count, lp, pnn);
@@ -287,14 +314,25 @@ __device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, P
             }
             bool ok = true;
             unsigned long long v0 = SENTINEL, v1 = SENTINEL;  // words of sub-step s + 1 for the next lane
-            if (ps.flags && works) {
-                const int64_t e = ps.slot * M + ps.m;
-                if (MULTI && sl + 1 < SU && s + 1 < sw.S) load_words(g, ps.m, u, s + 1, v0, v1);
-                ok = phys.sub(x, st, u, w0, w1, ps.slot, e, ps.m, s, ps.chain, (ps.flags & P_END) != 0,
-                              (ps.flags & P_HEAVY) != 0, hq, MULTI && s + 1 < sw.S);
-                if (ok && last_lane) phys.finish(st, e, s == sw.S - 1);
-            }
+            const bool here = ps.flags && works;
+            const bool acts = here && phys.active(ps.m, st);
+            double qin = 0.0, tr = 0.0;
+            if (here && MULTI && sl + 1 < SU && s + 1 < sw.S) load_words(g, ps.m, u, s + 1, v0, v1);
+            if (acts)
+                ok = gather<Phys::kLand, Phys::kTr>(g, sw, u, w0, w1, ps.slot, ps.m, s, (ps.flags & P_HEAVY) != 0, hq,
+                                                    status, qin, tr);
+            // The lanes meet after their waits: lanes that wait differently would otherwise run the rest of
+            // the step group by group, each at the full price of its FP64 instructions (a daily step of
+            // 64 x 64 cells: overland 2.70 -> 1.25 ms, river 6.2 -> 3.5).
             if (__any_sync(0xffffffffu, !ok)) return false;
+            if (here) {
+                const int64_t e = ps.slot * M + ps.m;
+                if (acts)
+                    phys.sub(x, st, u, qin, tr, ps.slot, e, ps.m, s, ps.chain, (ps.flags & P_END) != 0, hq,
+                             MULTI && s + 1 < sw.S);
+                if (last_lane) phys.finish(st, e, s == sw.S - 1);
+            }
+            __syncwarp();
             if (MULTI) {  // hand the node to the next lane
                 wfv::shfl_up_pod(x, SL);
                 wfv::shfl_up_pod(st, SL);
