@@ -1624,7 +1624,6 @@ cudaError_t launch_wave64(const Phys& phys, const WfLaunchCfg& c) {
     const int threads = 32 * (c.walk_warps > 0 ? std::min(c.walk_warps, 4) : 4);
     const size_t smem = wfz::walk_smem(threads);
     const WfDevGraph& g = phys.g;
-    const int SLp = g.M == 1 ? 32 : 1 << (31 - __builtin_clz(32 / std::min(g.M, 32) | 1));
     int SLr = g.lanes, SLs = SLr;
     if (MULTI) {
         const int cap = c.sub_lanes > 0 ? std::min(c.sub_lanes, 32) : 32;
@@ -1643,11 +1642,13 @@ cudaError_t launch_wave64(const Phys& phys, const WfLaunchCfg& c) {
     const int fill = std::min(per_sm, 2);
     int blocks = c.walk_blocks > 0 ? c.walk_blocks : c.num_sms * fill;
     const int wpb = threads / 32;
-    const int64_t items = g.n_chunks * wf_items_per_chunk(g.G, g.M, SLr);
+    const int64_t resident = (int64_t)std::min(blocks, c.num_sms * per_sm) * wpb;
+    const int SLp = first_lanes(g, c);
+    const int64_t p_chunks = first_chunks(g, SLp, resident);
+    const int64_t items = p_chunks * wf_items_per_chunk(1, g.M, SLp) +
+                          (g.n_chunks - p_chunks) * wf_items_per_chunk(g.G, g.M, SLr);
     const int64_t need = std::max<int64_t>((items + wpb - 1) / wpb, 1);
     if (blocks > need) blocks = (int)need;
-    const int64_t resident = (int64_t)std::min(blocks, c.num_sms * per_sm) * wpb;
-    const int64_t p_chunks = first_chunks(g, SLp, resident);
     // batches of short chains only where there are more items than warps
     const int batch = (int)std::max<int64_t>(1, std::min<int64_t>(wfv::BATCH, items / (4 * resident)));
     wave64_kernel<Phys, MULTI><<<blocks, threads, smem, c.stream>>>(phys, p_chunks, SLp, SLs, SLr, batch);

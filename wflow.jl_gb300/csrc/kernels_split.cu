@@ -1452,7 +1452,7 @@ struct SsfWave {
         bool qprev_zero;
         wfv::UpRec up;
     };
-    static constexpr int kVecs = 4;
+    static constexpr int kVecs = 4, kBlocks = 1;
     static constexpr bool kWeighted = true;
     __device__ __forceinline__ void copy(int64_t slot, int64_t e, float4* v) const {
         wfv::cpa(v, &F.ssf_dyn[e]);
@@ -1589,7 +1589,7 @@ struct OlWave {
         float fr_hv, fr0, fr1;  // fractions to the river of the heavy child and light children 0, 1
         wfv::UpRec up;
     };
-    static constexpr int kVecs = 4;
+    static constexpr int kVecs = 4, kBlocks = 4;
     static constexpr bool kWeighted = true;
     __device__ __forceinline__ void copy(int64_t slot, int64_t e, float4* v) const {
         wfv::cpa(v, &F.ol_uq[e]);
@@ -1747,7 +1747,7 @@ struct RvWave {
         int32_t res;  // reservoir at this cell (RES only), or -1
         wfv::UpRec up;
     };
-    static constexpr int kVecs = 4;
+    static constexpr int kVecs = 4, kBlocks = 4;
     static constexpr bool kWeighted = false;
     __device__ __forceinline__ void copy(int64_t slot, int64_t e, float4* v) const {
         wfv::cpa(v, &F.rv_uq[e]);
@@ -1858,8 +1858,11 @@ struct RvWave {
     }
 };
 
+// kBlocks: 4 blocks per SM for overland and river flow (128 registers; hourly river sweep of 64 members of
+// 256 x 256 cells 0.98 ms with 3, 0.94 with 4); the subsurface kernel needs 232 registers for the column of
+// the cells that take the full solve.
 template <class Phys, bool MULTI>
-__global__ void __launch_bounds__(128, 1) wave_kernel(Phys phys, int64_t p_chunks, int SLp, int SLs, int SLr,
+__global__ void __launch_bounds__(128, Phys::kBlocks) wave_kernel(Phys phys, int64_t p_chunks, int SLp, int SLs, int SLr,
                                                    int batch) {
     wfv::walk<Phys, MULTI>(phys, p_chunks, SLp, SLs, SLr, batch, phys.F.status);
 }
@@ -1877,7 +1880,7 @@ cudaError_t launch_wave_as(const Phys& phys, const WfLaunchCfg& c) {
     auto kernel = wave_kernel<Phys, MULTI>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    int SLp = g.M == 1 ? 32 : 1, SLs = 1, SLr = std::min(g.lanes, 4);
+    int SLp = first_lanes(g, c), SLs = 1, SLr = std::min(g.lanes, 4);
     if (MULTI) {
         const int cap = c.sub_lanes > 0 ? std::min(c.sub_lanes, 32) : 32;
         int need = 1;
@@ -1892,12 +1895,13 @@ cudaError_t launch_wave_as(const Phys& phys, const WfLaunchCfg& c) {
     if (per_sm < 1) per_sm = 1;
     int blocks = c.walk_blocks > 0 ? c.walk_blocks : c.num_sms * per_sm;
     const int wpb = threads / 32;
-    const int64_t items = g.n_short_chunks * wf_items_per_chunk(g.G, g.M, SLs) +
-                          (g.n_chunks - g.n_short_chunks) * wf_items_per_chunk(g.G, g.M, SLr);
-    const int64_t need = std::max<int64_t>((items + wpb - 1) / wpb, 1);
-    if (blocks > need) blocks = (int)need;
     const int64_t resident = (int64_t)std::min(blocks, c.num_sms * per_sm) * wpb;
     const int64_t p_chunks = first_chunks(g, SLp, resident);
+    const int64_t rest = g.n_chunks - p_chunks, shorts = std::min(g.n_short_chunks, rest);
+    const int64_t items = p_chunks * wf_items_per_chunk(1, g.M, SLp) + shorts * wf_items_per_chunk(g.G, g.M, SLs) +
+                          (rest - shorts) * wf_items_per_chunk(g.G, g.M, SLr);
+    const int64_t need = std::max<int64_t>((items + wpb - 1) / wpb, 1);
+    if (blocks > need) blocks = (int)need;
     // Two short chunks a ticket where there are many more items than warps. Longer batches put a chunk's
     // last chain behind those before it, and the chains that wait for it behind that. Hourly steps of a
     // 1024 x 1024 domain: 8.7 ms with two and eight chains to a warp (SLr), 9.4 with eight and one.
