@@ -29,7 +29,7 @@ namespace wfr {
 
 // Wflow.scurve (utils.jl:27-30)
 __device__ __forceinline__ double scurve(double x, double a, double b, double c) {
-    return 1.0 / (b + wfm::exp(-c * (x - a)));
+    return wfm::div_(1.0, b + wfm::exp(-c * (x - a)));
 }
 
 // Tables of reservoir r: meta[4 r .. 4 r + 3] = start of the S-H table in F.res_tab (levels, then
@@ -59,26 +59,29 @@ __device__ __forceinline__ double level_after(const WfDevFields& F, int32_t r, d
         const double* h = F.res_tab + mt[0];
         return interpolate_linear(storage, h + mt[1], h, 1, mt[1]);
     }
-    return wl0 + (storage - s0) / area;
+    return wl0 + wfm::div_(storage - s0, area);
 }
 
 // Net inflow, storage update and outflow of reservoir r for member m over a sub-step dt, with q
 // the river discharge of the reservoir's cell after its kinematic-wave update. Accumulates the
-// step's inflow, outflow, evaporation and abstraction; returns the outflow.
+// step's inflow, outflow, evaporation and abstraction; returns the outflow. On a river's main chain some
+// lane is at a reservoir in most steps of the wavefront, so the divisions and comparisons are the short
+// ones of wf_math.cuh (daily river sweep of 160 x 160 cells with reservoirs: 8.9 -> 8.7 ms).
 __device__ inline double reservoir_node(const WfDevFields& F, int32_t r, int m, double q, double dt) {
     using wfm::jmax;
     using wfm::jmin;
     const int64_t e = (int64_t)r * F.M + m;
     double* const* RS = F.RS;
     double* const* RP = F.RP;
-    const double area = RP[RP_AREA][r];
+    const double area = RP[RP_AREA][r], rdt = wfm::div_(1.0, dt);
+    auto per_dt = [&](double x) { return wfm::div_by_(x, dt, rdt); };
     const double s0 = RS[RS_STORAGE][e];
     const double wl0 = RS[RS_WATERLEVEL][e];
     // negative external inflow: abstraction limited to 98 % of the storage (surface_kinwave.jl:461-469)
     const double ext = RS[RS_EXT][e];
     double inflow;
-    if (ext < 0.0) {
-        const double abstraction = jmin(-ext, (s0 / dt) * 0.98);
+    if (wfm::lt_(ext, 0.0)) {
+        const double abstraction = jmin(-ext, per_dt(s0) * 0.98);
         RS[RS_ABS_CUM][e] += abstraction * dt;
         inflow = -abstraction;
     } else {
@@ -89,27 +92,27 @@ __device__ inline double reservoir_node(const WfDevFields& F, int32_t r, int m, 
     const double precipitation = RS[RS_PRECIP][e] * area;
     const double available = s0 + (net + precipitation) * dt;
     const double potential_evaporation = RS[RS_EVAP][e] * area;
-    const double evaporation = jmin(available / dt, potential_evaporation);
+    const double evaporation = jmin(per_dt(available), potential_evaporation);
     const double obs = RS[RS_OBS][e];
     const double smax = RP[RP_MAXSTOR][r];
     double outflow, storage;
-    if (obs == obs) {  // observed outflow (reservoir.jl:554-575)
-        const double input = jmax(s0 / dt + precipitation - evaporation + net, 0.0);
+    if (!wfm::isnan_(obs)) {  // observed outflow (reservoir.jl:554-575)
+        const double input = jmax(per_dt(s0) + precipitation - evaporation + net, 0.0);
         outflow = jmin(obs, input);
         storage = (input - outflow) * dt;
-        if (smax == smax) {
-            const double overflow = jmax(0.0, (storage - smax) / dt);
+        if (!wfm::isnan_(smax)) {
+            const double overflow = jmax(0.0, per_dt(storage - smax));
             storage -= overflow * dt;
             outflow += overflow;
         }
     } else if (F.res_type[r] == WF_RES_RATING_CURVE) {
-        const double input = s0 / dt + precipitation - evaporation + net;
+        const double input = per_dt(s0) + precipitation - evaporation + net;
         const int64_t* mt = F.res_tab_meta + 4 * (int64_t)r;
         const double* h = F.res_tab + mt[2];
         outflow = interpolate_linear(wl0, h, h + mt[3] + (*F.res_hq_day - 1), 365, mt[3]);
         outflow = jmin(outflow, input);
         storage = (input - outflow) * dt;
-        const double overflow = jmax(0.0, (storage - smax) / dt);
+        const double overflow = jmax(0.0, per_dt(storage - smax));
         storage = jmin(storage, smax);
         outflow += overflow;
     } else if (F.res_type[r] == WF_RES_FREE_WEIR) {
@@ -117,19 +120,19 @@ __device__ inline double reservoir_node(const WfDevFields& F, int32_t r, int m, 
         const int64_t elo = (int64_t)lo * F.M + m;
         const double wl_lo = lo >= 0 ? RS[RS_WATERLEVEL][elo] : 0.0;
         const double diff_wl = lo >= 0 ? wl0 - wl_lo : 0.0;
-        const double input = jmax(s0 / dt + precipitation - evaporation + net, 0.0);
+        const double input = jmax(per_dt(s0) + precipitation - evaporation + net, 0.0);
         const double thr = RP[RP_THRESHOLD][r];
         outflow = 0.0;
         if (diff_wl >= 0.0) {
             if (wl0 > thr) {
                 const double dh = wl0 - thr;
                 outflow = RP[RP_RC_COEF][r] * wfm::pow(dh, RP[RP_RC_EXP][r]);
-                outflow = jmin(outflow, dh * area / dt);
+                outflow = jmin(outflow, per_dt(dh * area));
             }
         } else if (wl_lo > thr) {  // the lower reservoir's level is the higher: flow back
             const double dh = wl_lo - thr;
             outflow = -RP[RP_RC_COEF][r] * wfm::pow(dh, RP[RP_RC_EXP][r]);
-            outflow = jmax(outflow, -(dh * RP[RP_AREA][lo] / dt));
+            outflow = jmax(outflow, -per_dt(dh * RP[RP_AREA][lo]));
         }
         storage = (input - outflow) * dt;
         if (diff_wl < 0.0) {
@@ -141,23 +144,23 @@ __device__ inline double reservoir_node(const WfDevFields& F, int32_t r, int m, 
             RS[RS_STORAGE][elo] = s_lo_new;
         }
     } else if (F.res_type[r] == WF_RES_MODIFIED_PULS) {
-        const double res_factor = area / (dt * wfm::sqrt_(RP[RP_RC_COEF][r]));
-        const double si = s0 / dt + precipitation - evaporation + net;
-        const double si_adj = si - area * RP[RP_THRESHOLD][r] / dt;
+        const double res_factor = wfm::div_(area, dt * wfm::sqrt_(RP[RP_RC_COEF][r]));
+        const double si = per_dt(s0) + precipitation - evaporation + net;
+        const double si_adj = si - per_dt(area * RP[RP_THRESHOLD][r]);
         outflow = 0.0;
-        if (si_adj > 0.0) {
+        if (wfm::gt0_(si_adj)) {
             const double t = -res_factor + wfm::sqrt_((res_factor * res_factor + 4.0 * si_adj));
-            outflow = t > 0.0 ? 0.25 * t * t : 0.0;
+            outflow = wfm::gt0_(t) ? 0.25 * t * t : 0.0;
         }
         outflow = jmin(outflow, si);
         storage = (si - outflow) * dt;
     } else {  // simple reservoir
         storage = jmax(s0 + (net + precipitation - evaporation) * dt, 0.0);
-        const double fac = scurve(storage / smax, RP[RP_TMIN][r], 1.0, 30.0);
-        const double demand_release = jmin(fac * RP[RP_DEMAND][r], storage / dt);
+        const double fac = scurve(wfm::div_(storage, smax), RP[RP_TMIN][r], 1.0, 30.0);
+        const double demand_release = jmin(fac * RP[RP_DEMAND][r], per_dt(storage));
         storage -= demand_release * dt;
-        const double wanted = jmax(0.0, (storage - smax * RP[RP_TFULL][r]) / dt);
-        const double overflow_q = jmax(0.0, (storage - smax) / dt);
+        const double wanted = jmax(0.0, per_dt(storage - smax * RP[RP_TFULL][r]));
+        const double overflow_q = jmax(0.0, per_dt(storage - smax));
         const double realized = jmin(wanted, overflow_q + RP[RP_MAXREL][r] - demand_release);
         storage -= realized * dt;
         outflow = realized + demand_release;
@@ -170,7 +173,7 @@ __device__ inline double reservoir_node(const WfDevFields& F, int32_t r, int m, 
     // what went to the downstream river cell: the reservoir's own outflows only (RS_OUT_CUM of a
     // linked lower reservoir also counts the water its upper reservoir drew back)
     RS[RS_DOWN_CUM][e] += outflow * dt;
-    RS[RS_EVAP_CUM][e] += evaporation / area * dt;
+    RS[RS_EVAP_CUM][e] += wfm::div_(evaporation, area) * dt;
     return outflow;
 }
 
