@@ -1661,12 +1661,13 @@ struct OlWave {
             acc = wff::mul(q, r.w_hv);
             if (riv) t = wff::mul(q, x.fr_hv);
         }
-        if (!wfv::await_two(g, sw, r.lt0, r.lt1, m, s, w0, w1, F.status)) return false;
+        if (!wfv::await_one(g, sw, r.lt0, m, s, w0, F.status)) return false;
         if (r.lt0 >= 0) {
             const wff::ff q = wff::unpack(w0);
             acc = wff::add(acc, wff::mul(q, r.w_lt0));
             if (riv) t = wff::add(t, wff::mul(q, x.fr0));
         }
+        if (!wfv::await_one(g, sw, r.lt1, m, s, w1, F.status)) return false;
         if (r.lt1 >= 0) {
             const wff::ff q = wff::unpack(w1);
             acc = wff::add(acc, wff::mul(q, r.w_lt1));
