@@ -1298,7 +1298,8 @@ __global__ void __launch_bounds__(128) wave64_kernel(Phys phys, int64_t p_chunks
 // the reference's sweep hands them on); it passes min(material / dt, capacity) on to its
 // downstream cell and keeps the rest. MAT 0: snow storage (snow_out = its flux), MAT 1: snow
 // water (snow_out += its flux). FP64 in both forms (the split form's double-FP32 states are
-// converted on the way in and out).
+// converted on the way in and out). A chain position is bound by its loads in a row: the upstream list
+// in the transport's order (snow_up: its chains), then the words of up to four children together.
 template <int MAT>
 struct SnowPhys {
     WfDevFields F;
@@ -1309,14 +1310,19 @@ struct SnowPhys {
                          double& hq) {
         const int f = MAT == 0 ? SNOW : SNOW_WATER;
         double material = F.split ? (double)F.Mh[f][e] + (double)F.Ml[f][e] : F.Mf[f][e];
-        const int32_t o0 = g.up_ptr[slot], o1 = g.up_ptr[slot + 1];
-        for (int32_t k = o0; k < o1; ++k) {
-            double upd;
-            if (!wfw::upstream_q(g, sw, hq, g.snow_up[k], m, s, ep, F.status, upd)) return false;
-            material += upd;
+        const double cap = F.GM[MAT == 0 ? GM_CAP : GM_CAPW][e];
+        const double before = MAT == 0 ? 0.0 : F.GM[GM_SNOW_OUT][e];
+        const int32_t o0 = __ldg(g.up_ptr + slot), o1 = __ldg(g.up_ptr + slot + 1);
+        int skip = 0;
+        for (int32_t o = o0; o < o1; o += wfv::GROUP) {
+            wfv::UpGroup u;
+            if (!wfv::gather_group(g, sw, g.snow_up, o, o1, skip, m, s, F.status, u)) return false;
+#pragma unroll
+            for (int i = 0; i < wfv::GROUP; ++i)
+                if (u.chain[i] >= -1) material += u.chain[i] < 0 ? hq : wfm::from_bits(u.word[i]);
         }
         const double dt = sw.dt;
-        const double flux = jmin(material / dt, F.GM[MAT == 0 ? GM_CAP : GM_CAPW][e]);
+        const double flux = jmin(div_(material, dt), cap);
         const double update = flux * dt;
         material -= update;
         if (F.split) {
@@ -1326,9 +1332,9 @@ struct SnowPhys {
         } else {
             F.Mf[f][e] = material;
         }
-        F.GM[GM_SNOW_OUT][e] = MAT == 0 ? flux : F.GM[GM_SNOW_OUT][e] + flux;
+        F.GM[GM_SNOW_OUT][e] = MAT == 0 ? flux : before + flux;
         hq = update;
-        if (is_end) wfw::publish(g, chain, m, s, ep, update);
+        if (is_end) wfz::publish(g, chain, m, s, update);
         return true;
     }
 };

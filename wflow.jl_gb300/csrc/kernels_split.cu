@@ -1678,7 +1678,7 @@ struct OlWave {
             const int32_t o1 = __ldg(g.up_ptr + slot + 1);
             for (int32_t o = __ldg(g.up_ptr + slot); o < o1; o += wfv::GROUP) {
                 wfv::UpGroup u;
-                if (!wfv::gather_group(g, sw, o, o1, skip, m, s, F.status, u)) return false;
+                if (!wfv::gather_group(g, sw, g.up_chain, o, o1, skip, m, s, F.status, u)) return false;
 #pragma unroll
                 for (int i = 0; i < wfv::GROUP; ++i) {
                     if (u.chain[i] < 0) continue;

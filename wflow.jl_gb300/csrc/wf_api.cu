@@ -47,7 +47,7 @@ struct DevGraphAlloc {
     double* end_q = nullptr;
     unsigned long long* ticket = nullptr;
     int32_t s_cap = 1;
-    int32_t* snow_up = nullptr;  // land graph with snow transport: up entries in topological-sort order
+    int32_t* snow_up = nullptr;  // land graph with snow transport: up_chain in topological-sort order
 };
 
 }  // namespace
@@ -1248,7 +1248,7 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         }
     }
     if (F.snow_transport) {
-        // each slot's upstream entries in the order of the land graph's topological sort
+        // the chains of each slot's upstream entries in the order of the land graph's topological sort
         const std::vector<int64_t> order = topo_order_dfs(n, d->land_downstream);
         if ((int64_t)order.size() != n) {
             set_err(h, WF_ERR_CYCLE, "the land drainage graph has a cycle (routing/utils.jl:26-31)");
@@ -1263,6 +1263,7 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
             std::sort(su.begin() + o0, su.begin() + o1, [&](int32_t a, int32_t b) {
                 return pos[PL.node_of_slot[PL.up_slot[a]]] < pos[PL.node_of_slot[PL.up_slot[b]]];
             });
+            for (int32_t o = o0; o < o1; ++o) su[o] = PL.up_chain[su[o]];
         }
         CKR(upload(h, &h->land.snow_up, su));
     }
@@ -2101,7 +2102,8 @@ int enqueue_vertical(WfHandle* h, const WfLaunchCfg& lc, const WfDevGraph& gl, i
         sw.dts = h->dts_ssf;
         sw.wait_ns = h->wait_ns;
         sw.wait_offset = h->wait_offset;
-        CK(cudaMemsetAsync(gl.flags, 0, (size_t)h->land.plan.n_chains * h->M * sizeof(uint32_t), h->stream));
+        CK(cudaMemsetAsync(gl.end_q, 0xFF, (size_t)h->land.plan.n_chains * h->M * h->land.s_cap * sizeof(double),
+                           h->stream));
         CK(cudaMemsetAsync(gl.ticket, 0, sizeof(unsigned long long), h->stream));
         CK(wf_snow_transport_sweep(h->F, gl, sw, material, lc));
         ++nl;

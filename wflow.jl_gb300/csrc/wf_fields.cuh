@@ -236,7 +236,7 @@ struct WfDevGraph {
     unsigned long long* ticket;  // work counter of the current launch
     int32_t s_cap;        // sub-steps per launch
     // land graph with snow transport: for each slot's upstream entries up_ptr[slot] ..
-    // up_ptr[slot + 1], the entry indices in the order of the graph's topological sort (the
+    // up_ptr[slot + 1], their chains (up_chain) in the order of the graph's topological sort (the
     // order in which the transport hands material on)
     const int32_t* snow_up;
 };

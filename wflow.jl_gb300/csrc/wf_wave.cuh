@@ -121,11 +121,11 @@ struct UpGroup {
     int32_t chain[GROUP];  // -1: the heavy child, -2: no entry
     unsigned long long word[GROUP];
 };
-// Entries from o on (o1: end of the list) at sub-step s; the first `skip` light children are left out.
-__device__ __forceinline__ bool gather_group(const WfDevGraph& g, const WfSweep& sw, int32_t o, int32_t o1, int& skip,
-                                             int m, int s, int32_t* status, UpGroup& u) {
+// Entries from o on (o1: end of the list) of `chains` at sub-step s; the first `skip` light children are left out.
+__device__ __forceinline__ bool gather_group(const WfDevGraph& g, const WfSweep& sw, const int32_t* chains, int32_t o,
+                                             int32_t o1, int& skip, int m, int s, int32_t* status, UpGroup& u) {
 #pragma unroll
-    for (int i = 0; i < GROUP; ++i) u.chain[i] = o + i < o1 ? __ldg(g.up_chain + o + i) : -2;
+    for (int i = 0; i < GROUP; ++i) u.chain[i] = o + i < o1 ? __ldg(chains + o + i) : -2;
 #pragma unroll
     for (int i = 0; i < GROUP; ++i) {
         if (u.chain[i] >= 0 && --skip >= 0) u.chain[i] = -2;
@@ -189,7 +189,7 @@ __device__ __forceinline__ bool gather_w(const WfDevGraph& g, const WfSweep& sw,
         const int32_t o1 = __ldg(g.up_ptr + slot + 1);
         for (int32_t o = __ldg(g.up_ptr + slot); o < o1; o += GROUP) {
             UpGroup u;
-            if (!gather_group(g, sw, o, o1, skip, m, s, status, u)) return false;
+            if (!gather_group(g, sw, g.up_chain, o, o1, skip, m, s, status, u)) return false;
 #pragma unroll
             for (int i = 0; i < GROUP; ++i) {
                 if (u.chain[i] < 0) continue;

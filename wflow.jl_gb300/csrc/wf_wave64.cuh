@@ -102,7 +102,7 @@ __device__ __forceinline__ bool gather(const WfDevGraph& g, const WfSweep& sw, c
                         if (TR) fr[i] = __ldg(g.up_fr + o + i);
                     }
             wfv::UpGroup u;
-            if (!wfv::gather_group(g, sw, o, o1, skip, m, s, status, u)) return false;
+            if (!wfv::gather_group(g, sw, g.up_chain, o, o1, skip, m, s, status, u)) return false;
 #pragma unroll
             for (int i = 0; i < wfv::GROUP; ++i) {
                 if (u.chain[i] < -1) continue;
