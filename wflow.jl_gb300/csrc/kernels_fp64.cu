@@ -1643,9 +1643,11 @@ cudaError_t launch_wave64(const Phys& phys, const WfLaunchCfg& c) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wave64_kernel<Phys, MULTI>, threads, smem);
     if (err != cudaSuccess) return err;
     if (per_sm < 1) per_sm = 1;
-    // one or two warps per scheduler: a scheduler issues one FP64 instruction per 64 cycles, which one warp
-    // keeps busy, and more warps only slow the long chains down
-    const int fill = std::min(per_sm, 2);
+    // One or two warps per scheduler: a scheduler issues one FP64 instruction per 64 cycles, which one warp
+    // keeps busy, and more warps only slow the long chains down. River flow, whose positions are almost all
+    // arithmetic: one (hourly, 301 x 301 cells: 5.25 ms with two, 4.72 with one; 700 x 700: 13.7 and 12.6);
+    // the land sweeps, which wait more: two (daily overland flow of 200 x 200 cells: 3.22 and 3.50).
+    const int fill = std::min(per_sm, Phys::kLand ? 2 : 1);
     int blocks = c.walk_blocks > 0 ? c.walk_blocks : c.num_sms * fill;
     const int wpb = threads / 32;
     const int64_t resident = (int64_t)std::min(blocks, c.num_sms * per_sm) * wpb;
