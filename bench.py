@@ -407,20 +407,6 @@ def run_gpu(args):
                           "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback"}
     phases = {k: {"ms": kt[k], "achieved_gbs": achieved_of(k), "frac": achieved_of(k) / peak,
                   "algorithmic_bytes": phase_bytes(k)} for k in kt}
-    # the split form's overland sweep and the river's first sub-steps share one launch (timed as
-    # the overland phase; the river phase is then its completion kernel alone): one phase for both
-    shared_launch = (form == abi.WF_FORM_SPLIT and not cfg.adaptive_timestep and dom.n_river > 0
-                     and (tuning or {}).get("separate_overland_river", 0) == 0 and substeps["land"] <= 16)
-    if shared_launch:
-        b = phase_bytes("overland") + phase_bytes("river")
-        ms = kt["overland"] + kt["river"]
-        a = b / (ms / 1e3) / 1e9 if ms > 0 else 0.0
-        phases.pop("overland")
-        phases.pop("river")
-        phases["overland+river"] = {"ms": ms, "achieved_gbs": a, "frac": a / peak, "algorithmic_bytes": b,
-                                    "note": "overland sweep and the river sweep in one launch"}
-        result["kernel_ms_note"] = ("overland: the shared overland-river launch and the overland completion; "
-                                    "river: the river completion")
     result["roofline_phases"] = phases
     # ---- the FP64 plain form on the same workload and forcing: throughput ratio and the split
     # form's error against it (the FP64 form reproduces the FP64 oracle bit for bit)

@@ -324,12 +324,11 @@ typedef struct WfTuning {
     int32_t routing_blocks_per_sm;
     int32_t use_graph;        /* capture the step in a CUDA graph (1 = yes, default) */
     int32_t reserved[8];      /* [0] wait budget (us), [1] test hook (0), [2] per-kernel timing,
-                               * [3] cap of the routing sweeps' sub-step lanes (0 = default 8),
-                               * [4] bit k set: node-major sweep k (0 subsurface, 1 overland,
-                               * 2 river) holds its inputs in registers instead of staging them
-                               * in shared memory (0 = all staged); [5] blocks per SM of the
-                               * split vertical kernel's grid-stride loop, which sets the elements
-                               * each thread walks (0 = 16); [6..7] 0 */
+                               * [3] the routing sweeps' sub-step lanes (0 = by the packing rules,
+                               * at most 32), [4] 0..7 and [6] 0..1: accepted, without effect (one
+                               * way of staging inputs, one launch per sweep); [5] blocks per SM of
+                               * the split vertical kernel's grid-stride loop, which sets the
+                               * elements each thread walks (0 = 16); [7] 0 */
 } WfTuning;
 
 /* Library version / ABI check. */

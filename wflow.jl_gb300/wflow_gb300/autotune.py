@@ -65,7 +65,7 @@ def tune(model: Model, forcing, steps=1, verbose=False):
     best_lanes = 0
     if m["steps"] > 0 and max(m["substeps_land"], m["substeps_river"]) > m["steps"]:
         best_lanes_t = best_route_t
-        for lanes in [1, 2, 4, 16]:  # 0 (the default, 8) was measured above
+        for lanes in [1, 2, 4, 16]:  # 0 (the packing rules) was measured above
             model._tune_state = dict(vertical_block=0, routing_warps=best_route[0],
                                      routing_blocks_per_sm=best_route[1], substep_lanes=lanes,
                                      separate_overland_river=1)
@@ -76,8 +76,9 @@ def tune(model: Model, forcing, steps=1, verbose=False):
                 print(f"sub-step lanes={lanes}: {route:.3f} ms")
             if route < best_lanes_t:
                 best_lanes, best_lanes_t = lanes, route
-    # inputs of the node-major sweeps: staged in shared memory or held in registers, per sweep
-    # (both runs time every sweep; each keeps its faster mode)
+    # the two switches below select nothing in the current library (set_tuning); a library that has
+    # such variants is tuned by them as before. Inputs of the sweeps: staged in shared memory or held
+    # in registers, per sweep (both runs time every sweep; each keeps its faster mode)
     base = dict(vertical_block=0, routing_warps=best_route[0], routing_blocks_per_sm=best_route[1],
                 substep_lanes=best_lanes, separate_overland_river=1)
     model._tune_state = dict(base, sweep_inputs=0)

@@ -174,8 +174,10 @@ class Model:
                    wait_budget_us=0, wait_offset=0, kernel_timing=0, substep_lanes=0, sweep_inputs=0,
                    vertical_blocks_per_sm=0, separate_overland_river=0):
         """Launch shape of the step's kernels (results do not depend on it): threads per block of
-        the per-cell kernels, warps per block and blocks per SM of the routing sweeps, the cap of
-        the sub-step lanes of their diagonal schedule (0: default), the CUDA graph, and test hooks."""
+        the per-cell kernels, warps per block and blocks per SM of the routing sweeps, the
+        sub-step lanes of their diagonal schedule (0: by the packing rules), the CUDA graph, and test
+        hooks. sweep_inputs and separate_overland_river are accepted and without effect: the sweeps
+        stage their inputs one way and run in launches of their own."""
         t = abi.WfTuning()
         t.vertical_block, t.routing_warps, t.routing_blocks_per_sm, t.use_graph = (
             vertical_block, routing_warps, routing_blocks_per_sm, use_graph)
@@ -183,9 +185,9 @@ class Model:
         t.reserved[1] = wait_offset
         t.reserved[2] = kernel_timing
         t.reserved[3] = substep_lanes
-        t.reserved[4] = sweep_inputs  # bit k: sweep k (subsurface, overland, river) keeps its inputs in registers
+        t.reserved[4] = sweep_inputs  # without effect
         t.reserved[5] = vertical_blocks_per_sm  # grid of the split vertical kernel (elements per thread)
-        t.reserved[6] = separate_overland_river  # 1: split overland and river sweeps in separate launches
+        t.reserved[6] = separate_overland_river  # without effect
         self._check(self.lib.wf_set_tuning(self.h, C.byref(t)), "wf_set_tuning")
 
     def stream(self):
