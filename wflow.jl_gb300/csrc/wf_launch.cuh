@@ -13,10 +13,11 @@
 //
 // The grid is every block that fits on the device at once (occupancy), capped by the work.
 // The longest chains (the plan's trailing long chunks) carry the critical path, so up to half
-// of the resident warps take them first; the remaining warps take the other chunks in chain
-// length order. Progress is guaranteed: a chunk only waits for shorter chains; shorter chains
-// are either long chunks already resident or ordinary chunks, which at least half of the
-// resident warps keep dispatching in dependency order.
+// of the resident warps take them first; the remaining warps take the other chunks in the plan's
+// order. Progress is guaranteed: a chunk only waits for chains before it in that order, which are
+// either long chunks already resident or ordinary chunks, which at least half of the resident
+// warps keep dispatching in dependency order; and the chains of a chunk, which may share a warp,
+// end before another one of the chunk needs their discharge (wf_plan.cpp).
 template <class Kernel>
 cudaError_t wave_grid(Kernel kernel, int threads, size_t smem, const WfLaunchCfg& c, const WfDevGraph& g, int& blocks,
                       int64_t& prio_items, int64_t items_per_chunk = 0) {

@@ -113,8 +113,7 @@ int wf_build_plan(int64_t n, const int32_t* ds, int32_t members, WfRoutingPlan& 
     // Dispatch order. The sweeps first dispatch, all at once, the chains at the end of the order
     // (one chain per chunk; wave_grid caps them at half the resident warps), then the others in
     // key order (the length, without heavy-child hints), which is a dependency order (a light
-    // child is strictly shorter than its consumer, and its end strictly lower), short chains
-    // batched. The first group holds up to kFirst chains: the longest
+    // child's end is strictly lower than its consumer's), short chains batched. The first group holds up to kFirst chains: the longest
     // ones (at least max(64, longest / 8) nodes), which carry the critical path, and then the
     // most urgent of the rest: with one time unit per position, a chain ending at position k of
     // its consumer must start by LS(c) = LS(consumer) + k - len(c) (a chain ending at a pit by
@@ -159,6 +158,21 @@ int wf_build_plan(int64_t n, const int32_t* ds, int32_t members, WfRoutingPlan& 
                 first[by_ls[i]] = 1;
                 ++n_solo;
             }
+        // The lanes of a warp advance together, one position a step, so the chains of a chunk must
+        // end before a chain of the chunk needs them: length(light child) <= position of the join.
+        // That holds by itself where every heavy child is the highest; with hints a chain may be
+        // joined earlier than that, and such a chain gets a chunk of its own.
+        if (heavy_hint) {
+            for (int64_t u = 0; u < n; ++u) {
+                const int64_t v = ds[u];
+                if (v < 0 || heavy[v] == u) continue;
+                const int64_t c = chain_of[v];
+                if (chains[chain_of[u]].len > pos_of[v] && !first[c]) {
+                    first[c] = 1;
+                    ++n_solo;
+                }
+            }
+        }
         // the first group's consumers: the urgent prefix is closed under consumers, the long
         // chains too (a consumer is longer); add any consumer missed at the budget's edge
         for (bool grew = true; grew;) {
@@ -258,7 +272,8 @@ int wf_build_plan(int64_t n, const int32_t* ds, int32_t members, WfRoutingPlan& 
 bool wf_check_plan(const WfRoutingPlan& P, const int32_t* ds, std::string& err) {
     // chain lengths sorted before the first-dispatched group (padding chains have length 0;
     // with heavy-child hints the order is by end height, checked through the per-node condition
-    // below); every chain waits only for chains of smaller index (checked per node below)
+    // below); every chain waits only for chains of smaller index, and for one of its own chunk only
+    // at a position that the other's length does not exceed (checked per node below)
     int32_t prev = 0;
     for (int64_t c = 0; c < P.n_chains - P.n_long_chunks && !P.hinted; ++c) {
         if (P.chain_len[c] == 0) continue;
@@ -290,7 +305,9 @@ bool wf_check_plan(const WfRoutingPlan& P, const int32_t* ds, std::string& err) 
                 }
             } else {
                 int64_t uc = P.up_chain[o];
-                if (!P.is_chain_end[us] || uc >= my_chain || (!P.hinted && P.chain_len[uc] > k)) {
+                const bool same_chunk = us >= P.chunk_base[chunk] && us < P.chunk_base[chunk + 1];
+                if (!P.is_chain_end[us] || uc >= my_chain ||
+                    ((!P.hinted || same_chunk) && P.chain_len[uc] > k)) {
                     err = "light child chain does not precede its consumer";
                     return false;
                 }

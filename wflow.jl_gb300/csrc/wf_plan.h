@@ -8,7 +8,10 @@
 // lane with the heavy inflow carried in registers, and the other (light) upstream children are
 // ends of strictly shorter chains. A node at position k of its chain has height k, so chains
 // sorted by length form a valid dependency order: a lane only ever waits for chains dispatched
-// before its own, which guarantees forward progress of the persistent kernels.
+// before its own, which guarantees forward progress of the persistent kernels. With heavy-child
+// hints the order is by the height of the chains' ends; a chain that another chain of its chunk
+// would join before that one has ended gets a chunk of its own, because the chains of a chunk may
+// share a warp, whose lanes advance together.
 //
 // A first group of chains is placed at the end, one chain per chunk: the longest chains (which
 // carry the critical path) and the most urgent tributaries (smallest latest start;
@@ -56,5 +59,6 @@ int wf_build_plan(int64_t n, const int32_t* downstream, int32_t members, WfRouti
                   const int64_t* heavy_hint = nullptr);
 
 // Host check of the schedule invariants (tests): every light upstream chain precedes the
-// chain that consumes it, and positions equal heights.
+// chain that consumes it, and one of the same chunk is no longer than the position it joins at
+// (without hints: every one).
 bool wf_check_plan(const WfRoutingPlan& plan, const int32_t* downstream, std::string& err);

@@ -2,10 +2,10 @@
 //
 // Work items are (chunk, group of chain-member pairs) in dependency order, taken from a global
 // ticket counter: a bounded number of the longest chains first (see wave_grid in wf_launch.cuh
-// for why that keeps progress guaranteed), then the others in chain-length order, so an ordinary
-// item only waits for chain ends of items dispatched earlier. A node at chain position k depends
-// on its heavy child (position k - 1 of the same chain) and on light children (ends of shorter
-// chains). Its sub-step s depends on (k - 1, s) and (k, s - 1) only, so a launch of S sub-steps
+// for why that keeps progress guaranteed), then the others in the plan's order, so an ordinary
+// item only waits for chain ends of items dispatched earlier or its own. A node at chain position k
+// depends on its heavy child (position k - 1 of the same chain) and on light children (ends of
+// chains before it in the order). Its sub-step s depends on (k - 1, s) and (k, s - 1) only, so a launch of S sub-steps
 // runs on a diagonal schedule: SL lanes per chain-member pair (a power of two), lane l takes
 // sub-step r * SL + l of round r, and at time t works on position t - l. A chain of length L takes
 // ceil(S / SL) * (L + SL - 1) time steps instead of L * S. Lane l reads the node state that lane

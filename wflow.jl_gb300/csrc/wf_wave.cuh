@@ -217,8 +217,9 @@ __device__ __forceinline__ void load_words(const WfDevGraph& g, int m, int32_t l
 // short tributary chains, and a ticket per chain would pay the ticket, the descriptor loads and the
 // prefetch start-up per chain), or a single longer item. The items of a batch are walked as one
 // sequence of positions, so the prefetch runs on across item boundaries. Order and progress are
-// unchanged: a batch holds consecutive items and a chain waits only for strictly shorter chains,
-// which come earlier in the batch or in the order.
+// unchanged: a batch holds consecutive items and a chain waits only for chains that come earlier in
+// the order, or for chains of its own chunk that end before it needs them (wf_plan.cpp: the lanes
+// of a warp advance together).
 //
 // SL lanes (a power of two) serve a chain-member pair, of which the first SU = min(SL, S) work. Sub-step
 // s of the node at chain position k depends only on (k - 1, s), its heavy child, and (k, s - 1), its own
