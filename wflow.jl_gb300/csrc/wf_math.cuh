@@ -201,24 +201,34 @@ WF_HD double jclamp(double x, double lo, double hi) { return gt_(x, hi) ? hi : (
 // A quotient q = a r from a reciprocal r of b, corrected once by its exact remainder, is the
 // correctly rounded a / b (Markstein, IBM J. Res. Dev. 34 (1990); Cornea, Harrison & Tang,
 // Scientific Computing on Itanium-based Systems (2002), ch. 8) as long as nothing over- or
-// underflows on the way, which quot_in_range checks on the exponents; the other cases take the
-// compiler's division. That holds with the correctly rounded r; rcp_raw's is only within an ulp of it,
-// which decides wrongly where a / b lies within 2^-105 of a rounding boundary: a and b a few ulps
-// below powers of two (1 / (1 - 2^-53), root fractions summing to just below 1), so such divisors
-// (below_power) take the compiler's division as well. With the reciprocal of a divisor that is used several times (a step size, a
-// cell length) at hand the quotient costs 3 FP64 instructions, else 6 (563 cycles -> 192 / 403).
+// underflows on the way, which quot_in_range checks on the exponents (the other cases take the
+// compiler's division), and r is close enough to 1 / b. How close: with m_b the mantissa of b, a / b
+// is at least 2^-53 / m_b ulps away from the middle of two values. Near a middle q is half an ulp
+// from a / b, and the corrected quotient is off by half the relative error of r. A correctly rounded
+// r, off by at most 2^-54 m_b, therefore always will do. rcp_raw's error is larger by the cube of its
+// seed's, which is below 2^-22: at most 2^-53 (m_b / 2 + 2^-13). With that the condition holds, and q is
+// next to a / b, for m_b below 2 - 2^-12; divisors closer below a power of two (below_power) take the
+// compiler's division. (A seed of 2^-20, as rcp.approx.ftz.f64 gives it, does not do: of the quotients
+// 2^-53 ulps from a middle 1 in 48,000 came out wrong, with m_b above 1.99.)
+// With the reciprocal of a divisor that is used several times (a step size, a cell length) at hand
+// the quotient costs 3 FP64 instructions, else 6 (563 cycles -> 192 / 403).
 #ifdef __CUDACC__
 __device__ __forceinline__ bool quot_in_range(double a, double b) {
     const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
     return ((unsigned)(ea - 160) <= 1700u || to_bits(a) == 0) && (unsigned)(eb - 160) <= 1700u &&
            ((unsigned)(ea - eb + 800) <= 1600u || to_bits(a) == 0);
 }
+// 1 / b to within 2^-22, b in range: the FP32 reciprocal (2^-23) of the leading 24 bits of b's mantissa,
+// its exponent set on the integer pipe
 __device__ __forceinline__ double rcp_seed(double b) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    return r;
+    const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
+    const float m = __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | 0x3f800000u);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));
+    const unsigned rb = __float_as_uint(r);
+    return __hiloint2double((int)((rb >> 3) + 0x77f00000u - (hi & 0xfff00000u)), (int)(rb << 29));
 }
-// 1 / b to within an ulp, b in range: the seed's relative error e is taken to e^3
+// 1 / b to within 0.501 ulps, b in range: the seed's relative error e is taken to e^3
 __device__ __forceinline__ double rcp_raw(double b) {
     const double r = rcp_seed(b);
     const double e = __fma_rn(-b, r, 1.0);
@@ -228,8 +238,12 @@ __device__ __forceinline__ double quot_raw(double a, double b, double rb) {
     const double q = a * rb;
     return __fma_rn(__fma_rn(-b, q, a), rb, q);
 }
-// mantissa within 16 ulps of all ones
-__device__ __forceinline__ bool below_power(double b) { return (to_bits(b) & 0x000fffffffffffffULL) >= 0x000ffffffffffff0ULL; }
+// mantissa at least 2 - 2^-11
+__device__ __forceinline__ bool below_power(double b) { return (__double2hiint(b) & 0xfffff) >= 0xffe00; }
+// The reciprocal of b to keep for div_by_, 0 where the quotient has to take the compiler's division
+__device__ __forceinline__ double rcp_kept(double b) {
+    return quot_in_range(1.0, b) && !below_power(b) ? rcp_raw(b) : 0.0;
+}
 #endif
 // a / b, correctly rounded
 WF_HD double div_(double a, double b) {
@@ -238,7 +252,7 @@ WF_HD double div_(double a, double b) {
 #endif
     return a / b;
 }
-// a / b, correctly rounded, with rb = 1 / b (correctly rounded or within an ulp)
+// a / b, correctly rounded, with rb = 1 / b (correctly rounded, or rcp_kept's unless that is 0)
 WF_HD double div_by_(double a, double b, double rb) {
 #ifdef __CUDA_ARCH__
     if (quot_in_range(a, b)) return quot_raw(a, b, rb);

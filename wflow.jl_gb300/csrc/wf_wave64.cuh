@@ -138,8 +138,7 @@ __device__ __forceinline__ bool gather(const WfDevGraph& g, const WfSweep& sw, c
 constexpr double MIN_FLOW_QROOT = 0x1.0c6f7a0b5ed8ap-20;  // 1e-30^0.2 (routing/utils.jl:2)
 
 // What the solve needs of the node's previous discharge: u = q^0.2, A = alpha u^3, and of the first
-// Newton iterate u (u > 0) P = u^3 (dt_dx u^2 + alpha), the derivative df and 1 / df to within an ulp
-// (0 where the quotient has to take the compiler's division, see div_).
+// Newton iterate u (u > 0) P = u^3 (dt_dx u^2 + alpha), the derivative df and 1 / df (rcp_kept).
 struct KwState {
     double u, A, P, df, rdf;
 };
@@ -154,7 +153,7 @@ __device__ __forceinline__ void kw_state(double q_prev, double dt_dx, double alp
         const double u3 = u2 * k.u;
         k.P = u3 * (dt_dx * u2 + alpha);
         k.df = u2 * (c1 * u2 + c2);
-        k.rdf = wfm::quot_in_range(1.0, k.df) && !wfm::below_power(k.df) ? wfm::rcp_raw(k.df) : 0.0;
+        k.rdf = wfm::rcp_kept(k.df);
     }
 }
 
