@@ -1097,7 +1097,7 @@ struct KwWave64 {
     struct In {
         wfz::KwState k;
         double b, dt_dx, c1, c2, alpha, q_prev;
-        double u;                // river: final iterate of this launch's last sub-step (0: none yet)
+        double u;                // river: final iterate of the round before, if there was one
         double c_q, c_qin, c_x;  // cumulative discharge, inflow, flow to the river (abstraction)
     };
     struct St {
@@ -1157,9 +1157,9 @@ struct KwWave64 {
         const bool draws = !LAND && (r.flags & wfz::REC_ABSTRACTION);
         if (draws) {  // abstraction up to 80 % of the storage (surface_kinwave.jl:523-532)
             const double len = F.R[R_LENGTH][slot], ext = F.R[R_EXT_INFLOW][slot];
-            // the storage that the previous sub-step left (of this launch: its final iterate in st.u)
+            // the storage that the previous sub-step left (of this launch: from its final iterate st.u)
             const double storage =
-                gt0_(st.u) ? len * (wfm::is_zero_(st.q_prev) ? 0.0 : x.alpha * (st.u * st.u * st.u)) : F.RM[RV_STORAGE][e];
+                s > 0 ? len * (wfm::is_zero_(st.q_prev) ? 0.0 : x.alpha * (st.u * st.u * st.u)) : F.RM[RV_STORAGE][e];
             taken = jmin(-ext, div_(storage, dt_s) * 0.80);
             q_lat = F.RM[RV_QLAT][e] + (div_(-taken, len) - 0.0);
             b = dt_s * q_lat;
