@@ -1167,10 +1167,10 @@ struct KwWave64 {
         double q, u;
         bool zero = false;
         // q_in + q_prev + q_lat == 0: only without a positive previous discharge or with a negative term,
-        // and then not where FP32 sees a difference
-        const float in32 = wfm::f32_of(qin) + wfm::f32_of(st.q_prev), lat32 = wfm::f32_of(b) * r_dt32;
+        // and then not where the sum in FP32 is far above what the three terms' roundings leave
+        const float in32 = wfm::f32_of(qin), prev32 = wfm::f32_of(st.q_prev), lat32 = wfm::f32_of(b) * r_dt32;
         if (!(gt0_(st.q_prev) && !lt_(b, 0.0) && !lt_(qin, 0.0)) &&
-            !(fabsf(in32 + lat32) > 1e-4f * (fabsf(in32) + fabsf(lat32)))) {
+            !(fabsf(in32 + prev32 + lat32) > 1e-4f * (fabsf(in32) + fabsf(prev32) + fabsf(lat32)))) {
             if (!draws)
                 q_lat = LAND ? F.Mf[OL_QLAT][e]
                              : F.RM[RV_QLAT][e] + (div_(F.R[R_EXT_INFLOW][slot], F.R[R_LENGTH][slot]) - 0.0);
