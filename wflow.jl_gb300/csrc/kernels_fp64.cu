@@ -189,11 +189,14 @@ __device__ __forceinline__ double rwu_feddes(double h, double h1, double h2, dou
 }
 
 // rwu_feddes of a layer's Brooks-Corey head. The reduction is 0 below h4 and, for a1 != 0, 1 from h3
-// up: an FP32 head (within 1e-5) decides those cases when it is more than 0.1 % away from both
-// heads, and only the heads between them pay the power and three divisions (80 FP64 instructions).
+// up: an FP32 head decides those cases when it is more than 0.1 % away from both heads, and only the
+// heads between them pay the power and three divisions (80 FP64 instructions). The porosity range is
+// subtracted in FP64, so that the saturation x is within 4e-7 also where the two porosities are close. The
+// head is then within 1e-4 over the range that the FP32 path takes: (c - 3) / 2 < 29 times the error of
+// log2 x, below 3e-6, and half the error of c, 2e-6, times |log2 x| < 20.
 __device__ __forceinline__ double rwu_layer(double vwc, double ts, double tr, double c, double psi, double h1, double h2,
                                             double h3, double h4, double a1) {
-    const float x = wfm::f32_of(vwc) / (wfm::f32_of(ts) - wfm::f32_of(tr));
+    const float x = wfm::f32_of(vwc) / wfm::f32_of(ts - tr);
     const float p32 = wfm::f32_of(psi), c32 = wfm::f32_of(c), lo = wfm::f32_of(h4), hi = wfm::f32_of(h3);
     if (c32 > 3.01f && c32 < 60.0f && p32 < 0.0f && lo < hi && hi < 0.0f && x > 1e-6f && x < 1e6f) {
         const float head = p32 * exp2f(-0.5f * (c32 - 3.0f) * log2f(x));
