@@ -1,6 +1,6 @@
 """The root water uptake reduction that an FP32 estimate of the soil-water head decides (FP64 form),
-where FP32 says little: a porosity range theta_s - theta_r that is small against theta_s. Against the
-oracle, relative 1e-9."""
+where FP32 says little: a porosity range theta_s - theta_r that is small against theta_s, and
+parameters without a value. Against the oracle, relative 1e-9."""
 
 import numpy as np
 import pytest
@@ -27,4 +27,17 @@ def test_small_porosity_range(gpu_lib, decades):
     p, rng = soil(dom, 61)
     p["theta_r"] = p["theta_s"] - 10.0 ** rng.uniform(*decades, dom.n_land)
     _, _, res = run_pair(dom, synthetic.make_config(86400.0), 6, params=p)
+    assert_parity(res)
+
+
+def test_air_entry_pressure_without_a_value(gpu_lib):
+    # NaN of either sign (a quotient 0 / 0 gives a negative one on x86)
+    dom = synthetic.make_domain(24, 1000.0, seed=62)
+    p, rng = soil(dom, 62)
+    psi = p["air_entry_pressure"] = p["air_entry_pressure"].copy()
+    some = rng.random(dom.n_land) < 0.2
+    psi[some] = np.where(rng.random(some.sum()) < 0.5, 1.0, -1.0) * np.nan
+    psi[some] = np.copysign(psi[some], np.where(rng.random(some.sum()) < 0.5, 1.0, -1.0))
+    assert np.signbit(psi[some]).any()
+    _, _, res = run_pair(dom, synthetic.make_config(86400.0), 4, params=p)
     assert_parity(res)

@@ -198,7 +198,8 @@ __device__ __forceinline__ double rwu_layer(double vwc, double ts, double tr, do
                                             double h3, double h4, double a1) {
     const float x = wfm::f32_of(vwc) / wfm::f32_of(ts - tr);
     const float p32 = wfm::f32_of(psi), c32 = wfm::f32_of(c), lo = wfm::f32_of(h4), hi = wfm::f32_of(h3);
-    if (c32 > 3.01f && c32 < 60.0f && p32 < 0.0f && lo < hi && hi < 0.0f && x > 1e-6f && x < 1e6f) {
+    // (f32_of gives an infinity for a NaN: the FP64 path takes those)
+    if (c32 > 3.01f && c32 < 60.0f && p32 < 0.0f && p32 > -1e30f && lo < hi && hi < 0.0f && x > 1e-6f && x < 1e6f) {
         const float head = p32 * exp2f(-0.5f * (c32 - 3.0f) * log2f(x));
         if (head > hi * 0.999f && !wfm::is_zero_(a1)) return 1.0;
         if (head < lo * 1.001f) return 0.0;
