@@ -1,9 +1,10 @@
-// Device paths of wf_math.cuh on given values, for tests/test_fp64_bits_gpu.py (built there with the
-// FP64 kernels' flags).
+// Device paths of wf_math.cuh and li_scheme.cuh on given values, for tests/test_fp64_bits_gpu.py (built
+// there with the FP64 kernels' flags).
 #include <cstdint>
 
 #include <cuda_runtime.h>
 
+#include "li_scheme.cuh"
 #include "wf_math.cuh"
 
 namespace {
@@ -27,6 +28,21 @@ __global__ void quotient_kernel(const double* a, const double* b, double* out, i
     double o[N_QUOT];
     quotients(a[i], b[i], o);
     for (int k = 0; k < N_QUOT; ++k) out[k * n + i] = o[k];
+}
+
+// the edge flows of the local-inertial schemes: columns q0, zs0, zs1, hf, width and n^2 (a
+// cell length of 100 m, a step of 5 s)
+constexpr int N_EDGE = 6;
+WF_HD void edge(const double* x, int64_t n, int64_t i, double* out) {
+    const double q0 = x[i], zs0 = x[n + i], zs1 = x[2 * n + i], hf = x[3 * n + i], w = x[4 * n + i],
+                 nsq = x[5 * n + i];
+    const double A = w * hf, R = wfm::div_(A, 2.0 * hf + w);
+    out[i] = wfli::flow(q0, zs0, zs1, hf, A, R, 100.0, 1.0 / 100.0, nsq, true, 5.0);
+    out[n + i] = wfli::flow_rect(0.9, q0, 0.5 * q0, 0.7 * q0, zs0, zs1, hf, w, 100.0, 1.0 / 100.0, nsq, true, 5.0);
+}
+__global__ void edge_kernel(const double* x, double* out, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) edge(x, n, i, out);
 }
 
 template <class Launch>
@@ -58,6 +74,15 @@ int quotients_host(const double* ab, double* out, int64_t n) {
 int quotients_device(const double* ab, double* out, int64_t n) {
     return on_device(ab, 16 * n, out, 8 * N_QUOT * n, [&](unsigned char* d, unsigned char* o) {
         quotient_kernel<<<blocks(n), 128>>>((const double*)d, (const double*)d + n, (double*)o, n);
+    });
+}
+int edges_host(const double* x, double* out, int64_t n) {
+    for (int64_t i = 0; i < n; ++i) edge(x, n, i, out);
+    return 0;
+}
+int edges_device(const double* x, double* out, int64_t n) {
+    return on_device(x, 8 * N_EDGE * n, out, 16 * n, [&](unsigned char* d, unsigned char* o) {
+        edge_kernel<<<blocks(n), 128>>>((const double*)d, (double*)o, n);
     });
 }
 }

@@ -1,5 +1,6 @@
 """Device paths against host paths to the last bit, signs of zeros included: the elementary functions and
-comparisons of wf_math.cuh, and quotients with the reciprocals that the kernels use."""
+comparisons of wf_math.cuh, quotients with the reciprocals that the kernels use, and the edge flows of the
+local-inertial schemes."""
 
 import ctypes as C
 import subprocess
@@ -76,3 +77,21 @@ def test_quotients(bits):
     for k in range(3):
         bad = differ(host[k], dev[k])
         assert not bad.any(), (k, bad.sum(), ab[:, bad][:, :3], host[k][bad][:3], dev[k][bad][:3])
+
+
+@pytest.mark.parametrize("decades", [(-3.0, 1.0), (-12.0, -3.0), (-32.0, -20.0)])
+def test_edge_flows(bits, decades):
+    # depths from the usual ones down to those whose limit of the flow leaves FP32's range; without
+    # friction and slope the discharge stays what it was, from the critical one to a part in 10^6 of it
+    rng, n = np.random.default_rng(15), 400_000
+    hf, w = 10.0 ** rng.uniform(*decades, n), 10.0 ** rng.uniform(-1, 2, n)
+    limit = w * hf * np.sqrt(9.80665 * hf)
+    q0 = rng.choice([-1.0, 1.0], n) * limit * (1.0 + rng.choice([-1.0, 1.0], n) * 10.0 ** rng.uniform(-6, 0, n))
+    still = rng.random(n) < 0.5
+    zs0 = np.where(still, 0.0, rng.uniform(0, 10, n))
+    zs1 = np.where(still, 0.0, zs0 + rng.uniform(-1, 1, n) * hf)
+    x = np.ascontiguousarray(np.stack([q0, zs0, zs1, hf, w, np.where(still, 0.0, 9e-4)]))
+    host, dev = call(bits.edges_host, x, 2, n), call(bits.edges_device, x, 2, n)
+    for k, name in enumerate(("general cross-section", "rectangular")):
+        bad = differ(host[k], dev[k])
+        assert not bad.any(), (name, bad.sum(), x[:, bad][:, :2], host[k][bad][:2], dev[k][bad][:2])
