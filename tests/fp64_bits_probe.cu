@@ -1,11 +1,12 @@
-// Device paths of wf_math.cuh and li_scheme.cuh on given values, for tests/test_fp64_bits_gpu.py (built
-// there with the FP64 kernels' flags).
+// Device paths of wf_math.cuh, li_scheme.cuh and wf_wave.cuh on given values, for
+// tests/test_fp64_bits_gpu.py (built there with the FP64 kernels' flags).
 #include <cstdint>
 
 #include <cuda_runtime.h>
 
 #include "li_scheme.cuh"
 #include "wf_math.cuh"
+#include "wf_wave.cuh"
 
 namespace {
 constexpr int N_QUOT = 3;
@@ -43,6 +44,12 @@ WF_HD void edge(const double* x, int64_t n, int64_t i, double* out) {
 __global__ void edge_kernel(const double* x, double* out, int64_t n) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) edge(x, n, i, out);
+}
+
+// words published to other warps
+__global__ void publish_kernel(const unsigned long long* w, unsigned long long* out, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) wfv::st_relaxed(&out[i], w[i]);
 }
 
 template <class Launch>
@@ -83,6 +90,11 @@ int edges_host(const double* x, double* out, int64_t n) {
 int edges_device(const double* x, double* out, int64_t n) {
     return on_device(x, 8 * N_EDGE * n, out, 16 * n, [&](unsigned char* d, unsigned char* o) {
         edge_kernel<<<blocks(n), 128>>>((const double*)d, (double*)o, n);
+    });
+}
+int publish_device(const uint64_t* w, uint64_t* out, int64_t n) {
+    return on_device(w, 8 * n, out, 8 * n, [&](unsigned char* d, unsigned char* o) {
+        publish_kernel<<<blocks(n), 128>>>((const unsigned long long*)d, (unsigned long long*)o, n);
     });
 }
 }

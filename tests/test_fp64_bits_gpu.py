@@ -1,6 +1,6 @@
 """Device paths against host paths to the last bit, signs of zeros included: the elementary functions and
-comparisons of wf_math.cuh, quotients with the reciprocals that the kernels use, and the edge flows of the
-local-inertial schemes."""
+comparisons of wf_math.cuh, quotients with the reciprocals that the kernels use, the edge flows of the
+local-inertial schemes, and what a chain end publishes."""
 
 import ctypes as C
 import subprocess
@@ -95,3 +95,13 @@ def test_edge_flows(bits, decades):
     for k, name in enumerate(("general cross-section", "rectangular")):
         bad = differ(host[k], dev[k])
         assert not bad.any(), (name, bad.sum(), x[:, bad][:, :2], host[k][bad][:2], dev[k][bad][:2])
+
+
+def test_published_words(bits):
+    # the one pattern that marks an unpublished word is a NaN in both readings of a word (a double, a pair
+    # of floats), and so is what stands for it; every other word passes unchanged
+    w = np.array([0xFFFFFFFFFFFFFFFF, 0, 1, 0x3FF0000000000000, 0x7FF8000000000000, 0xFFFFFFFFFFFFFFFE], np.uint64)
+    out = call(bits.publish_device, w, 1, w.size)[0]
+    assert (out[1:] == w[1:]).all()
+    assert out[0] != w[0]
+    assert np.isnan(out[:1].view(np.float64)).all() and np.isnan(out[:1].view(np.float32)).all()

@@ -28,9 +28,12 @@
 
 namespace wfv {
 
-constexpr unsigned long long SENTINEL = 0xFFFFFFFFFFFFFFFFULL;   // end_q fill (a NaN pair no arithmetic yields here)
-constexpr unsigned long long QUIET_NAN = 0x7FC000007FC00000ULL;  // published in place of the sentinel pattern
-constexpr int MAX_GROUP = 16;                                    // sub-steps per launch of the slim walker
+// The fill of end_q: a NaN, read as a double (the FP64 form, snow transport) or as a pair of floats (the
+// split form). A NaN of that pattern from the inputs keeps it through FP64 arithmetic, so another
+// pattern that is NaN in both readings is published in its place.
+constexpr unsigned long long SENTINEL = 0xFFFFFFFFFFFFFFFFULL;
+constexpr unsigned long long QUIET_NAN = 0x7FFFFFFF7FFFFFFFULL;
+constexpr int MAX_GROUP = 16;  // sub-steps per launch of the slim walker
 
 // The relaxed loads and stores of published discharges carry no ordering duty (a consumer uses
 // only the value it reads), so they have no compiler memory clobber: a clobber would make the
