@@ -320,7 +320,7 @@ typedef struct WfMetrics {
 /* Tuning knobs (filled by the autotuner; zero = library default). */
 typedef struct WfTuning {
     int32_t vertical_block;   /* threads per block of the per-cell kernels */
-    int32_t routing_warps;    /* warps per block of the routing wavefront kernels */
+    int32_t routing_warps;    /* warps per block of the routing wavefront kernels (0: 4, at most 4 take effect) */
     int32_t routing_blocks_per_sm;
     int32_t use_graph;        /* capture the step in a CUDA graph (1 = yes, default) */
     int32_t reserved[8];      /* [0] wait budget (us), [1] test hook (0), [2] per-kernel timing,

@@ -1565,7 +1565,7 @@ int grid_for(int64_t n, int block, int num_sms) {
 
 template <class Phys>
 cudaError_t launch_walk(const Phys& phys, const WfLaunchCfg& c) {
-    const int threads = 32 * (c.walk_warps > 0 ? c.walk_warps : 4);
+    const int threads = wave_threads(c);
     int blocks;
     Phys p = phys;
     p.sw.SL = p.sw.aflag ? 1 : wave_sub_lanes(p.sw.S, c);
@@ -1631,7 +1631,7 @@ namespace {
 // chains are packed as loosely as their number allows (wave_lanes).
 template <class Phys, bool MULTI>
 cudaError_t launch_wave64(const Phys& phys, const WfLaunchCfg& c) {
-    const int threads = 32 * (c.walk_warps > 0 ? std::min(c.walk_warps, 4) : 4);
+    const int threads = wave_threads(c);
     const size_t smem = wfz::walk_smem(threads);
     const WfDevGraph& g = phys.g;
     int SLr = g.lanes, SLs = SLr;

@@ -1875,7 +1875,7 @@ __global__ void __launch_bounds__(128, Phys::kBlocks) wave_kernel(Phys phys, int
 // eight of those chains share a warp at least.
 template <class Phys, bool MULTI>
 cudaError_t launch_wave_as(const Phys& phys, const WfLaunchCfg& c) {
-    const int threads = 32 * (c.walk_warps > 0 ? std::min(c.walk_warps, 4) : 4);
+    const int threads = wave_threads(c);
     const WfDevGraph& g = phys.g;
     const size_t smem = wfv::lean_smem(threads, Phys::kVecs);
     auto kernel = wave_kernel<Phys, MULTI>;
@@ -2282,7 +2282,7 @@ __global__ void __launch_bounds__(128) walk_split_kernel(Phys phys) {
 
 template <class Phys>
 cudaError_t launch_walk_split(const Phys& phys, const WfLaunchCfg& c) {
-    const int threads = 32 * (c.walk_warps > 0 ? c.walk_warps : 4);
+    const int threads = wave_threads(c);
     int blocks;
     Phys p = phys;
     p.sw.SL = 1;

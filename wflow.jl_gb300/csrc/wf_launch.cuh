@@ -9,6 +9,10 @@
 #include "wf_fields.cuh"
 #include "wf_kernels.h"
 
+// Threads per block of a wavefront launch: 4 warps, which the kernels are bounded to, or fewer by the tuning
+// (which accepts up to 32; more than 4 give 4).
+inline int wave_threads(const WfLaunchCfg& c) { return 32 * (c.walk_warps > 0 ? std::min(c.walk_warps, 4) : 4); }
+
 // Blocks of a persistent wavefront launch and the number of work items dispatched first.
 //
 // The grid is every block that fits on the device at once (occupancy), capped by the work.
