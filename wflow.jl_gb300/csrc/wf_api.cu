@@ -46,7 +46,7 @@ struct DevGraphAlloc {
     uint32_t* flags = nullptr;
     double* end_q = nullptr;
     unsigned long long* ticket = nullptr;
-    int32_t s_cap = 1;
+    int32_t s_cap = 1;  // sub-steps that end_q has room for
     int32_t* snow_up = nullptr;  // land graph with snow transport: up_chain in topological-sort order
 };
 
@@ -2079,6 +2079,15 @@ namespace {
 
 constexpr int64_t kMaxAdaptiveSubsteps = 100000;
 
+// Fills the published discharges of a launch of S sub-steps with the sentinel and gives its view of the
+// graph: the launch uses (and clears) a word per chain end and sub-step of its own, not the s_cap that
+// the buffer has room for.
+int clear_end_q(WfHandle* h, WfDevGraph& g, int S) {
+    g.s_cap = S;
+    CK(cudaMemsetAsync(g.end_q, 0xFF, (size_t)g.n_chains * h->M * S * sizeof(double), h->stream));
+    return WF_OK;
+}
+
 // The per-cell update of the step. With gravitational snow transport its snow part, the two
 // material sweeps over the land graph (one sub-step of the model step each, in the land graph's
 // wavefront scratch) and the inflow kernel run before its soil part (sbm.jl:92-131).
@@ -2102,10 +2111,11 @@ int enqueue_vertical(WfHandle* h, const WfLaunchCfg& lc, const WfDevGraph& gl, i
         sw.dts = h->dts_ssf;
         sw.wait_ns = h->wait_ns;
         sw.wait_offset = h->wait_offset;
-        CK(cudaMemsetAsync(gl.end_q, 0xFF, (size_t)h->land.plan.n_chains * h->M * h->land.s_cap * sizeof(double),
-                           h->stream));
-        CK(cudaMemsetAsync(gl.ticket, 0, sizeof(unsigned long long), h->stream));
-        CK(wf_snow_transport_sweep(h->F, gl, sw, material, lc));
+        WfDevGraph g = gl;
+        const int rc = clear_end_q(h, g, 1);
+        if (rc) return rc;
+        CK(cudaMemsetAsync(g.ticket, 0, sizeof(unsigned long long), h->stream));
+        CK(wf_snow_transport_sweep(h->F, g, sw, material, lc));
         ++nl;
     }
     CK(wf_snow_in(h->F, gl, lc));
@@ -2117,7 +2127,7 @@ int enqueue_vertical(WfHandle* h, const WfLaunchCfg& lc, const WfDevGraph& gl, i
 
 // One FP64 sweep (0 subsurface, 1 overland, 2 river) with the slim wavefronts: launches of up to s_cap
 // sub-steps of one size, each with its per-cell kernels before and after it.
-int sweep_wave64(WfHandle* h, const DevGraphAlloc& G, const WfDevGraph& g, const std::vector<double>& dts,
+int sweep_wave64(WfHandle* h, const DevGraphAlloc& G, WfDevGraph g, const std::vector<double>& dts,
                  const double* d_dts, int which, const WfLaunchCfg& lc, int64_t& nl) {
     const int total = (int)dts.size();
     for (int first = 0; first < total;) {
@@ -2133,7 +2143,8 @@ int sweep_wave64(WfHandle* h, const DevGraphAlloc& G, const WfDevGraph& g, const
         sw.dt_s = dts[first];
         sw.wait_ns = h->wait_ns;
         sw.wait_offset = h->wait_offset;
-        CK(cudaMemsetAsync(g.end_q, 0xFF, (size_t)G.plan.n_chains * h->M * G.s_cap * sizeof(double), h->stream));
+        const int rc = clear_end_q(h, g, sw.S);
+        if (rc) return rc;
         CK(cudaMemsetAsync(g.ticket, 0, sizeof(unsigned long long), h->stream));
         CK(which == 0   ? wf_fp64_ssf_wave(h->F, g, sw, lc)
            : which == 1 ? wf_fp64_overland(h->F, g, sw, lc)

@@ -232,9 +232,9 @@ struct WfDevGraph {
     int32_t lanes;        // packing lanes per chain-member pair of the slim wavefronts,
     int32_t lanes_multi;  // and the most of them that a launch of several sub-steps is worth
     uint32_t* flags;      // [n_chains * M] epoch of the last published sub-step
-    double* end_q;        // [n_chains * M * s_cap] q of each chain end per sub-step
+    double* end_q;        // [n_chains * s_cap * M] q of each chain end per sub-step
     unsigned long long* ticket;  // work counter of the current launch
-    int32_t s_cap;        // sub-steps per launch
+    int32_t s_cap;        // sub-steps that end_q is laid out for
     // land graph with snow transport: for each slot's upstream entries up_ptr[slot] ..
     // up_ptr[slot + 1], their chains (up_chain) in the order of the graph's topological sort (the
     // order in which the transport hands material on)
