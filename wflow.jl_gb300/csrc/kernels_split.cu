@@ -1552,10 +1552,10 @@ struct SsfWave {
 
 // The lateral inflow of river cell rs (element re) from the land cell of element le, with trsum
 // the step's sum of the overland flow to the river (update_lateral_inflow!,
-// surface_kinwave.jl:710-734): stores the river cell's inflow, lateral inflow and the lateral
-// inflow with the external inflow, and returns the latter. 
-__device__ __forceinline__ wff::ff river_lateral(const WfDevFields& F, int64_t le, int64_t rs, int64_t re,
-                                                 wff::ff trsum) {
+// surface_kinwave.jl:710-734): stores the river cell's inflow and its lateral inflow with the external
+// inflow (an abstraction is the river sweep's).
+__device__ __forceinline__ void river_lateral(const WfDevFields& F, int64_t le, int64_t rs, int64_t re,
+                                              wff::ff trsum) {
     using wff::ff;
     const ff tr_avg = wff::mul(trsum, ff{F.inv_dt_hi, F.inv_dt_lo});
     const ff inv_len = ldrs(F, R_INV_LENGTH, rs);
@@ -1563,11 +1563,9 @@ __device__ __forceinline__ wff::ff river_lateral(const WfDevFields& F, int64_t l
                             wff::mul(ldm(F, NET_RUNOFF_RIVER, le), ldrs(F, R_AREA, rs)));
     str(F, RV_INWATER, re, inw);
     const ff qlat = wff::mul(inw, inv_len);
-    str(F, RV_QLAT, re, qlat);
     const float ext = F.Rf[R_EXT_INFLOW][rs];
     const ff qlt = ext < 0.0f ? qlat : wff::add(qlat, wff::mul(inv_len, ext));
     F.rv_lat[re] = make_float2(qlt.hi, qlt.lo);
-    return qlt;
 }
 
 // Overland flow (surface_process.jl:24-70 per node, routing/surface_kinwave.jl sub-steps) in

@@ -36,7 +36,6 @@ struct DevGraphAlloc {
     int64_t *chunk_base = nullptr, *up_slot = nullptr, *node_of_slot = nullptr;
     int32_t *chunk_len = nullptr, *chain_len = nullptr, *up_ptr = nullptr, *up_chain = nullptr, *chunk_g = nullptr;
     int64_t* chunk_chain0 = nullptr;
-    uint8_t* is_chain_end = nullptr;
     double *up_w = nullptr, *up_fr = nullptr;
     float *up_wf = nullptr, *up_frf = nullptr;
     int4* up_rec = nullptr;
@@ -62,6 +61,7 @@ struct WfHandle {
     int M = 1, N = 4;
     DevGraphAlloc land, river;
     WfDevFields F{};
+    double* river_scratch[10] = {};  // FP64 form: F.W of the river sweep where the land's fields are too small
     std::vector<void*> allocs;
     int32_t* status = nullptr;  // device status word
     double* staging = nullptr;  // [max(n, nr) * M] external-order staging
@@ -235,7 +235,6 @@ int plan_graph(WfHandle* h, DevGraphAlloc& G, int64_t n, const int32_t* ds, int 
     if ((rc = upload(h, &G.up_ptr, P.up_ptr))) return rc;
     if ((rc = upload(h, &G.up_slot, P.up_slot))) return rc;
     if ((rc = upload(h, &G.up_chain, P.up_chain))) return rc;
-    if ((rc = upload(h, &G.is_chain_end, P.is_chain_end))) return rc;
     if ((rc = upload(h, &G.node_of_slot, P.node_of_slot))) return rc;
     G.s_cap = s_cap;
     const int s_most = h->cfg.form == WF_FORM_SPLIT ? std::min<int>(s_cap, wfv::MAX_GROUP) : s_cap;
@@ -265,7 +264,6 @@ WfDevGraph dev_graph(const DevGraphAlloc& G, int M) {
     g.up_ptr = G.up_ptr;
     g.up_slot = G.up_slot;
     g.up_chain = G.up_chain;
-    g.is_chain_end = G.is_chain_end;
     g.up_w = G.up_w;
     g.up_fr = G.up_fr;
     g.up_wf = G.up_wf;
@@ -1170,7 +1168,8 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
         ls.push_back({INV_AREA, inv_area});
         ls.push_back({INV_SFW, inv_sfw});
     }
-    for (auto& x : ls) CKR(upload_slots(h, &F.L[x.idx], x.v, PL, M, n, false));
+    for (auto& x : ls)
+        if (F.split || !wf_split_only_static(x.idx)) CKR(upload_slots(h, &F.L[x.idx], x.v, PL, M, n, false));
     for (int k = 0; k < N; ++k) {
         std::vector<double> va(act.begin() + (size_t)k * n, act.begin() + (size_t)(k + 1) * n);
         std::vector<double> vr(rootfrac.begin() + (size_t)k * n, rootfrac.begin() + (size_t)(k + 1) * n);
@@ -1205,7 +1204,7 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
     // ---- land member fields
     std::vector<double> zeros_m((size_t)n * M, 0.0);
     for (int f = 0; f < M_COUNT; ++f) {
-        if (!F.split && wf_split_only_member(f)) continue;
+        if (F.split ? wf_fp64_only_member(f) : wf_split_only_member(f)) continue;
         if (F.split && !wf_split_ff_member(f) && !wf_split_fp64_member(f)) continue;  // FP32 arrays only (below)
         const std::vector<double>* src = &zeros_m;
         switch (f) {
@@ -1286,14 +1285,13 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
     CKR(upload_slots(h, &F.R[R_ALPHA], r_alpha, PR, M, nr, false));
     CKR(upload_slots(h, &F.R[R_EXT_INFLOW], r_ext, PR, M, nr, false));
     CKR(upload_slots(h, &F.R[R_AREA], r_area, PR, M, nr, false));
-    CKR(upload_slots(h, &F.R[R_INV_LENGTH], r_inv_len, PR, M, nr, false));
-    CKR(upload_slots(h, &F.R[R_INV_WIDTH], r_inv_w, PR, M, nr, false));
     std::vector<double> zeros_r((size_t)std::max<int64_t>(nr, 1) * M, 0.0);
     for (int f = 0; f < RM_COUNT; ++f) {
         if (wf_split_only_river_member(f)) {
             if (F.split) CKR(upload_slots_f32(h, &F.RMh[f], zeros_r, PR, M, nr, true));
             continue;
         }
+        if (F.split && wf_fp64_only_river_member(f)) continue;
         if (F.split) CKR(upload_slots_ff(h, &F.RMh[f], &F.RMl[f], zeros_r, PR, M, nr, true));
         else CKR(upload_slots(h, &F.RM[f], zeros_r, PR, M, nr, true));
     }
@@ -1323,11 +1321,14 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
             w[o] = 1.0 - f;
             fr[o] = f;
         }
-        CKR(upload(h, &G.up_w, w));
-        CKR(upload(h, &G.up_fr, fr));
         std::vector<float> wf(w.begin(), w.end()), frf(fr.begin(), fr.end());
-        CKR(upload(h, &G.up_wf, wf));
-        CKR(upload(h, &G.up_frf, frf));
+        if (F.split) {
+            CKR(upload(h, &G.up_wf, wf));
+            CKR(upload(h, &G.up_frf, frf));
+        } else {
+            CKR(upload(h, &G.up_w, w));
+            CKR(upload(h, &G.up_fr, fr));
+        }
         if (F.split) {  // per-slot records and constants of the slim wavefronts
             std::vector<int4> rec(std::max<int64_t>(P.n_slots, 1), int4{-1, -1, 0, 0});
             std::vector<float4> st(2 * rec.size(), float4{0.0f, 0.0f, 0.0f, 0.0f}), ssf(st);
@@ -1554,8 +1555,8 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
     // adaptive sub-steps that sub-step is the whole model step (used when every member's first
     // Courant sub-step reaches the end of the step, the usual case)
     F.ssf_single = h->h_dts_ssf.size() == 1 && (F.split || !h->adaptive);
-    if (!F.split)
-        for (int k = 0; k < 10; ++k) CKR(dalloc(h, &F.W[k], (size_t)std::max(PL.n_slots, PR.n_slots) * M));
+    if (!F.split && PR.n_slots > PL.n_slots)  // padding can make the river's layout the larger one
+        for (auto& w : h->river_scratch) CKR(dalloc(h, &w, (size_t)PR.n_slots * M));
     F.dt_ssf = h->h_dts_ssf[0];
     F.inv_dt_ssf = 1.0 / h->h_dts_ssf[0];
     F.inv_dt_hi = (float)F.inv_dt;
@@ -2125,11 +2126,36 @@ int enqueue_vertical(WfHandle* h, const WfLaunchCfg& lc, const WfDevGraph& gl, i
     return WF_OK;
 }
 
+// The fields of an FP64 sweep with the slim wavefronts (0 subsurface, 1 overland, 2 river), its terms W in
+// land fields that hold nothing while it runs, so that they take no memory of their own: the subsurface
+// flow's cumulative fluxes (done with after its own sweep, and not used when that has one sub-step), the
+// total storage (written at the end of the step) and, for the first three terms (which the sweep's
+// completion kernel does not read), the overland sweep's cumulative fluxes or, while those are in use, its
+// averages (written by its last completion kernel).
+WfDevFields sweep_fields(const WfHandle* h, int which) {
+    WfDevFields F = h->F;
+    double* const* M = F.Mf;
+    double* const held[] = {M[which == 1 ? OL_Q_AVG : OL_Q_CUM],
+                            M[which == 1 ? OL_QIN_AVG : OL_QIN_CUM],
+                            M[which == 1 ? OL_TR_AVG : OL_TR_CUM],
+                            M[SSF_QIN_CUM],
+                            M[SSF_Q_CUM],
+                            M[SSF_TR_CUM],
+                            M[SSF_EXF_CUM],
+                            M[SSF_QNET_CUM],
+                            M[RCH_FLUX_CUM],
+                            M[TOTAL_STORAGE]};
+    const bool own = which == 2 && h->river_scratch[0];
+    for (int k = 0; k < 10; ++k) F.W[k] = own ? h->river_scratch[k] : held[k];
+    return F;
+}
+
 // One FP64 sweep (0 subsurface, 1 overland, 2 river) with the slim wavefronts: launches of up to s_cap
 // sub-steps of one size, each with its per-cell kernels before and after it.
 int sweep_wave64(WfHandle* h, const DevGraphAlloc& G, WfDevGraph g, const std::vector<double>& dts,
                  const double* d_dts, int which, const WfLaunchCfg& lc, int64_t& nl) {
     const int total = (int)dts.size();
+    const WfDevFields F = sweep_fields(h, which);
     for (int first = 0; first < total;) {
         WfSweep sw{};
         sw.S = 1;
@@ -2146,9 +2172,9 @@ int sweep_wave64(WfHandle* h, const DevGraphAlloc& G, WfDevGraph g, const std::v
         const int rc = clear_end_q(h, g, sw.S);
         if (rc) return rc;
         CK(cudaMemsetAsync(g.ticket, 0, sizeof(unsigned long long), h->stream));
-        CK(which == 0   ? wf_fp64_ssf_wave(h->F, g, sw, lc)
-           : which == 1 ? wf_fp64_overland(h->F, g, sw, lc)
-                        : wf_fp64_river(h->F, g, sw, lc));
+        CK(which == 0   ? wf_fp64_ssf_wave(F, g, sw, lc)
+           : which == 1 ? wf_fp64_overland(F, g, sw, lc)
+                        : wf_fp64_river(F, g, sw, lc));
         nl += 3;
         first += sw.S;
     }
@@ -2275,7 +2301,8 @@ int enqueue_step(WfHandle* h, int64_t* launches) {
             if (!split && kind != WF_ADAPT_SSF) {
                 CK(cudaMemsetAsync(G.end_q, 0xFF, (size_t)G.plan.n_chains * h->M * G.s_cap * sizeof(double),
                                    h->stream));
-                e = kind == WF_ADAPT_LAND ? wf_fp64_overland(h->F, g, sw, lc) : wf_fp64_river(h->F, g, sw, lc);
+                e = kind == WF_ADAPT_LAND ? wf_fp64_overland(sweep_fields(h, 1), g, sw, lc)
+                                          : wf_fp64_river(sweep_fields(h, 2), g, sw, lc);
                 nl += 2;
             } else if (slim) {
                 CK(cudaMemsetAsync(G.end_q, 0xFF, (size_t)G.plan.n_chains * h->M * G.s_cap * sizeof(double),

@@ -83,6 +83,15 @@ __host__ __device__ inline bool wf_split_f32_member(int f) {
            f == INTERCEPTION || f == TRANSPIRATION || f == SOIL_EVAP || f == ACT_INFILT || f == SWE;
 }
 
+// What one of the two forms does not use is not allocated by it: the cell constants of the split
+// form's kernels, the FP64 form's lateral inflows and cumulative discharges.
+__host__ __device__ inline bool wf_split_only_static(int f) { return f >= INV_FLOW_LENGTH; }
+__host__ __device__ inline bool wf_fp64_only_member(int f) {
+    return f == OL_QLAT || f == OL_Q_CUM || f == OL_QIN_CUM || f == OL_TR_CUM;
+}
+__host__ __device__ inline bool wf_fp64_only_river_member(int f) {
+    return f == RV_QLAT || f == RV_Q_CUM || f == RV_QIN_CUM || f == RV_ABS_CUM;
+}
 // Member fields only the split form's slim wavefronts use (not allocated by the FP64 form).
 __host__ __device__ inline bool wf_split_only_member(int f) { return f >= SSF_QNET; }
 __host__ __device__ inline bool wf_split_only_river_member(int f) { return f >= RV_QSUMH; }
@@ -188,7 +197,8 @@ struct WfDevFields {
     // the overland and river balances are the scheme's
     int32_t li_coupled;
     // FP64 form: terms of the sweep in hand, per element of its graph, written by the per-cell kernel
-    // before the slim wavefront and read by it (WfW64Kw, WfW64Ssf); [max(land, river slots) * M] each
+    // before the slim wavefront and read by it (WfW64Kw, WfW64Ssf). Set for each sweep (wf_api.cu
+    // sweep_fields): member fields that hold nothing while the sweep runs.
     double* W[10];
 };
 
@@ -217,7 +227,6 @@ struct WfDevGraph {
     const int32_t* up_ptr;
     const int64_t* up_slot;
     const int32_t* up_chain;
-    const uint8_t* is_chain_end;
     const double* up_w;   // [up entries] weight of the upstream discharge (land: 1 - fraction to river)
     const double* up_fr;  // [up entries] fraction of the upstream discharge to the river (land only)
     const float* up_wf;   // FP32 copies of up_w / up_fr (split form)
