@@ -65,7 +65,7 @@ def tune(model: Model, forcing, steps=1, verbose=False):
     best_lanes = 0
     if m["steps"] > 0 and max(m["substeps_land"], m["substeps_river"]) > m["steps"]:
         best_lanes_t = best_route_t
-        for lanes in [1, 2, 4, 16]:  # 0 (the packing rules) was measured above
+        for lanes in [1, 2, 4, 8, 16]:  # 0 (the packing rules) was measured above
             model._tune_state = dict(vertical_block=0, routing_warps=best_route[0],
                                      routing_blocks_per_sm=best_route[1], substep_lanes=lanes,
                                      separate_overland_river=1)
