@@ -170,6 +170,9 @@ class Model:
         self._check(self.lib.wf_get_metrics(self.h, C.byref(m)), "wf_get_metrics")
         return {k: getattr(m, k) for k, _ in abi.WfMetrics._fields_}
 
+    # whether set_tuning's sweep_inputs and separate_overland_river select anything (autotune)
+    SWEEP_VARIANTS = False
+
     def set_tuning(self, vertical_block=0, routing_warps=0, routing_blocks_per_sm=0, use_graph=1,
                    wait_budget_us=0, wait_offset=0, kernel_timing=0, substep_lanes=0, sweep_inputs=0,
                    vertical_blocks_per_sm=0, separate_overland_river=0):
