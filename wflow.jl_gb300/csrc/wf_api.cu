@@ -376,7 +376,6 @@ WfLaunchCfg launch_cfg(const WfHandle* h) {
     c.walk_warps = h->tuning.routing_warps;
     c.walk_blocks = h->tuning.routing_blocks_per_sm > 0 ? h->tuning.routing_blocks_per_sm * h->num_sms : 0;
     c.sub_lanes = h->tuning.reserved[3];
-    c.walk_inputs = h->tuning.reserved[4];
     c.vertical_blocks_per_sm = h->tuning.reserved[5];
     return c;
 }
@@ -1009,9 +1008,9 @@ int32_t wf_create_with_reservoir_tables(const WfConfig* c, const WfDomain* d, co
     CKR(upload(h, &h->dts_river, h->h_dts_river));
     CKR(upload(h, &h->dts_ssf, h->h_dts_ssf));
     // wavefront schedules
-    // sub-steps per sweep launch: the split form's slim wavefronts take at most 16 (a shared-
-    // memory row per sub-step), the FP64 walker 32 (which bounds a launch to about a second on
-    // the largest domains)
+    // sub-steps per sweep launch: the split form's slim wavefronts take at most 16 (their sizes travel
+    // in the launch's arguments, WfSweep::dts_f, and the scratch of wf_step_static is laid out for as
+    // many), the FP64 form's 32, a lane each
     const size_t cap = c->form == WF_FORM_SPLIT ? (size_t)wfv::MAX_GROUP : (size_t)32;
     const int cap_land = (int)std::min<size_t>(std::max(h->h_dts_land.size(), h->h_dts_ssf.size()), cap);
     // linked reservoirs: the river runs one sub-step per launch and keeps every upper-to-lower
@@ -1979,12 +1978,10 @@ int32_t wf_set_tuning(WfHandle* h, const WfTuning* t) {
     if (t->reserved[7] != 0) return set_err(h, WF_ERR_INVALID, "reserved tuning fields must be 0");
     h->tuning = *t;
     h->graph_valid = false;
-    // reserved[]: [0] = wait budget in microseconds, [1] = awaited-epoch offset (test hooks),
-    // [2] = per-kernel event timing, [3] = cap of the routing sweeps' sub-step lanes (0 = default),
-    // [4] = bit k: node-major sweep k (0 subsurface, 1 overland, 2 river) keeps its inputs in
-    // registers instead of staging them in shared memory, [5] = blocks per SM of the split
-    // vertical kernel's grid-stride loop (0 = 16), [6] = 1: the split form's overland and river
-    // sweeps in separate launches (0: one launch where the model allows it)
+    // reserved[]: [0] = wait budget in microseconds, [1] = not 0: every wait runs out (test hooks),
+    // [2] = per-kernel event timing, [3] = sub-step lanes of the routing sweeps (0 = by the packing
+    // rules), [5] = blocks per SM of the split vertical kernel's grid-stride loop (0 = 16); [4] and [6]
+    // are accepted and select nothing
     if (t->reserved[0] > 0) h->wait_ns = (uint64_t)t->reserved[0] * 1000ull;
     h->wait_offset = (uint32_t)t->reserved[1];
     h->kernel_timing = t->reserved[2] != 0;

@@ -9,12 +9,11 @@ struct WfLaunchCfg {
     cudaStream_t stream;
     int num_sms;
     int vertical_block;   // threads per block of per-cell kernels
-    int walk_warps;       // warps per block of wavefront kernels
+    int walk_warps;       // warps per block of wavefront kernels (wave_threads)
     int walk_blocks;      // blocks of the persistent wavefront grid (0 = occupancy)
-    int sub_lanes;        // cap of the sub-step lanes of the diagonal schedule (0 = default)
+    int sub_lanes;        // sub-step lanes per chain-member pair (0: the slim wavefronts by their packing rules,
+                          // the plain walker up to 8)
     int vertical_blocks_per_sm;  // grid of the split vertical kernel (0 = 16 per SM)
-    int walk_inputs;      // bit k: node-major sweep k (0 subsurface, 1 overland, 2 river) holds its inputs
-                          // in registers instead of staging them in shared memory
 };
 
 // FP64 plain form (kernels_fp64.cu)

@@ -330,10 +330,11 @@ __device__ __forceinline__ void shfl_up_pod(T& v, int width) {
 
 // ---- staged walk ---------------------------------------------------------------------------------
 //
-// The lead lane of a pair (lane 0 of its SL) copies the inputs of its next RING_D positions into a
+// The lead lane of a pair (lane 0 of its SL) copies the inputs of the position RING_D ahead into a
 // per-warp ring in shared memory with asynchronous copies (cp.async, one commit group per position,
-// issued whether or not the lane has work there), so a position's inputs have had RING_D positions to
-// arrive; the light children's words are loaded two positions ahead from the staged records. Each
+// issued whether or not the lane has work there). The light children's words are loaded two positions
+// ahead from the staged records, so the copies issued in a step are waited for at the start of the
+// next: they have one position to arrive, the words two. Each
 // lane reads back only what it copied itself, so the waits are per thread (cp.async.wait_group) and
 // no barrier is involved. At the end of a time step every lane hands what the node's next sub-step needs
 // (Pass, its state, the words of its light children, loaded during the step) to the next lane with warp
@@ -368,7 +369,9 @@ __device__ __forceinline__ void shfl_up_pod(T& v, int width) {
 // value held in registers to be reloaded after each copy); cp.async.wait_group has one, so the
 // reads of a slot stay after the wait that covers it, and a slot's earlier reads stay before the
 // next wait, which precedes its refill.
-constexpr int RING_D = 3;           // positions staged ahead: each takes 1000 cycles and more, a memory round trip
+// positions staged ahead: one for the copies to arrive (1000 cycles and more, a memory round trip) and the
+// two for the words
+constexpr int RING_D = 3;
 constexpr int RING_R = RING_D + 1;  // ring slots (the slot refilled is the one read a position ago)
 
 __device__ __forceinline__ void cpa16(void* smem, const void* gmem) {
@@ -465,7 +468,7 @@ __device__ __forceinline__ bool ticket(const WfDevGraph& g, const WfSweep& sw, P
         auto step = [&](unsigned long long& ac, unsigned long long& bc, unsigned long long& af,
                         unsigned long long& bf) -> bool {
             if (tt >= steps) return false;
-            cpa_wait<RING_D - 3>();  // groups up to position t + 2 complete
+            cpa_wait<RING_D - 3>();  // every group, up to position t + 2, complete
             look((tt + 2) & (RING_R - 1), af, bf);
             if (lead) {
                 const int k = tt & (RING_R - 1);
