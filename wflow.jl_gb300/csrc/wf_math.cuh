@@ -252,6 +252,13 @@ WF_HD double div_(double a, double b) {
 #endif
     return a / b;
 }
+// a / b, correctly rounded, for operands that are known to be in range (or a is +0)
+WF_HD double div_mid_(double a, double b) {
+#ifdef __CUDA_ARCH__
+    if (!below_power(b)) return quot_raw(a, b, rcp_raw(b));
+#endif
+    return a / b;
+}
 // a / b, correctly rounded, with rb = 1 / b (correctly rounded, or rcp_kept's unless that is 0)
 WF_HD double div_by_(double a, double b, double rb) {
 #ifdef __CUDA_ARCH__
@@ -319,7 +326,7 @@ WF_HD double log(double x) {
         const double mx = from_bits((to_bits(x) & 0x000fffffffffffffULL) | (up ? 0x3fe0000000000000ULL : 0x3ff0000000000000ULL));
         const double f = mx - 1.0;
         const double b = 2.0 + f;
-        const double s = below_power(b) ? f / b : quot_raw(f, b, rcp_raw(b));
+        const double s = div_mid_(f, b);
         const double s2 = s * s;
         double R = 0x1.8618618618618p-4;
         R = __fma_rn(R, s2, 0x1.af286bca1af28p-4);
@@ -392,7 +399,8 @@ WF_HD double cbrt(double x) {
     if (r == 1) m *= 2.0;
     if (r == 2) m *= 4.0;
     double y = 0.6 + 0.2 * m;
-    for (int i = 0; i < 6; ++i) y = y - div_(y * y * y - m, 3.0 * y * y);
+    // m in [1, 8), y in (0.5, 3): the residual is +0 or at least 2^-54
+    for (int i = 0; i < 6; ++i) y = y - div_mid_(y * y * y - m, 3.0 * y * y);
     y = y * from_bits((uint64_t)(q + 1023) << 52);
     return x < 0.0 ? -y : y;
 }
