@@ -10,8 +10,9 @@ the tuning's switches (Model.SWEEP_VARIANTS; the current library has none) is tu
 well: whether a sweep's inputs are staged in shared memory or held in registers, and whether the
 overland and river sweeps share one launch or run one after the other. The tuner times a few steps
 of each candidate with per-kernel CUDA events and keeps the fastest for
-each kernel family. Candidates only change the schedule, never the result: the wavefront
-produces the same values for any dispatch order and any lane count.
+each kernel family. Candidates only change the schedule. The FP64 form gives the same values for
+any dispatch order and any lane count; the split form's river discharge can differ in its last bits
+between lane counts (2e-14 to 5e-13 of it, in a few cells of a daily step).
 """
 
 import itertools

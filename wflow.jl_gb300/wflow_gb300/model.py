@@ -176,7 +176,8 @@ class Model:
     def set_tuning(self, vertical_block=0, routing_warps=0, routing_blocks_per_sm=0, use_graph=1,
                    wait_budget_us=0, wait_offset=0, kernel_timing=0, substep_lanes=0, sweep_inputs=0,
                    vertical_blocks_per_sm=0, separate_overland_river=0):
-        """Launch shape of the step's kernels (results do not depend on it): threads per block of
+        """Launch shape of the step's kernels (results do not depend on it, but for the last bits of
+        the split form's discharges between numbers of sub-step lanes): threads per block of
         the per-cell kernels, warps per block and blocks per SM of the routing sweeps, the
         sub-step lanes of their diagonal schedule (0: by the packing rules), the CUDA graph, and test
         hooks. sweep_inputs and separate_overland_river are accepted and without effect: the sweeps
